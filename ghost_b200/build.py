@@ -19,7 +19,7 @@ INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 SOURCES = ["api.cu", "mlp.cu", "les.cu", "io.cu", "ic_host.cpp"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC",
-              "-Xptxas", "-warn-spills"]
+              "-Xptxas", "-warn-spills", "--split-compile=0"]
 
 
 def nvcc() -> str:

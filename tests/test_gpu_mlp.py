@@ -60,6 +60,29 @@ def test_gradients_match_oracle(B):
         o += n
 
 
+@pytest.mark.parametrize("B", [1, 127, 129, 148 * 128, 148 * 128 + 1, 2 * 148 * 128 + 77])
+def test_gradients_at_tile_edges(B):
+    """Ragged tiles, an idle second tile slot (at most one tile per CTA), a
+    single tile in the second slot, and a second round of tiles: gradients
+    and loss against the BF16-emulating oracle (test_gradients_match_oracle's
+    bound), and inference at the same batch sizes."""
+    import torch
+    p = M.glorot(51)
+    p[M.NH * M.NIN:M.NH * M.NIN + M.NH] = np.linspace(-0.2, 0.2, M.NH)
+    x, t = _data(52, B)
+    m = _mlp(p)
+    xd = torch.from_numpy(x).cuda()
+    g, loss = m.gradients(xd, torch.from_numpy(t).cuda())
+    ge, le = M.gradients(p, x, t, emulate=True)
+    assert abs(loss - le) / le < 1e-5
+    o = 0
+    for name, shape in M.SHAPES:
+        n = int(np.prod(shape))
+        assert rel_l2(g[o:o + n], ge[o:o + n]) < 5e-3, name
+        o += n
+    assert rel_l2(m.forward(xd).cpu().numpy(), M.forward(p, x, emulate=True)) < 2e-3
+
+
 def test_adam_steps_match_oracle():
     import torch
     p = M.glorot(31)
