@@ -16,10 +16,10 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libghost_b200.so")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
-SOURCES = ["api.cu", "mlp.cu", "les.cu", "io.cu", "ic_host.cpp"]
+SOURCES = ["api.cu", "reduce.cu", "mlp.cu", "les.cu", "io.cu", "ic_host.cpp"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC",
-              "-Xptxas", "-warn-spills", "--split-compile=0"]
+              "-Xptxas", "-warn-spills"]
 
 
 def nvcc() -> str:

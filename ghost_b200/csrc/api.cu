@@ -68,7 +68,7 @@ int scratch(ghost_ctx *c, int n, void **out) {
   return GHOST_OK;
 }
 
-static int partials(ghost_ctx *c, size_t n, double **out) {
+int partials(ghost_ctx *c, size_t n, double **out) {
   if (c->partials_elems < n) {
     if (c->partials) cudaFree(c->partials);
     c->partials = nullptr;
@@ -448,14 +448,14 @@ static cudaEvent_t take_event(ghost_ctx *c) {
 }
 
 // Records the start event of a launch; returns the pending slot or -1.
-static int timer_begin(ghost_ctx *c, int kind) {
+int timer_begin(ghost_ctx *c, int kind) {
   if (!c->timers_on) return -1;
   ghost_ctx::Pending p{kind, take_event(c), take_event(c)};
   cudaEventRecord(p.a, c->stream);
   c->ev_pending.push_back(p);
   return (int)c->ev_pending.size() - 1;
 }
-static void timer_end(ghost_ctx *c, int slot) {
+void timer_end(ghost_ctx *c, int slot) {
   if (slot >= 0) cudaEventRecord(c->ev_pending[slot].b, c->stream);
 }
 static int timers_collect(ghost_ctx *c) {
@@ -1185,61 +1185,6 @@ int advect3_dev(ghost_ctx *c, const void *a, const void *b, const void *cc, cons
   return launch_z<R>(c, zf);
 }
 
-// ---------------------------------------------------------------------
-// reductions
-template <typename R>
-int reduce_dev(ghost_ctx *c, int kind, const void *a, const void *b, const void *cc, const void *d, const void *e,
-               const void *f, double *out_host) {
-  const size_t n = c->ntot;
-  const int nb = grid1d(n);
-  double *part;
-  GB_CHECK(partials(c, (size_t)nb + 1, &part));
-  RedArgs<R> ra{(const cx<R> *)a, (const cx<R> *)b, (const cx<R> *)cc, (const cx<R> *)d, (const cx<R> *)e,
-                (const cx<R> *)f};
-  const int ts = timer_begin(c, GHOST_TIMER_REDUCE);
-  reduce_kernel<R><<<nb, 256, 0, c->stream>>>(kparams<R>(c), ra, kind, n, part);
-  GB_CHECK(post_launch(c));
-  finalize_kernel<<<1, 256, 0, c->stream>>>(part, nb, 1, part + nb);
-  timer_end(c, ts);
-  GB_CHECK(post_launch(c));
-  GB_CUDA(cudaMemcpyAsync(out_host, part + nb, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-  GB_CUDA(cudaStreamSynchronize(c->stream));
-  return check_status(c);
-}
-
-// Shell-binned sums of a reduction term over two field triplets (the
-// transfer spectra of entrans / heltrans); spectrum_dev is its one-triplet form.
-// rnd is the shell rounding: GHOST's spectra add the default-REAL literal
-// .501 (0.501f), spectrscc adds shift + .501 in GP
-template <typename R>
-int spectrum6_dev(ghost_ctx *c, int kind, const void *a, const void *b, const void *cc, const void *d, const void *e,
-                  const void *f, double *out_host, R rnd = (R)0.501f) {
-  const size_t n = c->ntot;
-  const int nbins = c->nmax / 2 + 1;
-  const int nblk = std::min(grid1d(n), 148 * 4);
-  double *part;
-  GB_CHECK(partials(c, (size_t)(nblk + 1) * nbins, &part));
-  RedArgs<R> ra{(const cx<R> *)a, (const cx<R> *)b, (const cx<R> *)cc, (const cx<R> *)d, (const cx<R> *)e,
-                (const cx<R> *)f};
-  const size_t smem = (size_t)(256 / 32) * nbins * sizeof(double);
-  GB_CUDA(cudaFuncSetAttribute(spectrum_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int ts = timer_begin(c, GHOST_TIMER_REDUCE);
-  spectrum_kernel<R><<<nblk, 256, smem, c->stream>>>(kparams<R>(c), ra, kind, n, nbins, (R)c->Dkk, rnd, part);
-  GB_CHECK(post_launch(c));
-  double *fin = part + (size_t)nblk * nbins;
-  finalize_kernel<<<1, 256, 0, c->stream>>>(part, nblk, nbins, fin);
-  timer_end(c, ts);
-  GB_CHECK(post_launch(c));
-  GB_CUDA(cudaMemcpyAsync(out_host, fin, sizeof(double) * nbins, cudaMemcpyDeviceToHost, c->stream));
-  GB_CUDA(cudaStreamSynchronize(c->stream));
-  return GHOST_OK;
-}
-
-template <typename R>
-int spectrum_dev(ghost_ctx *c, int kind, const void *a, const void *b, const void *cc, double *out_host) {
-  return spectrum6_dev<R>(c, kind, a, b, cc, nullptr, nullptr, nullptr, out_host);
-}
-
 // Anisotropic sums (aniso_kernel): out_host[3 nb] = total, horizontal, vertical.
 template <typename R>
 int aniso_dev(ghost_ctx *c, int kind, int mode, int nb, const void *a, const void *b, const void *cc, const void *d,
@@ -1258,32 +1203,11 @@ int aniso_dev(ghost_ctx *c, int kind, int mode, int nb, const void *a, const voi
   aniso_kernel<R><<<nblk, 256, smem, c->stream>>>(kparams<R>(c), ra, kind, mode, n, nb, (R)c->Lz, (R)c->Dkk, part);
   GB_CHECK(post_launch(c));
   double *fin = part + (size_t)nblk * nb3;
-  finalize_kernel<<<1, 256, 0, c->stream>>>(part, nblk, nb3, fin);
+  GB_CHECK(finalize_dev(c, part, nblk, nb3, fin));
   timer_end(c, ts);
-  GB_CHECK(post_launch(c));
   GB_CUDA(cudaMemcpyAsync(out_host, fin, sizeof(double) * nb3, cudaMemcpyDeviceToHost, c->stream));
   GB_CUDA(cudaStreamSynchronize(c->stream));
   return check_status(c);
-}
-
-// The same shell spectrum left on the device (out_dev[nmax/2+1]); no
-// synchronisation, for closures that consume it in later kernels.
-template <typename R>
-int spectrum_dev_async(ghost_ctx *c, int kind, const void *a, const void *b, const void *cc, double *out_dev) {
-  const size_t n = c->ntot;
-  const int nbins = c->nmax / 2 + 1;
-  const int nblk = std::min(grid1d(n), 148 * 4);
-  double *part;
-  GB_CHECK(partials(c, (size_t)nblk * nbins, &part));
-  RedArgs<R> ra{(const cx<R> *)a, (const cx<R> *)b, (const cx<R> *)cc, nullptr, nullptr, nullptr};
-  const size_t smem = (size_t)(256 / 32) * nbins * sizeof(double);
-  GB_CUDA(cudaFuncSetAttribute(spectrum_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int ts = timer_begin(c, GHOST_TIMER_REDUCE);
-  spectrum_kernel<R><<<nblk, 256, smem, c->stream>>>(kparams<R>(c), ra, kind, n, nbins, (R)c->Dkk, (R)0.501f, part);
-  GB_CHECK(post_launch(c));
-  finalize_kernel<<<1, 256, 0, c->stream>>>(part, nblk, nbins, out_dev);
-  timer_end(c, ts);
-  return post_launch(c);
 }
 
 // twiddles exp(-2 pi i e/n), e < n, evaluated in extended precision and
@@ -1493,9 +1417,8 @@ int batch_reduce_dev(ghost_ctx *c, int kind, const void *a, const void *b, const
   reduce_runs_kernel<R><<<dim3(nb, c->nruns), 256, 0, c->stream>>>(kparams<R>(c), ra, kind, c->nspec, c->nruns, part);
   GB_CHECK(post_launch(c));
   double *fin = part + (size_t)nb * c->nruns;
-  finalize_kernel<<<1, 256, 0, c->stream>>>(part, nb, c->nruns, fin);
+  GB_CHECK(finalize_dev(c, part, nb, c->nruns, fin));
   timer_end(c, ts);
-  GB_CHECK(post_launch(c));
   GB_CUDA(cudaMemcpyAsync(out_host, fin, sizeof(double) * c->nruns, cudaMemcpyDeviceToHost, c->stream));
   GB_CUDA(cudaStreamSynchronize(c->stream));
   return check_status(c);
@@ -1541,11 +1464,7 @@ int batch_init_random_dev(ghost_ctx *c, const int32_t *seeds, int32_t *seeds_out
   template int r2c6_dev<R>(ghost_ctx *, const void *const[6], void *const[6]);                                 \
   template int grad9_features_dev<R>(ghost_ctx *, const void *const[3], void *const[9], float *, float, float);     \
   template int hd_substep_dev<R>(ghost_ctx *, int, double, double, void *const[3], void *const[3],             \
-                                 const void *const[3], int, bool);                                             \
-  template int spectrum_dev<R>(ghost_ctx *, int, const void *, const void *, const void *, double *);          \
-  template int reduce_dev<R>(ghost_ctx *, int, const void *, const void *, const void *, const void *,         \
-                             const void *, const void *, double *);                                            \
-  template int spectrum_dev_async<R>(ghost_ctx *, int, const void *, const void *, const void *, double *);
+                                 const void *const[3], int, bool);
 GB_INST(float)
 GB_INST(double)
 #undef GB_INST
@@ -1945,14 +1864,14 @@ int ghost_spectrumc(ghost_ctx *c, const void *a, const void *b, const void *cc, 
   GB_CHECK(st.map(a, c->cbytes, 1, &da));
   GB_CHECK(st.map(b, c->cbytes, 1, &db));
   GB_CHECK(st.map(cc, c->cbytes, 1, &dc));
-  const bool sp = c->precision == GHOST_SINGLE;
-  if (kin <= 1) {
-    const int kind = kin == 1 ? RED_ENERGY : RED_ENSTROPHY;
-    GB_CHECK(sp ? spectrum_dev<float>(c, kind, da, db, dc, Ek) : spectrum_dev<double>(c, kind, da, db, dc, Ek));
-  }
-  if (hel == 1)
-    GB_CHECK(sp ? spectrum_dev<float>(c, RED_HELICITY, da, db, dc, Hk)
-                : spectrum_dev<double>(c, RED_HELICITY, da, db, dc, Hk));
+  unsigned mask = kin == 1 ? 1u << RED_ENERGY : (kin == 0 ? 1u << RED_ENSTROPHY : 0u);
+  double *out[2] = {Ek, Hk};
+  double *const *o = kin <= 1 ? out : out + 1;
+  if (hel == 1) mask |= 1u << RED_HELICITY;
+  if (mask)
+    GB_CHECK(c->precision == GHOST_SINGLE
+                 ? shells_host<float>(c, mask, da, db, dc, nullptr, nullptr, nullptr, o, 0.501f)
+                 : shells_host<double>(c, mask, da, db, dc, nullptr, nullptr, nullptr, o, (double)0.501f));
   return st.finish();
 }
 
@@ -1971,8 +1890,9 @@ static int transfer(ghost_ctx *c, int kind, const void *a, const void *b, const 
   GB_CHECK(st.map(d, c->cbytes, 1, &dd));
   GB_CHECK(st.map(e, c->cbytes, 1, &de));
   GB_CHECK(st.map(f, c->cbytes, 1, &df));
-  GB_CHECK(c->precision == GHOST_SINGLE ? spectrum6_dev<float>(c, kind, da, db, dc, dd, de, df, out)
-                                        : spectrum6_dev<double>(c, kind, da, db, dc, dd, de, df, out));
+  GB_CHECK(c->precision == GHOST_SINGLE
+               ? shells_host<float>(c, 1u << kind, da, db, dc, dd, de, df, &out, 0.501f)
+               : shells_host<double>(c, 1u << kind, da, db, dc, dd, de, df, &out, (double)0.501f));
   return st.finish();
 }
 
@@ -2237,8 +2157,8 @@ int ghost_spectrscc(ghost_ctx *c, const void *a, double shift, double *Ek) {
   GB_CHECK(st.map(a, c->cbytes, 1, &da));
   // round = shift + .501_GP (a GP literal here, unlike spectrumc's default REAL)
   GB_CHECK(c->precision == GHOST_SINGLE
-               ? spectrum6_dev<float>(c, RED_SC_VAR, da, da, da, da, da, da, Ek, (float)shift + 0.501f)
-               : spectrum6_dev<double>(c, RED_SC_VAR, da, da, da, da, da, da, Ek, shift + 0.501));
+               ? shells_host<float>(c, 1u << RED_SC_VAR, da, da, da, da, da, da, &Ek, (float)shift + 0.501f)
+               : shells_host<double>(c, 1u << RED_SC_VAR, da, da, da, da, da, da, &Ek, shift + 0.501));
   return st.finish();
 }
 
@@ -2250,8 +2170,9 @@ int ghost_sctrans(ghost_ctx *c, const void *a, const void *b, int isc, double *E
   const void *da, *db;
   GB_CHECK(st.map(a, c->cbytes, 1, &da));
   GB_CHECK(st.map(b, c->cbytes, 1, &db));
-  GB_CHECK(c->precision == GHOST_SINGLE ? spectrum6_dev<float>(c, RED_SC_CROSS, da, da, da, db, db, db, Ek)
-                                        : spectrum6_dev<double>(c, RED_SC_CROSS, da, da, da, db, db, db, Ek));
+  GB_CHECK(c->precision == GHOST_SINGLE
+               ? shells_host<float>(c, 1u << RED_SC_CROSS, da, da, da, db, db, db, &Ek, 0.501f)
+               : shells_host<double>(c, 1u << RED_SC_CROSS, da, da, da, db, db, db, &Ek, (double)0.501f));
   return st.finish();
 }
 
@@ -2503,16 +2424,15 @@ int ghost_hdcheck(ghost_ctx *c, const void *vx, const void *vy, const void *vz, 
   GB_CHECK(st.map(fx, c->cbytes, 1, &d));
   GB_CHECK(st.map(fy, c->cbytes, 1, &e));
   GB_CHECK(st.map(fz, c->cbytes, 1, &f));
-  const bool sp = c->precision == GHOST_SINGLE;
-  auto red = [&](int kind, const void *p, const void *q, const void *r, double *o) {
-    return sp ? reduce_dev<float>(c, kind, a, b, cc, p, q, r, o) : reduce_dev<double>(c, kind, a, b, cc, p, q, r, o);
-  };
-  for (int q = 0; q < 5; ++q) out[q] = 0.0;
-  GB_CHECK(red(RED_ENERGY, nullptr, nullptr, nullptr, &out[0]));
-  GB_CHECK(red(RED_ENSTROPHY, nullptr, nullptr, nullptr, &out[1]));
-  if (hel == 1) GB_CHECK(red(RED_HELICITY, nullptr, nullptr, nullptr, &out[2]));
-  GB_CHECK(red(RED_CROSS, d, e, f, &out[3]));
-  if (chk == 1) GB_CHECK(red(RED_DIVERGENCE, nullptr, nullptr, nullptr, &out[4]));
+  // ascending kinds: energy, enstrophy, helicity, cross, divergence
+  unsigned mask = 1u << RED_ENERGY | 1u << RED_ENSTROPHY | 1u << RED_CROSS;
+  if (hel == 1) mask |= 1u << RED_HELICITY;
+  if (chk == 1) mask |= 1u << RED_DIVERGENCE;
+  double got[5];
+  GB_CHECK(c->precision == GHOST_SINGLE ? sums_dev<float>(c, mask, a, b, cc, d, e, f, got)
+                                        : sums_dev<double>(c, mask, a, b, cc, d, e, f, got));
+  int n = 0;
+  for (int q = 0; q < 5; ++q) out[q] = (q == 2 && hel != 1) || (q == 4 && chk != 1) ? 0.0 : got[n++];
   return st.finish();
 }
 
@@ -2837,15 +2757,12 @@ int ghost_bouss_run(ghost_ctx *c, int nsteps, int ord, double dt, double nu, dou
 // ------------------------------------------------- no-allocation spectrum
 // Partial sums of ghost_spectrumc_noalloc: nblk blocks write one
 // histogram row of nbins each, then the final row follows them; nblk is
-// chosen per call so that the (nblk + 1) rows fit the static array.  Every
+// capped so that the (nblk + 1) rows fit the static array.  Every
 // slot a call reads was written earlier by that same call, so nothing needs
 // clearing between calls.
 static_assert(2 * GHOST_SPECTRUM_NOALLOC_MAX_BINS <= GHOST_SPECTRUM_NOALLOC_DOUBLES,
               "static spectrum scratch too small for the advertised shell count");
-static int noalloc_blocks(size_t n, int nbins) {
-  const int fit = GHOST_SPECTRUM_NOALLOC_DOUBLES / nbins - 1;  // rows left after the final one
-  return std::max(1, std::min(std::min(grid1d(n), 148 * 4), fit));
-}
+static int noalloc_blocks(int nbins) { return GHOST_SPECTRUM_NOALLOC_DOUBLES / nbins - 1; }  // rows left after the final one
 static __device__ __align__(256) double g_spectrum_scratch[GHOST_SPECTRUM_NOALLOC_DOUBLES];
 
 static std::mutex g_spectrum_scratch_mu;
@@ -2875,22 +2792,9 @@ static int spectrum_scratch_address(int dev, double **out) {
 template <typename R>
 static int spectrum_noalloc_dev(ghost_ctx *c, double *scratch, int kind, const void *a, const void *b, const void *cc,
                                 double *out_host) {
-  const int nbins = c->nmax / 2 + 1;
   // every run of a batched context, as ghost_spectrumc sums them
-  const size_t n = c->ntot;
-  const int nblk = noalloc_blocks(n, nbins);
-  RedArgs<R> ra{(const cx<R> *)a, (const cx<R> *)b, (const cx<R> *)cc, nullptr, nullptr, nullptr};
-  const size_t smem = (size_t)(256 / 32) * nbins * sizeof(double);
-  GB_CUDA(cudaFuncSetAttribute(spectrum_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  spectrum_kernel<R><<<nblk, 256, smem, c->stream>>>(kparams<R>(c), ra, kind, n, nbins, (R)c->Dkk, (R)0.501f,
-                                                     scratch);
-  GB_CHECK(post_launch(c));
-  double *fin = scratch + (size_t)nblk * nbins;
-  finalize_kernel<<<1, 256, 0, c->stream>>>(scratch, nblk, nbins, fin);
-  GB_CHECK(post_launch(c));
-  GB_CUDA(cudaMemcpyAsync(out_host, fin, sizeof(double) * nbins, cudaMemcpyDeviceToHost, c->stream));
-  GB_CUDA(cudaStreamSynchronize(c->stream));
-  return GHOST_OK;
+  return shells_host<R>(c, 1u << kind, a, b, cc, nullptr, nullptr, nullptr, &out_host, (R)0.501f, scratch,
+                        noalloc_blocks(c->nmax / 2 + 1));
 }
 
 extern "C" {

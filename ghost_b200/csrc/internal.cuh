@@ -30,16 +30,29 @@ template <typename R> int r2c6_dev(ghost_ctx *c, const void *const in[6], void *
 template <typename R>
 int hd_substep_dev(ghost_ctx *c, int o, double dt, double nu, void *const v[3], void *const C[3], const void *const f[3],
                    int copy, bool prune = false);
-// reductions of ops.cuh (kind 0: <|v|^2>) into one host double
+// FP64 partial sums owned by the context, grown on demand
+int partials(ghost_ctx *c, size_t n, double **out);
+// per-kernel timers around a launch (kind GHOST_TIMER_*)
+int timer_begin(ghost_ctx *c, int kind);
+void timer_end(ghost_ctx *c, int slot);
+// out[b] = sum over q < nparts of part[q][b], in a fixed order
+int finalize_dev(ghost_ctx *c, const double *part, int nparts, int nbins, double *out);
+// reductions (reduce.cu; kinds of ops.cuh, kind 0: <|v|^2>) into host doubles:
+// one kind, or the kinds of a mask in one pass over the fields
 template <typename R>
 int reduce_dev(ghost_ctx *c, int kind, const void *a, const void *b, const void *cc, const void *d, const void *e,
                const void *f, double *out_host);
-// kinetic (kind 1) shell spectrum into out_host[nmax/2+1]
 template <typename R>
-int spectrum_dev(ghost_ctx *c, int kind, const void *a, const void *b, const void *cc, double *out_host);
-// the same into a device array, without synchronising
+int sums_dev(ghost_ctx *c, unsigned mask, const void *a, const void *b, const void *cc, const void *d, const void *e,
+             const void *f, double *out_host);
+// shell spectra of the kinds of a mask, on the device without synchronising
+// (shells_dev) or into host arrays
 template <typename R>
-int spectrum_dev_async(ghost_ctx *c, int kind, const void *a, const void *b, const void *cc, double *out_dev);
+int shells_dev(ghost_ctx *c, unsigned mask, const void *a, const void *b, const void *cc, const void *d, const void *e,
+               const void *f, double *out_dev, R rnd, double *part = nullptr, int maxblk = 0, double **fin = nullptr);
+template <typename R>
+int shells_host(ghost_ctx *c, unsigned mask, const void *a, const void *b, const void *cc, const void *d, const void *e,
+                const void *f, double *const *out_host, R rnd, double *part = nullptr, int maxblk = 0);
 
 }  // namespace gb
 

@@ -1045,8 +1045,8 @@ static int eddy_force_dev(ghost_les *L, const void *const v[3], const void *cons
   ghost_ctx *c = L->c;
   const int nb = c->nx / 2 + 1;
   const int hel = L->heli;
-  GB_CHECK(spectrum_dev_async<R>(c, RED_ENERGY_KIND, v[0], v[1], v[2], L->Ek_dev));
-  if (hel == 1) GB_CHECK(spectrum_dev_async<R>(c, RED_HELICITY_KIND, v[0], v[1], v[2], L->Hk_dev));
+  GB_CHECK(shells_dev<R>(c, 1u << RED_ENERGY_KIND, v[0], v[1], v[2], nullptr, nullptr, nullptr, L->Ek_dev, (R)0.501f));
+  if (hel == 1) GB_CHECK(shells_dev<R>(c, 1u << RED_HELICITY_KIND, v[0], v[1], v[2], nullptr, nullptr, nullptr, L->Hk_dev, (R)0.501f));
   edqnm_fit_kernel<R><<<1, 128, 0, c->stream>>>(c->nx, (R)c->kmax, (R)L->kolmo, L->Ek_dev, L->Hk_dev, hel,
                                                 L->tepq_dev, L->thpq_dev, L->tve_dev, L->tvh_dev, L->Ext_dev,
                                                 L->Hxt_dev, (R *)L->mu_dev, L->go_dev);
@@ -1074,7 +1074,7 @@ template <typename R>
 static int spectral_force_dev(ghost_les *L, const void *const v[3], const void *const f[3], void *const o[3]) {
   ghost_ctx *c = L->c;
   const int nb = c->nx / 2 + 1;
-  GB_CHECK(spectrum_dev_async<R>(c, RED_ENERGY_KIND, v[0], v[1], v[2], L->Ek_dev));
+  GB_CHECK(shells_dev<R>(c, 1u << RED_ENERGY_KIND, v[0], v[1], v[2], nullptr, nullptr, nullptr, L->Ek_dev, (R)0.501f));
   spec_features_kernel<<<1, 64, 0, c->stream>>>(L->Ek_dev, L->kc, L->x);
   GB_CHECK(post_launch(c));
   GB_CHECK(ghost_mlp_set_stream(L->mlp, c->stream));

@@ -127,10 +127,15 @@ template <typename R> struct RedArgs {
   const cx<R> *a, *b, *c, *d, *e, *f;
 };
 
+// the values of one mode of up to six fields
+template <typename R> struct RedVals {
+  cx<R> a, b, c, d, e, f;
+};
+
 template <typename R>
-__device__ __forceinline__ R red_term(const KParams<R> &kp, const RedArgs<R> &ra, int kind, size_t p, int i, int j, int k) {
+__device__ __forceinline__ R red_value(const KParams<R> &kp, const RedVals<R> &x, int kind, int i, int j, int k) {
   using C = cx<R>;
-  const C va = ra.a[p], vb = ra.b[p], vc = ra.c[p];
+  const C va = x.a, vb = x.b, vc = x.c;
   switch (kind) {
     case RED_ENERGY:
       return (va.x * va.x + va.y * va.y + vb.x * vb.x + vb.y * vb.y + vc.x * vc.x + vc.y * vc.y) * kp.tmp;
@@ -151,13 +156,13 @@ __device__ __forceinline__ R red_term(const KParams<R> &kp, const RedArgs<R> &ra
     }
     case RED_CROSS:
     case RED_CROSS_K2: {
-      const C vd = ra.d[p], ve = ra.e[p], vf = ra.f[p];
+      const C vd = x.d, ve = x.e, vf = x.f;
       R s = cmulc(va, vd).x + cmulc(vb, ve).x + cmulc(vc, vf).x;
       if (kind == RED_CROSS_K2) s = s * kk2_of(kp, i, j, k);
       return s * kp.tmp;
     }
     case RED_SC_CROSS: {  // sctrans: Re(a conj(d)) of two scalars
-      const C vd = ra.d[p];
+      const C vd = x.d;
       return cmulc(va, vd).x * kp.tmp;
     }
     case RED_SC_VAR:  // variance / spectrscc: |a|^2
@@ -167,7 +172,7 @@ __device__ __forceinline__ R red_term(const KParams<R> &kp, const RedArgs<R> &ra
     case RED_CURL_CROSS: {  // heltrans: Re(curl(a,b,c) . conj(d,e,f))
       const C w1 = curl_at(kp, 1, i, j, k, va, vb, vc), w2 = curl_at(kp, 2, i, j, k, va, vb, vc),
               w3 = curl_at(kp, 3, i, j, k, va, vb, vc);
-      const C vd = ra.d[p], ve = ra.e[p], vf = ra.f[p];
+      const C vd = x.d, ve = x.e, vf = x.f;
       return (cmulc(w1, vd).x + cmulc(w2, ve).x + cmulc(w3, vf).x) * kp.tmp;
     }
     default: {  // RED_DIVERGENCE
@@ -175,6 +180,20 @@ __device__ __forceinline__ R red_term(const KParams<R> &kp, const RedArgs<R> &ra
       return (s.x * s.x + s.y * s.y) * kp.tmp;
     }
   }
+}
+
+template <typename R>
+__device__ __forceinline__ R red_term(const KParams<R> &kp, const RedArgs<R> &ra, int kind, size_t p, int i, int j, int k) {
+  RedVals<R> x{};
+  x.a = ra.a[p];
+  x.b = ra.b[p];
+  x.c = ra.c[p];
+  if (kind == RED_CROSS || kind == RED_CROSS_K2 || kind == RED_CURL_CROSS || kind == RED_SC_CROSS) x.d = ra.d[p];
+  if (kind == RED_CROSS || kind == RED_CROSS_K2 || kind == RED_CURL_CROSS) {
+    x.e = ra.e[p];
+    x.f = ra.f[p];
+  }
+  return red_value(kp, x, kind, i, j, k);
 }
 
 __device__ __forceinline__ double block_sum(double v, double *sh) {
@@ -189,22 +208,8 @@ __device__ __forceinline__ double block_sum(double v, double *sh) {
   return s;
 }
 
-template <typename R>
-__global__ void __launch_bounds__(256) reduce_kernel(KParams<R> kp, RedArgs<R> ra, int kind, size_t n, double *partials) {
-  __shared__ double sh[32];
-  double acc = 0.0;
-  for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x) {
-    int i, j, k;
-    unflat(kp, p, i, j, k);
-    const double w = i == 0 ? 1.0 : 2.0;
-    acc += w * (double)red_term(kp, ra, kind, p, i, j, k);
-  }
-  const double s = block_sum(acc, sh);
-  if (threadIdx.x == 0) partials[blockIdx.x] = s;
-}
-
 // Per-run sums of a batched field: block (x, run) covers run `run`;
-// partials laid out [block][run] for finalize_kernel.
+// partials laid out [block][run].
 template <typename R>
 __global__ void __launch_bounds__(256) reduce_runs_kernel(KParams<R> kp, RedArgs<R> ra, int kind, size_t nspec,
                                                           int nruns, double *partials) {
@@ -236,21 +241,6 @@ __global__ void scale3_runs_kernel(cx<R> *x, cx<R> *y, cx<R> *z, size_t nspec, i
   }
 }
 
-// Sums nparts partials in a fixed order (one block).  Also used for the
-// per-bin spectrum partials with stride.
-__global__ void __launch_bounds__(256) finalize_kernel(const double *partials, int nparts, int nbins, double *out) {
-  __shared__ double sh[32];
-  for (int b = 0; b < nbins; ++b) {
-    double acc = 0.0;
-    for (int q = threadIdx.x; q < nparts; q += blockDim.x) acc += partials[(size_t)q * nbins + b];
-    const double s = block_sum(acc, sh);
-    if (threadIdx.x == 0) out[b] = s;
-  }
-}
-
-// Shell spectra (spectrumc, pseudospec3D_hd.f90:1190-1415).  Each warp
-// owns a shared histogram; lanes add in lane order, warps are combined in
-// warp order, blocks in block order: reproducible bit for bit.
 // One warp's contribution to a shared-memory histogram: every lane with
 // bin >= 0 adds its NV values to hw[bin + q * stride].  Lanes that share a bin
 // are summed in lane order through shuffles and the group's lowest lane adds
@@ -276,42 +266,6 @@ __device__ __forceinline__ void warp_bin_add(double *hw, int stride, int bin, co
     for (int q = 0; q < NV; ++q) hw[(size_t)q * stride + bin] += s[q];
   }
   __syncwarp();
-}
-
-template <typename R>
-__global__ void __launch_bounds__(256) spectrum_kernel(KParams<R> kp, RedArgs<R> ra, int kind, size_t n, int nb,
-                                                       R Dkk, R rnd, double *partials) {
-  extern __shared__ double hist[];  // (blockDim/32) * nb
-  const int nw = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int q = threadIdx.x; q < nw * nb; q += blockDim.x) hist[q] = 0.0;
-  __syncthreads();
-  double *hw = hist + (size_t)w * nb;
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
-  const size_t start = blockIdx.x * (size_t)blockDim.x + (size_t)w * 32;
-  for (size_t base = start; base < n; base += stride) {
-    const size_t p = base + lane;
-    int bin = -1;
-    double val = 0.0;
-    if (p < n) {
-      int i, j, k;
-      unflat(kp, p, i, j, k);
-      const R kk2 = kk2_of(kp, i, j, k);
-      const int kmn = (int)(sqrt(kk2) / Dkk + rnd);  // rnd: .501 rounding of the caller's GHOST routine
-      if (kmn > 0 && kmn <= nb) {
-        const R wgt = i == 0 ? (R)1 : (R)2;
-        bin = kmn - 1;
-        val = (double)(wgt * red_term(kp, ra, kind, p, i, j, k));
-      }
-    }
-    const double vals[1] = {val};
-    warp_bin_add<1>(hw, nb, bin, vals, lane);
-  }
-  __syncthreads();
-  for (int b = threadIdx.x; b < nb; b += blockDim.x) {
-    double s = 0.0;
-    for (int q = 0; q < nw; ++q) s += hist[(size_t)q * nb + b];
-    partials[(size_t)blockIdx.x * nb + b] = s;
-  }
 }
 
 // Anisotropic spectra (pseudospec3D_rot.f90): mode 0 bins by |kz|
