@@ -476,35 +476,14 @@ static int timers_collect(ghost_ctx *c) {
   return GHOST_OK;
 }
 
-template <class Op> struct ZKind;
-template <typename R, int S, int NF> struct ZKind<ZC2C<R, S, NF>> { static constexpr int value = GHOST_TIMER_Z_C2C; };
-template <typename R, int P> struct ZKind<ZInv<R, P>> { static constexpr int value = GHOST_TIMER_Z_INV; };
-template <typename R> struct ZKind<ZGrad<R>> { static constexpr int value = GHOST_TIMER_Z_INV; };
-template <typename R> struct ZKind<ZFwdHD<R>> { static constexpr int value = GHOST_TIMER_Z_FWD; };
-template <typename R> struct ZKind<ZFwdBouss<R>> { static constexpr int value = GHOST_TIMER_Z_FWD; };
-
 int grid1d(size_t n) {
   size_t b = (n + 255) / 256;
   return (int)std::min<size_t>(b, 148 * 16);
 }
 
 // ---------------------------------------------------------------------
-// pass launchers
-template <typename R> constexpr int xE() { return sizeof(R) == 4 ? 8 : 4; }
-template <typename R> constexpr int xBZ() { return sizeof(R) == 4 ? 8 : 4; }
-
-// Pruning state for one substep: null tables = every line.
-struct Prune {
-  const int *lines = nullptr;
-  int nlines = 0;
-  const int *jpos = nullptr, *jneg = nullptr;
-  int ni = 0;    // kx indices processed by the y passes
-  int rows = 0;  // kx rows present in / written by the x pass
-};
-
-template <typename R> constexpr int zE() { return sizeof(R) == 4 ? 8 : 4; }
-
-static int sm_count(ghost_ctx *c) {
+// pass launchers (passes_z.cu, passes_y.cu, passes_x.cu)
+int sm_count(ghost_ctx *c) {
   if (c->num_sms <= 0) {
     int n = 0;
     cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, c->device);
@@ -513,23 +492,13 @@ static int sm_count(ghost_ctx *c) {
   return c->num_sms;
 }
 
-// Persistent grid: as many CTAs as fit on the device at once, or fewer
-// when there are fewer tiles.
-template <class K> static int persistent_grid(ghost_ctx *c, K kern, int threads, size_t smem, long ntiles) {
-  int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
-  if (per_sm < 1) per_sm = 1;
-  const long g = (long)per_sm * sm_count(c);
-  return (int)std::max<long>(1, std::min<long>(g, ntiles));
-}
-
 // ---------------------------------------------------------------------
 // TMA tensor maps of spectral fields: a 3D tensor (z in 8-byte units, y,
 // kx) over one field, with the box the pass loads.
 static PFN_cuTensorMapEncodeTiled_v12000 g_encode_tiled = nullptr;
 static std::mutex g_encode_mu;
 
-static int encode_fn(PFN_cuTensorMapEncodeTiled_v12000 *fn) {
+int encode_fn(PFN_cuTensorMapEncodeTiled_v12000 *fn) {
   std::lock_guard<std::mutex> lock(g_encode_mu);
   if (!g_encode_tiled) {
     void *p = nullptr;
@@ -545,8 +514,8 @@ static int encode_fn(PFN_cuTensorMapEncodeTiled_v12000 *fn) {
   return GHOST_OK;
 }
 
-static int field_map(ghost_ctx *c, const void *base, unsigned box0, unsigned box1, unsigned box2, CUtensorMap *out,
-                     CUtensorMapSwizzle swz = CU_TENSOR_MAP_SWIZZLE_NONE) {
+int field_map(ghost_ctx *c, const void *base, unsigned box0, unsigned box1, unsigned box2, CUtensorMap *out,
+              CUtensorMapSwizzle swz) {
   PFN_cuTensorMapEncodeTiled_v12000 enc;
   GB_CHECK(encode_fn(&enc));
   const cuuint64_t U = c->precision == GHOST_SINGLE ? 1 : 2;
@@ -561,308 +530,7 @@ static int field_map(ghost_ctx *c, const void *base, unsigned box0, unsigned box
   return GHOST_OK;
 }
 
-static PipeCtl pipe_ctl(ghost_ctx *c) { return PipeCtl{c->status, c->wait_cap, c->inject_stall}; }
-
-template <typename R, int N, int LPB, int STAGES0, int MINB, class Op>
-int launch_z_cfg(ghost_ctx *c, const Op &op, const Prune &pr) {
-  constexpr int E = zE<R>() < N ? zE<R>() : N, T = N / E;
-  using G = ZGeom<R, N, E, LPB, Op::NLOAD>;
-  constexpr int STAGES = G::smem_bytes(STAGES0) <= 200 * 1024 ? STAGES0 : 2;
-  const size_t smem = G::smem_bytes(STAGES);
-  const int nlines = pr.lines ? pr.nlines : c->ny * c->nxh * c->nruns;
-  auto kern = zpipe_kernel<R, N, E, LPB, STAGES, MINB, Op>;
-  GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int grid = persistent_grid(c, kern, LPB * T, smem, (nlines + LPB - 1) / LPB);
-  const int ts = timer_begin(c, ZKind<Op>::value);
-  kern<<<grid, LPB * T, smem, c->stream>>>(op, (const cx<R> *)c->tw_z, pr.lines, nlines, pipe_ctl(c));
-  timer_end(c, ts);
-  return post_launch(c);
-}
-
-// CTAs of 256 threads; with tile variant bit 1 of 128 threads; with bits 1
-// and 2 of 128 threads with a two-stage ring and at most 170 registers, so
-// that three CTAs share an SM (lines of 256 points or more)
-// lines per CTA, halved from want until a two-stage ring of NL fields fits
-template <typename R, int N, int NL> constexpr int fit_lines(int want) {
-  int lpb = want;
-  while (lpb > 1 && ((size_t)2 * NL * lpb * N + N + (size_t)2 * lpb * (N + N / 8)) * sizeof(cx<R>) + 24 > 220 * 1024)
-    lpb /= 2;
-  return lpb;
-}
-
-template <typename R, int N, class Op> int launch_z_n(ghost_ctx *c, const Op &op, const Prune &pr) {
-  constexpr int E = zE<R>() < N ? zE<R>() : N, T = N / E;
-  constexpr int L256 = fit_lines<R, N, Op::NLOAD>(256 / T > 0 ? 256 / T : 1);
-  constexpr int L128 = fit_lines<R, N, Op::NLOAD>(128 / T > 0 ? 128 / T : 1);
-  if constexpr (N >= 256 && L128 != L256) {
-    if ((c->tile_cfg & 38) == 38) return launch_z_cfg<R, N, L128, 1, 4>(c, op, pr);
-    if ((c->tile_cfg & 6) == 6) return launch_z_cfg<R, N, L128, 2, 3>(c, op, pr);
-  }
-  if ((c->tile_cfg & 2) && L128 != L256) return launch_z_cfg<R, N, L128, 3, 1>(c, op, pr);
-  return launch_z_cfg<R, N, L256, 3, 1>(c, op, pr);
-}
-
-template <typename R, class Op> int launch_z(ghost_ctx *c, const Op &op, const Prune &pr = Prune()) {
-  switch (c->nz) {
-    case 16: return launch_z_n<R, 16>(c, op, pr);
-    case 32: return launch_z_n<R, 32>(c, op, pr);
-    case 64: return launch_z_n<R, 64>(c, op, pr);
-    case 128: return launch_z_n<R, 128>(c, op, pr);
-    case 256: return launch_z_n<R, 256>(c, op, pr);
-    case 512: return launch_z_n<R, 512>(c, op, pr);
-    case 1024: return launch_z_n<R, 1024>(c, op, pr);
-  }
-  return fail(GHOST_ERR_SIZE, "nz=%d unsupported", c->nz);
-}
-
-// y tile width: BZ0 z-lines, at most 1024 threads, narrowed until a
-// two-stage ring fits in shared memory (FP64 with 1024-point lines)
-template <typename R, int N, int BZ0> constexpr int y_tile_width() {
-  constexpr int E = N < 8 ? N : 8, T = N / E;
-  int bz = BZ0 * T <= 1024 ? BZ0 : 1024 / T;
-  while (bz > 1 && ((size_t)3 * bz * N + N) * sizeof(cx<R>) + 24 > 220 * 1024) bz /= 2;
-  return bz;
-}
-
-// kx indices per y tile: short lines put several kx in one tile so that a
-// CTA has at least 128 threads (not with the second exchange buffer)
-template <int N, int E, int BZ, bool DUAL> constexpr int y_kb() {
-  return (DUAL || BZ * (N / E) >= 128) ? 1 : 128 / (BZ * (N / E));
-}
-
-template <typename R, int N, int S, int BZ0, bool DUAL = false, int E0 = 8>
-int launch_y_cfg(ghost_ctx *c, const Fields<R> &f, int nf, const Prune &pr) {
-  constexpr int E = N < E0 ? N : E0, T = N / E;
-  constexpr int BZ = y_tile_width<R, N, BZ0>();
-  constexpr int KB = y_kb<N, E, BZ, DUAL>();
-  using G = YGeom<R, N, E, BZ, DUAL, KB>;
-  constexpr int STAGES = DUAL ? 2 : (G::smem_bytes(3) <= 200 * 1024 ? 3 : 2);
-  if (c->nz < BZ) return fail(GHOST_ERR_SIZE, "nz=%d below the y-pass tile width %d", c->nz, BZ);
-  const size_t smem = G::smem_bytes(STAGES);
-  auto kern = ypipe_kernel<R, N, E, BZ, STAGES, S, DUAL, KB>;
-  GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int ni = pr.jpos ? pr.ni : c->nxh;
-  const long ntiles = (long)(c->nz / BZ) * ((ni + KB - 1) / KB) * c->nruns * nf;
-  const int grid = persistent_grid(c, kern, KB * BZ * T, smem, ntiles);
-  // box rows: 32 (or N/2) for the pruned inverse, whole halves otherwise
-  const int rb = (pr.jpos && S > 0) ? std::min(32, N / 2) : std::min(N, 256);
-  // store boxes of the dual-buffer variant (TMA stores): whole halves for the
-  // inverse, 32 rows for the forward pass, whose pruned tiles store the live
-  // rows only; both divide N
-  const int rbo = S > 0 ? std::min(N, 256) : std::min(N, 32);
-  const unsigned U = sizeof(R) == 4 ? 1 : 2;
-  FieldMaps maps, omaps;
-  for (int q = 0; q < nf; ++q) GB_CHECK(field_map(c, f.p[q], BZ * U, rb, 1, &maps.m[q]));
-  if (DUAL)
-    for (int q = 0; q < nf; ++q) GB_CHECK(field_map(c, f.p[q], BZ * U, rbo, 1, &omaps.m[q]));
-  const int ts = timer_begin(c, S > 0 ? GHOST_TIMER_Y_INV : GHOST_TIMER_Y_FWD);
-  kern<<<grid, KB * BZ * T, smem, c->stream>>>(maps, DUAL ? omaps : maps, f, (const cx<R> *)c->tw_y, c->nz, ni, nf,
-                                          c->nruns, c->nxh, pr.jpos, pr.jneg, rb, rbo, pipe_ctl(c));
-  timer_end(c, ts);
-  return post_launch(c);
-}
-
-// tiles 8 z-lines wide, or 16 with tile variant bit 0
-template <typename R, int N, int S> int launch_y_n(ghost_ctx *c, const Fields<R> &f, int nf, const Prune &pr) {
-  // the 16-wide tile needs two stages of 16 lines in shared memory; where
-  // that does not fit (FP64, long lines) the variant falls back to 8
-  constexpr int E = N < 8 ? N : 8, T = N / E;
-  constexpr int BZ16 = 16 * T <= 1024 ? 16 : 1024 / T;
-  constexpr bool fits16 = YGeom<R, N, E, BZ16>::smem_bytes(2) <= 227 * 1024;
-  if constexpr (fits16) {
-    if ((c->tile_cfg & 1) && c->nz >= 16) return launch_y_cfg<R, N, S, 16>(c, f, nf, pr);
-  }
-  // bit 4 (FP32, lines of 256 points or more): 16 values per thread, two
-  // radix-8 butterflies per stage, half the threads per line
-  if constexpr (sizeof(R) == 4 && N >= 256) {
-    if (c->tile_cfg & 16) {
-      // bit 6 with bit 3: the inverse pass in tiles of 4 z-lines, four CTAs per SM
-      if constexpr (S > 0)
-        if ((c->tile_cfg & 72) == 72) return launch_y_cfg<R, N, S, 4, true, 16>(c, f, nf, pr);
-      if (c->tile_cfg & 8) return launch_y_cfg<R, N, S, 8, true, 16>(c, f, nf, pr);
-      return launch_y_cfg<R, N, S, 8, false, 16>(c, f, nf, pr);
-    }
-  }
-  // bit 3: two stages and a second exchange buffer (one barrier per exchange)
-  constexpr bool fits_dual = YGeom<R, N, E, 8, true>::smem_bytes(2) <= 113 * 1024;
-  if constexpr (N >= 256 && fits_dual) {
-    if (c->tile_cfg & 8) return launch_y_cfg<R, N, S, 8, true>(c, f, nf, pr);
-  }
-  return launch_y_cfg<R, N, S, 8>(c, f, nf, pr);
-}
-
-template <typename R, int S> int launch_y(ghost_ctx *c, const Fields<R> &f, int nf, const Prune &pr = Prune()) {
-  switch (c->ny) {
-    case 16: return launch_y_n<R, 16, S>(c, f, nf, pr);
-    case 32: return launch_y_n<R, 32, S>(c, f, nf, pr);
-    case 64: return launch_y_n<R, 64, S>(c, f, nf, pr);
-    case 128: return launch_y_n<R, 128, S>(c, f, nf, pr);
-    case 256: return launch_y_n<R, 256, S>(c, f, nf, pr);
-    case 512: return launch_y_n<R, 512, S>(c, f, nf, pr);
-    case 1024: return launch_y_n<R, 1024, S>(c, f, nf, pr);
-  }
-  return fail(GHOST_ERR_SIZE, "ny=%d unsupported", c->ny);
-}
-
-// X pass kinds
-enum XKind { X_HD = 0, X_C2R = 1, X_R2C = 2, X_BOUSS = 3 };
-
-// y rows per x tile: short lines put several y rows in one tile so that a
-// CTA has at least 128 threads
-template <typename R, int NX, int BZ> constexpr int x_yb() {
-  constexpr int E = xE<R>() < NX / 2 ? xE<R>() : NX / 2;
-  return BZ * (NX / 2 / E) >= 128 ? 1 : 128 / (BZ * (NX / 2 / E));
-}
-
-// The fused X pass with tiles of BZ z-values (MINB CTAs per SM).
-template <typename R, int NX, int KIND, int BZ, int MINB>
-int launch_x_fused(ghost_ctx *c, const void *const *ins, void *const *outs, int rows) {
-  constexpr int E = xE<R>() < NX / 2 ? xE<R>() : NX / 2;
-  constexpr int YB = x_yb<R, NX, BZ>();
-  if (c->ny % YB != 0) return fail(GHOST_ERR_SIZE, "ny=%d not a multiple of the x tile's %d rows", c->ny, YB);
-  constexpr int M = NX / 2, T = M / E, NT = YB * BZ * T;
-  typedef cx<R> C;
-  constexpr int PHYS = KIND == X_HD ? 0 : 1;
-  constexpr int NIN = PHYS == 0 ? 6 : 9, NOUT = PHYS == 0 ? 3 : 4;
-  using G = XGeom<R, NX, BZ, YB>;
-  constexpr size_t cap = 220 * 1024 / MINB;  // four stages while MINB CTAs fit an SM
-  constexpr int STAGES = G::smem_bytes(4) <= cap ? 4 : (G::smem_bytes(3) <= 200 * 1024 ? 3 : 2);
-  const size_t smem = G::smem_bytes(STAGES);
-  auto kern = xpipe_nl_kernel<R, NX, E, BZ, PHYS, STAGES, MINB, YB>;
-  GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  Fields<R> fo{};
-  for (int q = 0; q < NOUT; ++q) fo.p[q] = (C *)outs[q];
-  const R nn = (R)c->nx * (R)c->ny * (R)c->nz_glob;
-  const int nrows = rows > 0 ? rows : M + 1;
-  // tensor boxes: nbox boxes of rb kx-rows; rb keeps every box 128-byte aligned in shared memory
-  const int nbox = (nrows + 255) / 256;
-  const int align = std::max(1, 128 / (YB * BZ * (int)sizeof(C)));
-  const int rb = ((nrows + nbox - 1) / nbox + align - 1) / align * align;
-  if (nbox * rb > M + 8 || rb > 256) return fail(GHOST_ERR_STATE, "x-pass box plan %d x %d exceeds the tile", nbox, rb);
-  const unsigned U = sizeof(R) == 4 ? 1 : 2;
-  FieldMaps maps;
-  for (int q = 0; q < NIN; ++q) GB_CHECK(field_map(c, ins[q], BZ * U, YB, rb, &maps.m[q]));
-  const int pgrid = persistent_grid(c, kern, NT, smem, (long)(c->nz / BZ) * (c->ny / YB) * c->nruns);
-  kern<<<pgrid, NT, smem, c->stream>>>(maps, fo, (const C *)c->tw_x, c->ny, c->nz, (R)1 / (nn * nn), nrows, nbox, rb,
-                                       c->nruns, c->nxh, pipe_ctl(c));
-  return GHOST_OK;
-}
-
-// TMA map of a real FP32 field (x fastest) as 8-byte pairs: a box of
-// nx/2 pairs x 1 y-row x 8 z-values, the tiles of the plain x transforms.
-static int real_map(ghost_ctx *c, const void *base, CUtensorMap *out) {
-  PFN_cuTensorMapEncodeTiled_v12000 enc;
-  GB_CHECK(encode_fn(&enc));
-  const cuuint64_t dims[3] = {(cuuint64_t)c->nx / 2, (cuuint64_t)c->ny, (cuuint64_t)c->nz};
-  const cuuint64_t strides[2] = {(cuuint64_t)c->nx * 4, (cuuint64_t)c->nx * c->ny * 4};
-  const cuuint32_t box[3] = {(cuuint32_t)c->nx / 2, 1, 8};
-  const cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, const_cast<void *>(base), dims, strides, box, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return fail(GHOST_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
-  return GHOST_OK;
-}
-
-// The plain x transforms with one warp per line (FP32, nx = 512, one run).
-static bool xw_plain_ok(const ghost_ctx *c) {
-  return c->precision == GHOST_SINGLE && c->nx == 512 && c->nruns == 1 && c->nz % 8 == 0;
-}
-static int launch_xw_r2c(ghost_ctx *c, const void *in, void *out) {
-  constexpr int NX = 512, M = NX / 2, STAGES = 3;
-  using G = XWPlainGeom<NX, STAGES>;
-  auto kern = xwarp_r2c_kernel<NX, STAGES>;
-  GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::r2c_bytes));
-  const int rb = ((M + 1 + 1) / 2 + 15) / 16 * 16;  // 2 x 144 rows cover the M+1 kx rows
-  static_assert(2 * (((M + 2) / 2 + 15) / 16 * 16) <= G::OROWS, "r2c store boxes exceed the output tile");
-  CUtensorMap rm, cm;
-  GB_CHECK(real_map(c, in, &rm));
-  GB_CHECK(field_map(c, out, 8, 1, rb, &cm, CU_TENSOR_MAP_SWIZZLE_64B));
-  const int grid = persistent_grid(c, kern, 256, G::r2c_bytes, (long)(c->nz / 8) * c->ny);
-  kern<<<grid, 256, G::r2c_bytes, c->stream>>>(rm, cm, (const float2 *)c->tw_x, c->ny, c->nz, rb, pipe_ctl(c));
-  return GHOST_OK;
-}
-static int launch_xw_c2r(ghost_ctx *c, const void *in, void *out) {
-  constexpr int NX = 512, M = NX / 2, STAGES = 4;
-  using G = XWPlainGeom<NX, STAGES>;
-  auto kern = xwarp_c2r_kernel<NX, STAGES>;
-  GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::c2r_bytes));
-  const int nbox = 2, rb = ((M + 1 + 1) / 2 + 15) / 16 * 16;  // 2 x 144 rows cover the M+1 kx rows
-  static_assert(2 * (((M + 2) / 2 + 15) / 16 * 16) <= G::SROWS, "c2r box plan exceeds the slot");
-  CUtensorMap m;
-  GB_CHECK(field_map(c, in, 8, 1, rb, &m, CU_TENSOR_MAP_SWIZZLE_64B));
-  const int grid = persistent_grid(c, kern, 256, G::c2r_bytes, (long)(c->nz / 8) * c->ny);
-  kern<<<grid, 256, G::c2r_bytes, c->stream>>>(m, (float *)out, (const float2 *)c->tw_x, c->ny, c->nz, nbox, rb,
-                                               pipe_ctl(c));
-  return GHOST_OK;
-}
-
-template <typename R, int NX, int KIND> int launch_x_n(ghost_ctx *c, const void *in, void *out, const void *const *ins,
-                                                       void *const *outs, int rows) {
-  constexpr int E = xE<R>() < NX / 2 ? xE<R>() : NX / 2;
-  constexpr int M = NX / 2, T = M / E;
-  // rows of BZ z values; at most 256 threads so the register-resident
-  // real fields of the fused pass fit the register file
-  constexpr int BZ = xBZ<R>() * T <= 256 ? xBZ<R>() : (256 / T > 0 ? 256 / T : 1);
-  constexpr int NT = BZ * T;
-  typedef cx<R> C;
-  dim3 grid(c->nz / BZ, c->ny);
-  const C *tw = (const C *)c->tw_x;
-  const int ts = timer_begin(c, KIND == X_C2R ? GHOST_TIMER_X_C2R : (KIND == X_R2C ? GHOST_TIMER_X_R2C : GHOST_TIMER_X_NL));
-  if (KIND == X_HD || KIND == X_BOUSS) {
-    // FP32 512-point lines: tiles of 16 z-values (128-byte rows, one CTA of
-    // 512 threads per SM) where nz allows, else BZ
-    if constexpr (sizeof(R) == 4 && NX == 512 && BZ == 8) {
-      if (c->nz % 16 == 0) {
-        GB_CHECK((launch_x_fused<R, NX, KIND, 16, 1>(c, ins, outs, rows)));
-        timer_end(c, ts);
-        return post_launch(c);
-      }
-    }
-    // FP32 1024-point lines: tiles of 8 z-values (64-byte rows instead of
-    // 32, one CTA of 512 threads per SM) where nz allows (bit 8 of the tile
-    // variant asks for the 4-value tiles)
-    if constexpr (sizeof(R) == 4 && NX == 1024 && BZ == 4) {
-      if (c->nz % 8 == 0 && !(c->tile_cfg & 256)) {
-        GB_CHECK((launch_x_fused<R, NX, KIND, 8, 1>(c, ins, outs, rows)));
-        timer_end(c, ts);
-        return post_launch(c);
-      }
-    }
-    GB_CHECK((launch_x_fused<R, NX, KIND, BZ, 2>(c, ins, outs, rows)));
-  } else if (KIND == X_C2R && xw_plain_ok(c)) {
-    GB_CHECK(launch_xw_c2r(c, in, out));
-  } else if (KIND == X_R2C && xw_plain_ok(c)) {
-    GB_CHECK(launch_xw_r2c(c, in, out));
-  } else if (KIND == X_C2R) {
-    const size_t smem = (size_t)(NX + (M + 1) * BZ + M * BZ) * sizeof(C);
-    auto kern = xpass_c2r_kernel<R, NX, E, BZ>;
-    GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<grid, NT, smem, c->stream>>>((const C *)in, (R *)out, tw, c->ny, c->nz);
-  } else {
-    const size_t smem = (size_t)(NX + M * BZ) * sizeof(C);
-    auto kern = xpass_r2c_kernel<R, NX, E, BZ>;
-    GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<grid, NT, smem, c->stream>>>((const R *)in, (C *)out, tw, c->ny, c->nz);
-  }
-  timer_end(c, ts);
-  return post_launch(c);
-}
-
-template <typename R, int KIND>
-int launch_x(ghost_ctx *c, const void *in, void *out, const void *const *ins = nullptr, void *const *outs = nullptr,
-             int rows = 0) {
-  switch (c->nx) {
-    case 16: return launch_x_n<R, 16, KIND>(c, in, out, ins, outs, rows);
-    case 32: return launch_x_n<R, 32, KIND>(c, in, out, ins, outs, rows);
-    case 64: return launch_x_n<R, 64, KIND>(c, in, out, ins, outs, rows);
-    case 128: return launch_x_n<R, 128, KIND>(c, in, out, ins, outs, rows);
-    case 256: return launch_x_n<R, 256, KIND>(c, in, out, ins, outs, rows);
-    case 512: return launch_x_n<R, 512, KIND>(c, in, out, ins, outs, rows);
-    case 1024: return launch_x_n<R, 1024, KIND>(c, in, out, ins, outs, rows);
-  }
-  return fail(GHOST_ERR_SIZE, "nx=%d unsupported", c->nx);
-}
+PipeCtl pipe_ctl(ghost_ctx *c) { return PipeCtl{c->status, c->wait_cap, c->inject_stall}; }
 
 // ---------------------------------------------------------------------
 // zero-pruning tables.  After a substep, v is exactly zero outside
@@ -990,49 +658,6 @@ template <typename R> int c2r_dev(ghost_ctx *c, const void *in, void *out) {
   f.p[0] = (cx<R> *)w[0];
   GB_CHECK((launch_y<R, +1>(c, f, 1)));
   return launch_x<R, X_C2R>(c, w[0], out);
-}
-
-// The LES closure's input rows from a spectral velocity: the nine gradients
-// through z and y passes over all nine, then one x pass that writes
-// x[q][3a+b] = (d v_a / d x_b) * gs and x[q][9] = delta directly.
-template <typename R, int NX>
-int grad9_features_n(ghost_ctx *c, void *const spec[9], float *x, float gs, float delta) {
-  constexpr int E = xE<R>() < NX / 2 ? xE<R>() : NX / 2;
-  constexpr int M = NX / 2, T = M / E;
-  constexpr int BZ = xBZ<R>() * T <= 256 ? xBZ<R>() : (256 / T > 0 ? 256 / T : 1);
-  typedef cx<R> C;
-  const size_t smem = (size_t)(NX + (M + 1) * BZ + M * BZ) * sizeof(C);
-  auto kern = xpass_c2r_features_kernel<R, NX, E, BZ>;
-  GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  Fields<R> in{};
-  for (int q = 0; q < 9; ++q) in.p[q] = (C *)spec[q];
-  const int ts = timer_begin(c, GHOST_TIMER_X_C2R);
-  kern<<<dim3(c->nz / BZ, c->ny), BZ * T, smem, c->stream>>>(in, x, (const C *)c->tw_x, c->ny, c->nz,
-                                                              (R)(1.0 / (double)c->nreal), gs, delta);
-  timer_end(c, ts);
-  return post_launch(c);
-}
-
-template <typename R>
-int grad9_features_dev(ghost_ctx *c, const void *const v[3], void *const spec[9], float *x, float gs, float delta) {
-  ZGrad<R> zg{};
-  for (int a = 0; a < 3; ++a) zg.v.p[a] = (const cx<R> *)v[a];
-  for (int q = 0; q < 9; ++q) zg.w.p[q] = (cx<R> *)spec[q];
-  zg.kp = kparams<R>(c);
-  GB_CHECK(launch_z<R>(c, zg));
-  Fields<R> fy{};
-  for (int q = 0; q < 9; ++q) fy.p[q] = (cx<R> *)spec[q];
-  GB_CHECK((launch_y<R, +1>(c, fy, 9)));
-  switch (c->nx) {
-    case 16: return grad9_features_n<R, 16>(c, spec, x, gs, delta);
-    case 32: return grad9_features_n<R, 32>(c, spec, x, gs, delta);
-    case 64: return grad9_features_n<R, 64>(c, spec, x, gs, delta);
-    case 128: return grad9_features_n<R, 128>(c, spec, x, gs, delta);
-    case 256: return grad9_features_n<R, 256>(c, spec, x, gs, delta);
-    case 512: return grad9_features_n<R, 512>(c, spec, x, gs, delta);
-    case 1024: return grad9_features_n<R, 1024>(c, spec, x, gs, delta);
-  }
-  return fail(GHOST_ERR_SIZE, "nx=%d unsupported", c->nx);
 }
 
 // Six real fields to spectra at once (the stresses of the LES closure):
@@ -1462,7 +1087,6 @@ int batch_init_random_dev(ghost_ctx *c, const int32_t *seeds, int32_t *seeds_out
   template int r2c_dev<R>(ghost_ctx *, const void *, void *);                                                  \
   template int c2r_dev<R>(ghost_ctx *, const void *, void *);                                                  \
   template int r2c6_dev<R>(ghost_ctx *, const void *const[6], void *const[6]);                                 \
-  template int grad9_features_dev<R>(ghost_ctx *, const void *const[3], void *const[9], float *, float, float);     \
   template int hd_substep_dev<R>(ghost_ctx *, int, double, double, void *const[3], void *const[3],             \
                                  const void *const[3], int, bool);
 GB_INST(float)

@@ -2,7 +2,12 @@
 // translation units of the library (les.cu).  Explicit instantiations for
 // float and double live at the end of api.cu's gb namespace.
 #pragma once
+#include <cudaTypedefs.h>
+
+#include <algorithm>
+
 #include "common.cuh"
+#include "passes.cuh"
 
 namespace gb {
 
@@ -30,6 +35,48 @@ template <typename R> int r2c6_dev(ghost_ctx *c, const void *const in[6], void *
 template <typename R>
 int hd_substep_dev(ghost_ctx *c, int o, double dt, double nu, void *const v[3], void *const C[3], const void *const f[3],
                    int copy, bool prune = false);
+// E of the X and Z passes and z-values of an X tile
+template <typename R> constexpr int xE() { return sizeof(R) == 4 ? 8 : 4; }
+template <typename R> constexpr int xBZ() { return sizeof(R) == 4 ? 8 : 4; }
+
+template <typename R> constexpr int zE() { return sizeof(R) == 4 ? 8 : 4; }
+
+// Pruning state for one substep: null tables = every line.
+struct Prune {
+  const int *lines = nullptr;
+  int nlines = 0;
+  const int *jpos = nullptr, *jneg = nullptr;
+  int ni = 0;    // kx indices processed by the y passes
+  int rows = 0;  // kx rows present in / written by the x pass
+};
+
+// X pass kinds
+enum XKind { X_HD = 0, X_C2R = 1, X_R2C = 2, X_BOUSS = 3 };
+
+// the passes: Op of passes.cuh over z-lines; nf fields along y (in place);
+// an X pass of kind KIND (in, out: the plain transforms; ins, outs: the fused
+// ones, whose output fields may be any of the inputs that a tile has consumed)
+template <typename R, class Op> int launch_z(ghost_ctx *c, const Op &op, const Prune &pr = Prune());
+template <typename R, int S> int launch_y(ghost_ctx *c, const Fields<R> &f, int nf, const Prune &pr = Prune());
+template <typename R, int KIND>
+int launch_x(ghost_ctx *c, const void *in, void *out, const void *const *ins = nullptr, void *const *outs = nullptr,
+             int rows = 0);
+int encode_fn(PFN_cuTensorMapEncodeTiled_v12000 *fn);
+int sm_count(ghost_ctx *c);
+// Persistent grid: as many CTAs as fit on the device at once, or fewer
+// when there are fewer tiles.
+template <class K> int persistent_grid(ghost_ctx *c, K kern, int threads, size_t smem, long ntiles) {
+  int per_sm = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
+  if (per_sm < 1) per_sm = 1;
+  const long g = (long)per_sm * sm_count(c);
+  return (int)std::max<long>(1, std::min<long>(g, ntiles));
+}
+// TMA tensor map of a spectral field: a 3D tensor (z in 8-byte units, y, kx)
+// over one field, with the box the pass moves
+int field_map(ghost_ctx *c, const void *base, unsigned box0, unsigned box1, unsigned box2, CUtensorMap *out,
+              CUtensorMapSwizzle swz = CU_TENSOR_MAP_SWIZZLE_NONE);
+PipeCtl pipe_ctl(ghost_ctx *c);
 // FP64 partial sums owned by the context, grown on demand
 int partials(ghost_ctx *c, size_t n, double **out);
 // per-kernel timers around a launch (kind GHOST_TIMER_*)

@@ -1,0 +1,80 @@
+// passes_z.cuh -- launches of the Z passes (passes.cuh), one template instance
+// per line length; passes_z32.cu and passes_z64.cu instantiate them.
+#pragma once
+#include <algorithm>
+
+#include "internal.cuh"
+
+namespace gb {
+
+template <class Op> struct ZKind;
+template <typename R, int S, int NF> struct ZKind<ZC2C<R, S, NF>> { static constexpr int value = GHOST_TIMER_Z_C2C; };
+template <typename R, int P> struct ZKind<ZInv<R, P>> { static constexpr int value = GHOST_TIMER_Z_INV; };
+template <typename R> struct ZKind<ZGrad<R>> { static constexpr int value = GHOST_TIMER_Z_INV; };
+template <typename R> struct ZKind<ZFwdHD<R>> { static constexpr int value = GHOST_TIMER_Z_FWD; };
+template <typename R> struct ZKind<ZFwdBouss<R>> { static constexpr int value = GHOST_TIMER_Z_FWD; };
+
+template <typename R, int N, int LPB, int STAGES0, int MINB, class Op>
+int launch_z_cfg(ghost_ctx *c, const Op &op, const Prune &pr) {
+  constexpr int E = zE<R>() < N ? zE<R>() : N, T = N / E;
+  using G = ZGeom<R, N, E, LPB, Op::NLOAD>;
+  constexpr int STAGES = G::smem_bytes(STAGES0) <= 200 * 1024 ? STAGES0 : 2;
+  const size_t smem = G::smem_bytes(STAGES);
+  const int nlines = pr.lines ? pr.nlines : c->ny * c->nxh * c->nruns;
+  auto kern = zpipe_kernel<R, N, E, LPB, STAGES, MINB, Op>;
+  GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int grid = persistent_grid(c, kern, LPB * T, smem, (nlines + LPB - 1) / LPB);
+  const int ts = timer_begin(c, ZKind<Op>::value);
+  kern<<<grid, LPB * T, smem, c->stream>>>(op, (const cx<R> *)c->tw_z, pr.lines, nlines, pipe_ctl(c));
+  timer_end(c, ts);
+  return post_launch(c);
+}
+
+// CTAs of 256 threads; with tile variant bit 1 of 128 threads; with bits 1
+// and 2 of 128 threads with a two-stage ring and at most 170 registers, so
+// that three CTAs share an SM (lines of 256 points or more)
+// lines per CTA, halved from want until a two-stage ring of NL fields fits
+template <typename R, int N, int NL> constexpr int fit_lines(int want) {
+  int lpb = want;
+  while (lpb > 1 && ((size_t)2 * NL * lpb * N + N + (size_t)2 * lpb * (N + N / 8)) * sizeof(cx<R>) + 24 > 220 * 1024)
+    lpb /= 2;
+  return lpb;
+}
+
+template <typename R, int N, class Op> int launch_z_n(ghost_ctx *c, const Op &op, const Prune &pr) {
+  constexpr int E = zE<R>() < N ? zE<R>() : N, T = N / E;
+  constexpr int L256 = fit_lines<R, N, Op::NLOAD>(256 / T > 0 ? 256 / T : 1);
+  constexpr int L128 = fit_lines<R, N, Op::NLOAD>(128 / T > 0 ? 128 / T : 1);
+  if constexpr (N >= 256 && L128 != L256) {
+    if ((c->tile_cfg & 38) == 38) return launch_z_cfg<R, N, L128, 1, 4>(c, op, pr);
+    if ((c->tile_cfg & 6) == 6) return launch_z_cfg<R, N, L128, 2, 3>(c, op, pr);
+  }
+  if ((c->tile_cfg & 2) && L128 != L256) return launch_z_cfg<R, N, L128, 3, 1>(c, op, pr);
+  return launch_z_cfg<R, N, L256, 3, 1>(c, op, pr);
+}
+
+template <typename R, class Op> int launch_z(ghost_ctx *c, const Op &op, const Prune &pr) {
+  switch (c->nz) {
+    case 16: return launch_z_n<R, 16>(c, op, pr);
+    case 32: return launch_z_n<R, 32>(c, op, pr);
+    case 64: return launch_z_n<R, 64>(c, op, pr);
+    case 128: return launch_z_n<R, 128>(c, op, pr);
+    case 256: return launch_z_n<R, 256>(c, op, pr);
+    case 512: return launch_z_n<R, 512>(c, op, pr);
+    case 1024: return launch_z_n<R, 1024>(c, op, pr);
+  }
+  return fail(GHOST_ERR_SIZE, "nz=%d unsupported", c->nz);
+}
+
+#define GB_INST(R)                                                                    \
+  template int launch_z<R, ZInv<R, 0>>(ghost_ctx *, const ZInv<R, 0> &, const Prune &);   \
+  template int launch_z<R, ZInv<R, 1>>(ghost_ctx *, const ZInv<R, 1> &, const Prune &);   \
+  template int launch_z<R, ZGrad<R>>(ghost_ctx *, const ZGrad<R> &, const Prune &);       \
+  template int launch_z<R, ZFwdHD<R>>(ghost_ctx *, const ZFwdHD<R> &, const Prune &);     \
+  template int launch_z<R, ZFwdBouss<R>>(ghost_ctx *, const ZFwdBouss<R> &, const Prune &); \
+  template int launch_z<R, ZC2C<R, -1, 1>>(ghost_ctx *, const ZC2C<R, -1, 1> &, const Prune &); \
+  template int launch_z<R, ZC2C<R, -1, 3>>(ghost_ctx *, const ZC2C<R, -1, 3> &, const Prune &); \
+  template int launch_z<R, ZC2C<R, -1, 6>>(ghost_ctx *, const ZC2C<R, -1, 6> &, const Prune &); \
+  template int launch_z<R, ZC2C<R, +1, 1>>(ghost_ctx *, const ZC2C<R, +1, 1> &, const Prune &);
+
+}  // namespace gb
