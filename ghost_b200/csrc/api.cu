@@ -1630,56 +1630,53 @@ template <typename R> static int gauge3_dev(ghost_ctx *c, const void *a, const v
   return post_launch(c);
 }
 
-// One MHD substep (include/mhd_rkstep2.f90); Cv, Ca the RK copies of v, a
+// One MHD substep (include/mhd_rkstep2.f90) in five passes, with mhd_rkstep1
+// folded in when copy != 0: va = vx, vy, vz, ax, ay, az, Cva their RK copies,
+// fm the forcings (a triple null: none).  Twelve inverse and six forward
+// transforms: nonlin3 is linear, so w x v - j x b is formed in real space.
 template <typename R>
-static int mhd_substep_dev(ghost_ctx *c, int o, double dt, double nu, double mu, void *const v[3], void *const a[3],
-                           void *const Cv[3], void *const Ca[3], const void *const f[3], const void *const m[3]) {
-  void *sc[46];
-  GB_CHECK(scratch(c, 46, sc));
-  void *B[3] = {sc[22], sc[23], sc[24]}, *N1[3] = {sc[25], sc[26], sc[27]}, *N2[3] = {sc[28], sc[29], sc[30]};
-  void *G[3] = {sc[31], sc[32], sc[33]};
-  // b = curl a (rotor3(ay,az,C7,1), rotor3(ax,az,C8,2), rotor3(ax,ay,C9,3))
-  GB_CHECK(rotor3_impl<R>(c, a[1], a[2], B[0], 1));
-  GB_CHECK(rotor3_impl<R>(c, a[0], a[2], B[1], 2));
-  GB_CHECK(rotor3_impl<R>(c, a[0], a[1], B[2], 3));
-  GB_CHECK(prodre3_dev<R>(c, v[0], v[1], v[2], N1[0], N1[1], N1[2]));  // w x v
-  GB_CHECK(prodre3_dev<R>(c, B[0], B[1], B[2], N2[0], N2[1], N2[2]));  // j x b
-  const void *nl[6] = {N1[0], N1[1], N1[2], N2[0], N2[1], N2[2]};
-  for (int d = 0; d < 3; ++d) GB_CHECK(nonlin3_dev<R>(c, nl, G[d], d + 1));
-  // v x b into N1, its Coulomb-gauge projection into N2
-  const void *vb[6] = {v[0], v[1], v[2], B[0], B[1], B[2]};
-  GB_CHECK(vector3_dev<R>(c, vb, N1));
-  for (int d = 0; d < 3; ++d) GB_CHECK(gauge3_dev<R>(c, N1[0], N1[1], N1[2], N2[d], d + 1));
-  MhdUpd<R> u{};
-  for (int q = 0; q < 3; ++q) {
-    u.v[q] = (cx<R> *)v[q];
-    u.a[q] = (cx<R> *)a[q];
-    u.cv[q] = (const cx<R> *)Cv[q];
-    u.ca[q] = (const cx<R> *)Ca[q];
-    u.g[q] = (const cx<R> *)G[q];
-    u.h[q] = (const cx<R> *)N2[q];
-    u.f[q] = f ? (const cx<R> *)f[q] : nullptr;
-    u.m[q] = m ? (const cx<R> *)m[q] : nullptr;
+static int mhd_substep_dev(ghost_ctx *c, int o, double dt, double nu, double mu, void *const va[6], void *const Cva[6],
+                           const void *const fm[6], void *const w[12], int copy, bool prune) {
+  Prune pr;
+  GB_CHECK(prune_plan<R>(c, prune, &pr));
+  ZInvMhd<R> zi{};
+  Fields<R> fy{};
+  for (int q = 0; q < 6; ++q) {
+    zi.va.p[q] = (const cx<R> *)va[q];
+    zi.cpy.p[q] = (cx<R> *)Cva[q];
   }
-  mhd_update_kernel<R><<<grid1d(c->ntot), 256, 0, c->stream>>>(kparams<R>(c), u, c->ntot, (R)dt, (R)nu, (R)mu,
-                                                                (R)1 / (R)o);
-  return post_launch(c);
+  for (int q = 0; q < 12; ++q) fy.p[q] = zi.w.p[q] = (cx<R> *)w[q];
+  zi.kp = kparams<R>(c);
+  zi.copy = copy;
+  GB_CHECK(launch_z<R>(c, zi, pr));
+  GB_CHECK((launch_y<R, +1>(c, fy, 12, pr)));
+  GB_CHECK((launch_x<R, X_MHD>(c, nullptr, nullptr, (const void *const *)w, w, pr.rows)));
+  GB_CHECK((launch_y<R, -1>(c, fy, 6, pr)));
+  ZFwdMhd<R> zf{};
+  for (int q = 0; q < 6; ++q) {
+    zf.nl.p[q] = (const cx<R> *)w[(q + 3) % 6];  // the x pass left v x b first
+    zf.va.p[q] = (cx<R> *)va[q];
+    zf.c0.p[q] = (const cx<R> *)Cva[q];
+    zf.f.p[q] = (const cx<R> *)fm[q];
+  }
+  zf.kp = kparams<R>(c);
+  zf.dt = (R)dt;
+  zf.nu = (R)nu;
+  zf.mu = (R)mu;
+  zf.rmp = (R)1 / (R)o;
+  return launch_z<R>(c, zf, pr);
 }
 
 template <typename R>
-static int mhd_run_dev(ghost_ctx *c, int nsteps, int ord, double dt, double nu, double mu, void *const v[3],
-                       void *const a[3], const void *const f[3], const void *const m[3]) {
-  void *sc[46];
-  GB_CHECK(scratch(c, 46, sc));
-  void *Cv[3] = {sc[16], sc[17], sc[18]}, *Ca[3] = {sc[19], sc[20], sc[21]};
-  for (int s = 0; s < nsteps; ++s) {
-    // mhd_rkstep1: C1..C6 = v, a
-    for (int q = 0; q < 3; ++q) {
-      GB_CUDA(cudaMemcpyAsync(Cv[q], v[q], c->cbytes, cudaMemcpyDeviceToDevice, c->stream));
-      GB_CUDA(cudaMemcpyAsync(Ca[q], a[q], c->cbytes, cudaMemcpyDeviceToDevice, c->stream));
-    }
-    for (int o = ord; o >= 1; --o) GB_CHECK(mhd_substep_dev<R>(c, o, dt, nu, mu, v, a, Cv, Ca, f, m));
-  }
+static int mhd_run_dev(ghost_ctx *c, int nsteps, int ord, double dt, double nu, double mu, void *const va[6],
+                       const void *const fm[6]) {
+  void *sc[18];
+  GB_CHECK(scratch(c, 18, sc));
+  // as in ghost_hd_run: the first substep of a call may find modes outside
+  // the truncation, the later ones find zeros there
+  for (int s = 0; s < nsteps; ++s)
+    for (int o = ord; o >= 1; --o)
+      GB_CHECK(mhd_substep_dev<R>(c, o, dt, nu, mu, va, sc + 12, fm, sc, o == ord, !(s == 0 && o == ord)));
   return check_status(c);
 }
 }  // extern "C++"
@@ -1741,20 +1738,16 @@ int ghost_mhd_run(ghost_ctx *c, int nsteps, int ord, double dt, double nu, doubl
     return fail(GHOST_ERR_ARG, "forcing components must all be given or all be null");
   if (c->nruns != 1) return fail(GHOST_ERR_STATE, "batched contexts are not supported here");
   Staging st(c);
-  void *v[3], *a[3];
-  const void *f[3] = {nullptr, nullptr, nullptr}, *m[3] = {nullptr, nullptr, nullptr};
-  void *vs[3] = {vx, vy, vz}, *as[3] = {ax, ay, az};
-  const void *fs[3] = {fx, fy, fz}, *ms[3] = {mx, my, mz};
-  for (int q = 0; q < 3; ++q) {
-    GB_CHECK(st.map(vs[q], c->cbytes, 3, &v[q]));
-    GB_CHECK(st.map(as[q], c->cbytes, 3, &a[q]));
-    if (fx) GB_CHECK(st.map(fs[q], c->cbytes, 1, &f[q]));
-    if (mx) GB_CHECK(st.map(ms[q], c->cbytes, 1, &m[q]));
+  void *va[6];
+  const void *fm[6] = {};
+  void *vas[6] = {vx, vy, vz, ax, ay, az};
+  const void *fms[6] = {fx, fy, fz, mx, my, mz};
+  for (int q = 0; q < 6; ++q) {
+    GB_CHECK(st.map(vas[q], c->cbytes, 3, &va[q]));
+    if (fms[q]) GB_CHECK(st.map(fms[q], c->cbytes, 1, &fm[q]));
   }
-  GB_CHECK(c->precision == GHOST_SINGLE ? mhd_run_dev<float>(c, nsteps, ord, dt, nu, mu, v, a, fx ? f : nullptr,
-                                                             mx ? m : nullptr)
-                                        : mhd_run_dev<double>(c, nsteps, ord, dt, nu, mu, v, a, fx ? f : nullptr,
-                                                              mx ? m : nullptr));
+  GB_CHECK(c->precision == GHOST_SINGLE ? mhd_run_dev<float>(c, nsteps, ord, dt, nu, mu, va, fm)
+                                        : mhd_run_dev<double>(c, nsteps, ord, dt, nu, mu, va, fm));
   return st.finish();
 }
 

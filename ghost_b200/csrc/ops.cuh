@@ -444,42 +444,6 @@ __global__ void neg_kernel(cx<R> *x, size_t n) {
     x[p] = mk(-x[p].x, -x[p].y);
 }
 
-// The truncated update of mhd_rkstep2 (include/mhd_rkstep2.f90): with
-// laplak3 inline, v = C + dt (nu lap v + g + f)/o and a = C' + dt (mu lap a
-// + h + m)/o on tiny <= kn2 <= kmax, everything zero elsewhere.
-template <typename R> struct MhdUpd {
-  cx<R> *v[3], *a[3];
-  const cx<R> *cv[3], *ca[3], *g[3], *h[3], *f[3], *m[3];
-};
-template <typename R>
-__global__ void mhd_update_kernel(KParams<R> kp, MhdUpd<R> u, size_t n, R dt, R nu, R mu, R rmp) {
-  for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x) {
-    int i, j, k;
-    unflat(kp, p, i, j, k);
-    const R kn2 = kn2_of(kp, i, j, k);
-    if (kn2 <= kp.kmax && kn2 >= kp.tiny) {
-      const R kk2 = kk2_of(kp, i, j, k);
-#pragma unroll
-      for (int q = 0; q < 3; ++q) {
-        const cx<R> vv = u.v[q][p], aa = u.a[q][p];
-        const cx<R> lv = mk(-kk2 * vv.x, -kk2 * vv.y), la = mk(-kk2 * aa.x, -kk2 * aa.y);
-        cx<R> sv = mk(nu * lv.x + u.g[q][p].x, nu * lv.y + u.g[q][p].y);
-        cx<R> sa = mk(mu * la.x + u.h[q][p].x, mu * la.y + u.h[q][p].y);
-        if (u.f[q]) sv = cadd(sv, u.f[q][p]);
-        if (u.m[q]) sa = cadd(sa, u.m[q][p]);
-        u.v[q][p] = mk(u.cv[q][p].x + dt * sv.x * rmp, u.cv[q][p].y + dt * sv.y * rmp);
-        u.a[q][p] = mk(u.ca[q][p].x + dt * sa.x * rmp, u.ca[q][p].y + dt * sa.y * rmp);
-      }
-    } else {
-#pragma unroll
-      for (int q = 0; q < 3; ++q) {
-        u.v[q][p] = mk((R)0, (R)0);
-        u.a[q][p] = mk((R)0, (R)0);
-      }
-    }
-  }
-}
-
 // Horizontal (x, y) sums of real fields per z-plane (havgcomp,
 // pseudospec3D_bouss.f90:19-554): block (k, s) sums a strided part of plane k
 // of op(r1, r2, r3) into partials[k * gridDim.y + s].

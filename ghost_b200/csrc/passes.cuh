@@ -53,7 +53,7 @@ template <typename R, int N, int E, int LPB, int NL> struct ZGeom {
 
 // One 3D tensor map per field: (z in 8-byte units, y, kx).
 struct FieldMaps {
-  CUtensorMap m[9];
+  CUtensorMap m[12];
 };
 
 struct PipeCtl {
@@ -236,6 +236,70 @@ template <typename R, int PHYS> struct ZInv {
   }
 };
 
+// Inverse prologue of the MHD substep (include/mhd_rkstep2.f90): from v and
+// the vector potential a, per mode and with rotor3's operation order,
+//   w[0..2] = v, w[3..5] = curl v, w[6..8] = b = curl a, w[9..11] = curl b,
+// with their inverse z transforms; with copy != 0 also the copies of v and a.
+template <typename R> struct ZInvMhd {
+  using C = cx<R>;
+  static constexpr int NLOAD = 6;
+  CFields<R> va;  // vx, vy, vz, ax, ay, az
+  Fields<R> w;    // 12 outputs
+  Fields<R> cpy;  // 6 (when copy)
+  KParams<R> kp;
+  int copy;
+  __device__ __forceinline__ const C *load_src(int f) const { return va.p[f]; }
+  // component d of the curl of (x, y, z)
+  static __device__ __forceinline__ C curl(int d, R kx, R ky, R kz, C x, C y, C z) {
+    if (d == 0) return mk((-ky * z.y) - (-kz * y.y), (ky * z.x) - (kz * y.x));
+    if (d == 1) return mk((-kz * x.y) - (-kx * z.y), (kz * x.x) - (kx * z.x));
+    return mk((-kx * y.y) - (-ky * x.y), (kx * y.x) - (ky * x.x));
+  }
+  template <int N, int E, class Buf, class Sync, class In>
+  __device__ __forceinline__ void body(long line, bool act, int t, const C *tw, Buf buf, Sync sync, In src) const {
+    constexpr int T = N / E;
+    const int j = (int)(line % kp.ny), i = (int)(line / kp.ny) % kp.nxh + kp.i0;
+    const R kx = kx_of(kp, i), ky = ky_of(kp, j);
+    if (copy && act) {
+#pragma unroll
+      for (int c = 0; c < 6; ++c)
+#pragma unroll
+        for (int e = 0; e < E; ++e) cpy.p[c][(size_t)line * N + t + T * e] = src(c)[t + T * e];
+    }
+#pragma unroll
+    for (int f = 0; f < 12; ++f) {
+      const int d = f % 3;
+      C x[E];
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const int k = t + T * e;
+        const R kz = kz_of(kp, k);
+        if (f < 3) {
+          x[e] = src(f)[k];
+        } else if (f < 6) {
+          x[e] = curl(d, kx, ky, kz, src(0)[k], src(1)[k], src(2)[k]);
+        } else {
+          const C ax = src(3)[k], ay = src(4)[k], az = src(5)[k];
+          if (f < 9) {
+            x[e] = curl(d, kx, ky, kz, ax, ay, az);
+          } else {
+            C b[3];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) b[q] = curl(q, kx, ky, kz, ax, ay, az);
+            x[e] = curl(d, kx, ky, kz, b[0], b[1], b[2]);
+          }
+        }
+      }
+      line_fft<C, N, E, +1>(x, t, tw, buf, sync);
+      if (act) {
+        C *dst = w.p[f] + (size_t)line * N;
+#pragma unroll
+        for (int e = 0; e < E; ++e) dst[t + T * e] = x[e];
+      }
+    }
+  }
+};
+
 // The nine velocity gradients (derivk3 of each component along each axis,
 // pseudospec3D_hd.f90:22-88) with their inverse z transforms:
 // w[3a+b] = i k_b v_a, for the inputs of the LES closure.
@@ -272,9 +336,104 @@ template <typename R> struct ZGrad {
   }
 };
 
-// HD forward epilogue: forward z transform of the three components of
-// omega x v, then nonlhd3 x3 (pseudospec3D_hd.f90:399-509), laplak3 and
-// the truncated RK update of include/hd_rkstep2.f90:18-38, written to v.
+// Forward z transforms of three fields src(OFF..OFF+2) of a line and the truncated
+// RK update with them: x = nonlhd3 of the three (pseudospec3D_hd.f90:399-509;
+// GAUGE: its negative, gauge3 of pseudospec3D_mhd.f90:230-336), then
+// v = C + dt (nu laplak3(v) + x + f)/o on the kept modes, 0 elsewhere
+// (include/hd_rkstep2.f90:18-38).
+template <typename R, int N, int E, bool GAUGE, int OFF, class Buf, class Sync, class In>
+__device__ __forceinline__ void fwd_update(const KParams<R> &kp, long line, bool act, int i, int j, R kx, R ky, int t,
+                                           const cx<R> *tw, Buf buf, Sync sync, In src, const Fields<R> &v,
+                                           const CFields<R> &c0, const CFields<R> &f, R dt, R nuv, R rmp) {
+  using C = cx<R>;
+  constexpr int T = N / E;
+  const bool forced = f.p[OFF] != nullptr;
+  // The kept modes are known before the transforms: their v, C and f
+  // values are prefetched into L2 while the three lines are transformed.
+  bool keep[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const R kn2 = kn2_of(kp, i, j, t + T * e);
+    keep[e] = act && kn2 <= kp.kmax && kn2 >= kp.tiny;
+  }
+  {
+    const size_t base = (size_t)line * N + t;
+#pragma unroll
+    for (int e = 0; e < E; ++e)
+      if (keep[e]) {
+        const size_t p = base + (size_t)T * e;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          prefetch_l2(v.p[OFF + c] + p);
+          prefetch_l2(c0.p[OFF + c] + p);
+          if (forced) prefetch_l2(f.p[OFF + c] + p);
+        }
+      }
+  }
+  C g[3][E];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+#pragma unroll
+    for (int e = 0; e < E; ++e) g[c][e] = src(OFF + c)[t + T * e];
+    line_fft<C, N, E, -1>(g[c], t, tw, buf, sync);
+  }
+  if (!act) return;
+  // The projected nonlinear term replaces g in place; then, component by
+  // component, all of the line's operands (v, C, f at the kept modes) are
+  // loaded before any result is stored, so a thread waits for one round
+  // of loads per component rather than one per element.
+  R kk2e[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const int k = t + T * e;
+    kk2e[e] = (R)0;
+    if (keep[e]) {
+      const R kz = kz_of(kp, k);
+      const R kk2 = kk2_of(kp, i, j, k);
+      kk2e[e] = kk2;
+      const C a = g[0][e], b = g[1][e], cc = g[2][e];
+      const C s = mk(kx * a.x + ky * b.x + kz * cc.x, kx * a.y + ky * b.y + kz * cc.y);
+      g[0][e] = (i == 0) ? mk(-a.x, -a.y) : mk(-a.x + (kx * s.x) / kk2, -a.y + (kx * s.y) / kk2);
+      if (GAUGE) g[0][e] = mk(-g[0][e].x, -g[0][e].y);
+      g[1][e] = (j == 0) ? mk(-b.x, -b.y) : mk(-b.x + (ky * s.x) / kk2, -b.y + (ky * s.y) / kk2);
+      if (GAUGE) g[1][e] = mk(-g[1][e].x, -g[1][e].y);
+      g[2][e] = (k == 0) ? mk(-cc.x, -cc.y) : mk(-cc.x + (kz * s.x) / kk2, -cc.y + (kz * s.y) / kk2);
+      if (GAUGE) g[2][e] = mk(-g[2][e].x, -g[2][e].y);
+    }
+  }
+  const size_t base = (size_t)line * N + t;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    C vv[E], ff[E], cc0[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      vv[e] = mk((R)0, (R)0);
+      ff[e] = mk((R)0, (R)0);
+      cc0[e] = mk((R)0, (R)0);
+      if (keep[e]) {
+        const size_t p = base + (size_t)T * e;
+        vv[e] = v.p[OFF + c][p];
+        cc0[e] = c0.p[OFF + c][p];
+        if (forced) ff[e] = f.p[OFF + c][p];
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const size_t p = base + (size_t)T * e;
+      if (keep[e]) {
+        const R kk2 = kk2e[e];
+        const C lap = mk(-kk2 * vv[e].x, -kk2 * vv[e].y);
+        C sum = mk(nuv * lap.x + g[c][e].x, nuv * lap.y + g[c][e].y);
+        if (forced) sum = mk(sum.x + ff[e].x, sum.y + ff[e].y);
+        v.p[OFF + c][p] = mk(cc0[e].x + (dt * sum.x) * rmp, cc0[e].y + (dt * sum.y) * rmp);
+      } else {
+        v.p[OFF + c][p] = mk((R)0, (R)0);
+      }
+    }
+  }
+}
+
+// HD forward epilogue: fwd_update of the three components of omega x v.
 template <typename R> struct ZFwdHD {
   using C = cx<R>;
   static constexpr int NLOAD = 3;
@@ -287,91 +446,32 @@ template <typename R> struct ZFwdHD {
   __device__ __forceinline__ const C *load_src(int q) const { return nl.p[q]; }
   template <int N, int E, class Buf, class Sync, class In>
   __device__ __forceinline__ void body(long line, bool act, int t, const C *tw, Buf buf, Sync sync, In src) const {
-    constexpr int T = N / E;
     const int j = (int)(line % kp.ny), ir = (int)(line / kp.ny), i = ir % kp.nxh + kp.i0;
     const R kx = kx_of(kp, i), ky = ky_of(kp, j);
     const R nuv = kp.nu_run ? kp.nu_run[ir / kp.nxh] : nu;
-    const bool forced = f.p[0] != nullptr;
-    // The kept modes are known before the transforms: their v, C and f
-    // values are prefetched into L2 while the three lines are transformed.
-    bool keep[E];
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const R kn2 = kn2_of(kp, i, j, t + T * e);
-      keep[e] = act && kn2 <= kp.kmax && kn2 >= kp.tiny;
-    }
-    {
-      const size_t base = (size_t)line * N + t;
-#pragma unroll
-      for (int e = 0; e < E; ++e)
-        if (keep[e]) {
-          const size_t p = base + (size_t)T * e;
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            prefetch_l2(v.p[c] + p);
-            prefetch_l2(c0.p[c] + p);
-            if (forced) prefetch_l2(f.p[c] + p);
-          }
-        }
-    }
-    C g[3][E];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-#pragma unroll
-      for (int e = 0; e < E; ++e) g[c][e] = src(c)[t + T * e];
-      line_fft<C, N, E, -1>(g[c], t, tw, buf, sync);
-    }
-    if (!act) return;
-    // The projected nonlinear term replaces g in place; then, component by
-    // component, all of the line's operands (v, C, f at the kept modes) are
-    // loaded before any result is stored, so a thread waits for one round
-    // of loads per component rather than one per element.
-    R kk2e[E];
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const int k = t + T * e;
-      kk2e[e] = (R)0;
-      if (keep[e]) {
-        const R kz = kz_of(kp, k);
-        const R kk2 = kk2_of(kp, i, j, k);
-        kk2e[e] = kk2;
-        const C a = g[0][e], b = g[1][e], cc = g[2][e];
-        const C s = mk(kx * a.x + ky * b.x + kz * cc.x, kx * a.y + ky * b.y + kz * cc.y);
-        g[0][e] = (i == 0) ? mk(-a.x, -a.y) : mk(-a.x + (kx * s.x) / kk2, -a.y + (kx * s.y) / kk2);
-        g[1][e] = (j == 0) ? mk(-b.x, -b.y) : mk(-b.x + (ky * s.x) / kk2, -b.y + (ky * s.y) / kk2);
-        g[2][e] = (k == 0) ? mk(-cc.x, -cc.y) : mk(-cc.x + (kz * s.x) / kk2, -cc.y + (kz * s.y) / kk2);
-      }
-    }
-    const size_t base = (size_t)line * N + t;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      C vv[E], ff[E], cc0[E];
-#pragma unroll
-      for (int e = 0; e < E; ++e) {
-        vv[e] = mk((R)0, (R)0);
-        ff[e] = mk((R)0, (R)0);
-        cc0[e] = mk((R)0, (R)0);
-        if (keep[e]) {
-          const size_t p = base + (size_t)T * e;
-          vv[e] = v.p[c][p];
-          cc0[e] = c0.p[c][p];
-          if (forced) ff[e] = f.p[c][p];
-        }
-      }
-#pragma unroll
-      for (int e = 0; e < E; ++e) {
-        const size_t p = base + (size_t)T * e;
-        if (keep[e]) {
-          const R kk2 = kk2e[e];
-          const C lap = mk(-kk2 * vv[e].x, -kk2 * vv[e].y);
-          C sum = mk(nuv * lap.x + g[c][e].x, nuv * lap.y + g[c][e].y);
-          if (forced) sum = mk(sum.x + ff[e].x, sum.y + ff[e].y);
-          v.p[c][p] = mk(cc0[e].x + (dt * sum.x) * rmp, cc0[e].y + (dt * sum.y) * rmp);
-        } else {
-          v.p[c][p] = mk((R)0, (R)0);
-        }
-      }
-    }
+    fwd_update<R, N, E, false, 0>(kp, line, act, i, j, kx, ky, t, tw, buf, sync, src, v, c0, f, dt, nuv, rmp);
+  }
+};
+
+// MHD forward epilogue (include/mhd_rkstep2.f90): nl[0..2] holds w x v - j x b
+// (nonlin3 of the two, linear) for the update of v, nl[3..5] holds v x b
+// (gauge3) for the update of a.
+template <typename R> struct ZFwdMhd {
+  using C = cx<R>;
+  static constexpr int NLOAD = 6;
+  CFields<R> nl;  // 6
+  Fields<R> va;   // vx, vy, vz, ax, ay, az in/out
+  CFields<R> c0;  // their copies
+  CFields<R> f;   // fx, fy, fz, mx, my, mz (a triple null: none)
+  KParams<R> kp;
+  R dt, nu, mu, rmp;
+  __device__ __forceinline__ const C *load_src(int q) const { return nl.p[q]; }
+  template <int N, int E, class Buf, class Sync, class In>
+  __device__ __forceinline__ void body(long line, bool act, int t, const C *tw, Buf buf, Sync sync, In src) const {
+    const int j = (int)(line % kp.ny), i = (int)(line / kp.ny) % kp.nxh + kp.i0;
+    const R kx = kx_of(kp, i), ky = ky_of(kp, j);
+    fwd_update<R, N, E, false, 0>(kp, line, act, i, j, kx, ky, t, tw, buf, sync, src, va, c0, f, dt, nu, rmp);
+    fwd_update<R, N, E, true, 3>(kp, line, act, i, j, kx, ky, t, tw, buf, sync, src, va, c0, f, dt, mu, rmp);
   }
 };
 
@@ -752,6 +852,9 @@ template <typename C> __device__ __forceinline__ C r2c_unpack(C zk, C zm, C w) {
 //   PHYS 1 (BOUSS): in v, curl v, grad theta (9)
 //                   -> out omega x v (3), -v.grad(theta) (1)
 //                   (prodre3 + advect3, pseudospec3D_phd.f90:23-114)
+//   PHYS 2 (MHD):   in v, curl v, b, curl b (12)
+//                   -> out v x b (3), w x v - j x b (3) (vector3, and nonlin3's
+//                   difference of the two prodre3, pseudospec3D_mhd.f90:22-227)
 // A persistent CTA walks (z-block, y) tiles.  Every input field of a tile
 // is one TMA tensor load (nbox boxes of rb kx-rows x BZ z-values) into a
 // STAGES-deep ring, so the next fields (and the next tile) stream in while
@@ -786,7 +889,7 @@ __device__ __forceinline__ void xpipe_nl_body(int vb, int nvb, const FieldMaps &
   using G = XGeom<R, NX, BZ, YB>;
   constexpr int M = NX / 2, T = M / E, NT = YB * BZ * T;
   constexpr int LW = YB * BZ;  // lines of a tile: (y, z) with z fastest
-  constexpr int NIN = PHYS == 0 ? 6 : 9, NOUT = PHYS == 0 ? 3 : 4;
+  constexpr int NIN = PHYS == 0 ? 6 : (PHYS == 1 ? 9 : 12), NOUT = PHYS == 1 ? 4 : 3;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   C *stage = reinterpret_cast<C *>(smem_raw);
   C *tw = stage + STAGES * G::stage_elems;
@@ -825,8 +928,25 @@ __device__ __forceinline__ void xpipe_nl_body(int vb, int nvb, const FieldMaps &
   for (int k = 0;; ++k) {
     const int tile = vb + k * nvb;
     if (tile >= ntiles) break;
-    C V[3][E], P[NOUT][E];
+    C V[3][E], P[NOUT][E], B[PHYS == 2 ? 3 : 1][E], Q[PHYS == 2 ? 3 : 1][E];
     bool failed = false;
+    // forward: the real-to-complex line of a product, written to output c
+    auto emit = [&](C(&x)[E], int c) {
+      line_fft<C, M, E, -1, 2>(x, t, tw, buf, sync);
+#pragma unroll
+      for (int e = 0; e < E; ++e) buf(t + T * e) = x[e];
+      __syncthreads();
+      C *obase = out.p[c] + (size_t)(tile % nzb) * BZ + (size_t)nz * (((tile / nzb) % nyg) * YB + yb) +
+                 rowstride * (size_t)((tile / nzb / nyg) * nxh) + l;
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const int kk = t + T * e;
+        const C zk = buf(kk), zm = buf((M - kk) & (M - 1));
+        if (kk < rows) obase[rowstride * kk] = r2c_unpack(zk, zm, tw[kk]);
+        if (kk == 0 && M < rows) obase[rowstride * M] = r2c_unpack(zk, zm, mk((R)-1, (R)0));
+      }
+      buf.flip();  // the next write goes to the other half
+    };
 #pragma unroll
     for (int f = 0; f < NIN; ++f) {
       const int L = k * NIN + f;
@@ -879,7 +999,36 @@ __device__ __forceinline__ void xpipe_nl_body(int vb, int nvb, const FieldMaps &
           P[1][e] = mk((x[e].x * V[0][e].x + P[1][e].x) * scale, (x[e].y * V[0][e].y + P[1][e].y) * scale);
           P[2][e] = mk(P[2][e].x * scale, P[2][e].y * scale);
         }
-      } else if constexpr (NOUT > 3) {
+      } else if constexpr (PHYS == 2) {
+        if (f < 9) {  // v x b, sent out before curl b comes in
+#pragma unroll
+          for (int e = 0; e < E; ++e) {
+            B[f - 6][e] = x[e];
+            if (f == 6) {
+              Q[1][e] = mk(V[2][e].x * x[e].x, V[2][e].y * x[e].y);
+              Q[2][e] = mk(-(V[1][e].x * x[e].x), -(V[1][e].y * x[e].y));
+            } else if (f == 7) {
+              Q[0][e] = mk(-(V[2][e].x * x[e].x), -(V[2][e].y * x[e].y));
+              Q[2][e] = mk((Q[2][e].x + V[0][e].x * x[e].x) * scale, (Q[2][e].y + V[0][e].y * x[e].y) * scale);
+            } else {
+              Q[0][e] = mk((Q[0][e].x + V[1][e].x * x[e].x) * scale, (Q[0][e].y + V[1][e].y * x[e].y) * scale);
+              Q[1][e] = mk((Q[1][e].x - V[0][e].x * x[e].x) * scale, (Q[1][e].y - V[0][e].y * x[e].y) * scale);
+            }
+          }
+          if (f == 8)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) emit(Q[c], c);
+        } else {
+          // minus j x b: (j x b)_c = j_{c+1} b_{c+2} - j_{c+2} b_{c+1}
+          const int c1 = (f - 9 + 2) % 3, c2 = (f - 9 + 1) % 3;  // j_d enters (j x b)_{d+2} with b_{d+1} and (j x b)_{d+1} with -b_{d+2}
+#pragma unroll
+          for (int e = 0; e < E; ++e) {
+            const C y = mk(x[e].x * scale, x[e].y * scale);
+            P[c1][e] = mk(P[c1][e].x - y.x * B[c2][e].x, P[c1][e].y - y.y * B[c2][e].y);
+            P[c2][e] = mk(P[c2][e].x + y.x * B[c1][e].x, P[c2][e].y + y.y * B[c1][e].y);
+          }
+        }
+      } else if constexpr (PHYS == 1) {
         // advect3 accumulates vx th_x + vy th_y + vz th_z, then times -1/(nx ny nz)^2
         if (f == 6) {
 #pragma unroll
@@ -897,25 +1046,8 @@ __device__ __forceinline__ void xpipe_nl_body(int vb, int nvb, const FieldMaps &
       }
     }
     if (failed) return;
-    // forward: real-to-complex lines of the products
-    C *obase = nullptr;
 #pragma unroll
-    for (int c = 0; c < NOUT; ++c) {
-      line_fft<C, M, E, -1, 2>(P[c], t, tw, buf, sync);
-#pragma unroll
-      for (int e = 0; e < E; ++e) buf(t + T * e) = P[c][e];
-      __syncthreads();
-      obase = out.p[c] + (size_t)(tile % nzb) * BZ + (size_t)nz * (((tile / nzb) % nyg) * YB + yb) +
-              rowstride * (size_t)((tile / nzb / nyg) * nxh) + l;
-#pragma unroll
-      for (int e = 0; e < E; ++e) {
-        const int kk = t + T * e;
-        const C zk = buf(kk), zm = buf((M - kk) & (M - 1));
-        if (kk < rows) obase[rowstride * kk] = r2c_unpack(zk, zm, tw[kk]);
-        if (kk == 0 && M < rows) obase[rowstride * M] = r2c_unpack(zk, zm, mk((R)-1, (R)0));
-      }
-      buf.flip();  // the next write goes to the other half
-    }
+    for (int c = 0; c < NOUT; ++c) emit(P[c], PHYS == 2 ? 3 + c : c);
   }
 }
 

@@ -673,6 +673,26 @@ def test_mhd(prec):
 
 
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("shape", [(16, 16, 16), (512, 16, 32), (16, 512, 32), (32, 16, 512), (1024, 16, 16)])
+def test_mhd_line_lengths(prec, shape):
+    """The fused MHD passes at the shortest and longest lines of each axis:
+    two RK2 steps (the first substep full, the others zero-pruned) from fields
+    with modes outside the truncation, v forced and a not."""
+    o = Oracle(*shape)
+    g = ghost(*shape, precision=prec)
+    cd = g.cdtype_np
+    v, a = ([x + 0.01 * rand_spectral(o, s + q) for q, x in enumerate(o.random_solenoidal(s, 1.0, 6.0, 1, amp)[0])]
+            for s, amp in ((61, 1.0), (62, 0.3)))
+    f = o.random_solenoidal(63, 2.0, 3.0, 0, 1.0)[0]
+    V, A, F = ([to_dev(x.astype(cd)) for x in q] for q in (v, a, f))
+    rv, ra = o.mhd_run(2, 2, 1e-3, 1e-3, 2e-3, v, a, f=f)
+    g.mhd_run(2, 2, 1e-3, 1e-3, 2e-3, *V, *A, f=F)
+    tol = 1e-11 if prec == "fp64" else 1e-5
+    assert rel_l2([to_host(x) for x in V], rv) <= tol
+    assert rel_l2([to_host(x) for x in A], ra) <= tol
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
 @pytest.mark.parametrize("shape", [(16, 16, 16), (32, 16, 64)])
 def test_phaseshift(prec, shape):
     o = Oracle(*shape)
