@@ -761,11 +761,15 @@ int bouss_substep_dev(ghost_ctx *c, int o, double dt, double nu, double kappa, d
   Fields<R> fy{};
   for (int q = 0; q < 9; ++q) fy.p[q] = (cx<R> *)w[q];
   GB_CHECK((launch_y<R, +1>(c, fy, 9, pr)));
-  GB_CHECK((launch_x<R, X_BOUSS>(c, nullptr, nullptr, (const void *const *)w, (void *const *)w, pr.rows)));
+  // -v.grad(theta) replaces grad theta's first component: the x pass may send
+  // it out before it reads the vorticity
+  void *const nl[4] = {w[0], w[1], w[2], w[6]};
+  GB_CHECK((launch_x<R, X_BOUSS>(c, nullptr, nullptr, (const void *const *)w, nl, pr.rows)));
+  for (int q = 0; q < 4; ++q) fy.p[q] = (cx<R> *)nl[q];
   GB_CHECK((launch_y<R, -1>(c, fy, 4, pr)));
   ZFwdBouss<R> zf{};
   for (int q = 0; q < 4; ++q) {
-    zf.nl.p[q] = (const cx<R> *)w[q];
+    zf.nl.p[q] = (const cx<R> *)nl[q];
     zf.v.p[q] = (cx<R> *)v[q];
     zf.c0.p[q] = (const cx<R> *)C[q];
     zf.f.p[q] = f ? (const cx<R> *)f[q] : nullptr;
@@ -800,12 +804,13 @@ int advect3_dev(ghost_ctx *c, const void *a, const void *b, const void *cc, cons
   Fields<R> fy{};
   for (int q = 0; q < 9; ++q) fy.p[q] = (cx<R> *)w[q];
   GB_CHECK((launch_y<R, +1>(c, fy, 9)));
-  GB_CHECK((launch_x<R, X_BOUSS>(c, nullptr, nullptr, (const void *const *)w, (void *const *)w)));
+  void *const nl[4] = {w[0], w[1], w[2], w[6]};
+  GB_CHECK((launch_x<R, X_BOUSS>(c, nullptr, nullptr, (const void *const *)w, nl)));
   Fields<R> f1{};
-  f1.p[0] = (cx<R> *)w[3];
+  f1.p[0] = (cx<R> *)w[6];
   GB_CHECK((launch_y<R, -1>(c, f1, 1)));
   ZC2C<R, -1, 1> zf{};
-  zf.in.p[0] = (const cx<R> *)w[3];
+  zf.in.p[0] = (const cx<R> *)w[6];
   zf.out.p[0] = (cx<R> *)e;
   return launch_z<R>(c, zf);
 }
@@ -2742,14 +2747,17 @@ template <typename R> static int ens_substep_multi(ghost_ensemble *e, int o, dou
     for (int q = 0; q < nc; ++q) {
       ghost_ctx *c = e->cls[q];
       XClass<R> &k = P.cl[q];
-      const int M = c->nx / 2, yb = ens_x_yb_of<R>(c->nx), bz = ens_xBZ<R>();
+      const bool wl = ens_warp_lines(c->nx);
+      const int M = c->nx / 2, yb = wl ? 1 : ens_x_yb_of<R>(c->nx), bz = wl ? ens_warp_BZ<R>() : ens_xBZ<R>();
       if (c->ny % yb != 0) return fail(GHOST_ERR_SIZE, "ny=%d not a multiple of the x tile's %d rows", c->ny, yb);
       const int nrows = pr[q].rows > 0 ? pr[q].rows : M + 1;
       const int nbox = (nrows + 255) / 256;
       const int align = std::max(1, 128 / (yb * bz * (int)sizeof(cx<R>)));
       const int rb = ((nrows + nbox - 1) / nbox + align - 1) / align * align;
       if (nbox * rb > M + 8 || rb > 256) return fail(GHOST_ERR_STATE, "x-pass box plan %d x %d exceeds the tile", nbox, rb);
-      for (int f = 0; f < 6; ++f) GB_CHECK(field_map(c, w[q][f], bz * U, yb, rb, &k.maps.m[f]));
+      for (int f = 0; f < 6; ++f)
+        GB_CHECK(field_map(c, w[q][f], bz * U, yb, rb, &k.maps.m[f],
+                           wl ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE));
       for (int f = 0; f < 3; ++f) k.out.p[f] = (cx<R> *)w[q][f];
       const R nn = (R)c->nx * (R)c->ny * (R)c->nz_glob;
       k.scale = (R)1 / (nn * nn);

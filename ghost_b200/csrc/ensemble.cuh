@@ -17,6 +17,7 @@
 // so the arithmetic of a line is the one of the class's own launch.
 #pragma once
 #include "passes.cuh"
+#include "xnl.cuh"
 
 namespace gb {
 
@@ -133,13 +134,42 @@ template <typename R, int NX> constexpr int ens_x_E() { return ens_xE<R>() < NX 
 template <typename R, int NX> constexpr int ens_x_yb() {
   return kEnsThreads / (ens_xBZ<R>() * (NX / 2 / ens_x_E<R, NX>()));
 }
+// Lines of 64 points and more run the warp-line body of their own launches
+// (xnl.cuh), in as many groups of its size as make up the CTA.  Its outputs
+// replace its first inputs, so one set of tensor maps serves both.
+constexpr bool ens_warp_lines(int nx) { return nx >= 64; }
+template <typename R> constexpr int ens_warp_BZ() { return sizeof(R) == 4 ? 16 : 8; }
+template <typename R, int NX> struct EnsWarp {
+  template <int LE> using G = XnlGeom<R, NX, 8, ens_warp_BZ<R>(), LE>;
+  static constexpr int NT = G<8>::NT, groups = kEnsThreads / NT;
+  static constexpr size_t group = (G<8>::fixed + kEnsXStages * G<8>::tile + 1023) / 1024 * 1024;
+  static_assert(groups * NT == kEnsThreads, "one CTA size for all classes");
+};
 template <typename R, int NX> constexpr size_t ens_x_smem() {
+  if constexpr (ens_warp_lines(NX)) return EnsWarp<R, NX>::groups * EnsWarp<R, NX>::group + 1024;
+  else
   return XGeom<R, NX, ens_xBZ<R>(), ens_x_yb<R, NX>()>::smem_bytes(kEnsXStages);
 }
 
 template <typename R, int NX> __device__ __forceinline__ void ens_x_run(const XClass<R> &k, int vb, int nvb) {
-  xpipe_nl_body<R, NX, ens_x_E<R, NX>(), ens_xBZ<R>(), 0, kEnsXStages, ens_x_yb<R, NX>()>(
-      vb, nvb, k.maps, k.out, k.tw, k.ny, k.nz, k.scale, k.rows, k.nbox, k.rb, k.nruns, k.nxh, k.ctl);
+  if constexpr (ens_warp_lines(NX)) {
+    using W = EnsWarp<R, NX>;
+    extern __shared__ unsigned char smem_raw[];
+    const int g = (int)threadIdx.x / W::NT;
+    unsigned char *sm = align1024(smem_raw) + g * W::group;
+    vb = vb * W::groups + g;
+    nvb *= W::groups;
+    constexpr int BZ = ens_warp_BZ<R>();
+    if (k.rows <= 6 * W::template G<6>::T)
+      xnl_body<R, NX, 8, BZ, 0, 6, kEnsXStages>(vb, nvb, g, sm, k.maps, k.maps, k.tw, k.ny, k.nz, k.scale, k.rows, k.nbox,
+                                                k.rb, k.nruns, k.nxh, k.ctl);
+    else
+      xnl_body<R, NX, 8, BZ, 0, 8, kEnsXStages>(vb, nvb, g, sm, k.maps, k.maps, k.tw, k.ny, k.nz, k.scale, k.rows, k.nbox,
+                                                k.rb, k.nruns, k.nxh, k.ctl);
+  } else {
+    xpipe_nl_body<R, NX, ens_x_E<R, NX>(), ens_xBZ<R>(), 0, kEnsXStages, ens_x_yb<R, NX>()>(
+        vb, nvb, k.maps, k.out, k.tw, k.ny, k.nz, k.scale, k.rows, k.nbox, k.rb, k.nruns, k.nxh, k.ctl);
+  }
 }
 
 template <typename R>

@@ -77,6 +77,11 @@ template <class K> int persistent_grid(ghost_ctx *c, K kern, int threads, size_t
 int field_map(ghost_ctx *c, const void *base, unsigned box0, unsigned box1, unsigned box2, CUtensorMap *out,
               CUtensorMapSwizzle swz = CU_TENSOR_MAP_SWIZZLE_NONE);
 PipeCtl pipe_ctl(ghost_ctx *c);
+// the fused X pass with lines kept inside a warp (xnl.cuh): whether it
+// takes this grid, and its launch (ins: v, curl v (, grad theta); rows: live
+// kx rows, 0 for all)
+bool xnl_takes(const ghost_ctx *c);
+int launch_xnl(ghost_ctx *c, bool bouss, const void *const *ins, void *const *outs, int rows);
 // FP64 partial sums owned by the context, grown on demand
 int partials(ghost_ctx *c, size_t n, double **out);
 // per-kernel timers around a launch (kind GHOST_TIMER_*)

@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "../../include/ghost_b200.h"
+#include "f32x2.cuh"
 #include "pipeline.cuh"
 
 namespace gb {
@@ -32,6 +33,11 @@ int fail(int code, const char *fmt, ...);
 using gb::fail;
 
 namespace mlp {
+
+using gb::add2;
+using gb::both;
+using gb::fma2;
+using gb::mul2;
 
 constexpr int NIN = GHOST_MLP_NIN, NH = GHOST_MLP_NHID, NOUT = GHOST_MLP_NOUT;
 constexpr int KIN = 16, KOUT = 16;  // padded widths of the input and output layers
@@ -115,26 +121,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
 #pragma unroll
   for (int q = 0; q < 16; ++q) v[q] = __uint_as_float(r[q]);
 }
-
-// Two FP32 operations in one issue slot (each rounded like its scalar form).
-__device__ __forceinline__ unsigned long long pk(float2 a) { return *reinterpret_cast<unsigned long long *>(&a); }
-__device__ __forceinline__ float2 upk(unsigned long long a) { return *reinterpret_cast<float2 *>(&a); }
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-  unsigned long long r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pk(a)), "l"(pk(b)));
-  return upk(r);
-}
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-  unsigned long long r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pk(a)), "l"(pk(b)));
-  return upk(r);
-}
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-  unsigned long long r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(pk(a)), "l"(pk(b)), "l"(pk(c)));
-  return upk(r);
-}
-__device__ __forceinline__ float2 both(float a) { return make_float2(a, a); }
 
 // GELU in its tanh form (Hendrycks and Gimpel, 2016):
 //   gelu(z) = z/2 (1 + tanh(c (z + a z^3))), c = sqrt(2/pi), a = 0.044715,

@@ -114,26 +114,20 @@ template <typename R, int NX, int KIND> int launch_x_n(ghost_ctx *c, const void 
     constexpr int YB = x_yb<R, NX, BZ>();
     GB_CHECK((launch_x_fused<R, NX, KIND, BZ, (YB * NT <= 128 ? 2 : 1)>(c, ins, outs, rows)));
   } else if constexpr (KIND == X_HD || KIND == X_BOUSS) {
-    // FP32 512-point lines: tiles of 16 z-values (128-byte rows, one CTA of
-    // 512 threads per SM) where nz allows, else BZ
-    if constexpr (sizeof(R) == 4 && NX == 512 && BZ == 8) {
-      if (c->nz % 16 == 0) {
-        GB_CHECK((launch_x_fused<R, NX, KIND, 16, 1>(c, ins, outs, rows)));
+    // lines of 64 points and more: the warp-line kernel (xnl.cuh) where it
+    // takes the grid; bit 8 of the tile variant asks for the 4-value tiles of
+    // FP32 at nx = 1024.  Left to the other kernel: shorter lines, FP64 at
+    // nx = 1024, and at FP32 a z-slab that is no multiple of 16 planes.
+    constexpr bool kBoth = sizeof(R) == 4 || NX < 64 || NX == 1024;
+    if constexpr (NX >= 64) {
+      if (!kBoth || (xnl_takes(c) && !(NX == 1024 && (c->tile_cfg & 256)))) {
+        GB_CHECK(launch_xnl(c, KIND == X_BOUSS, ins, outs, rows));
         timer_end(c, ts);
         return post_launch(c);
       }
     }
-    // FP32 1024-point lines: tiles of 8 z-values (64-byte rows instead of
-    // 32, one CTA of 512 threads per SM) where nz allows (bit 8 of the tile
-    // variant asks for the 4-value tiles)
-    if constexpr (sizeof(R) == 4 && NX == 1024 && BZ == 4) {
-      if (c->nz % 8 == 0 && !(c->tile_cfg & 256)) {
-        GB_CHECK((launch_x_fused<R, NX, KIND, 8, 1>(c, ins, outs, rows)));
-        timer_end(c, ts);
-        return post_launch(c);
-      }
-    }
-    GB_CHECK((launch_x_fused<R, NX, KIND, BZ, 2>(c, ins, outs, rows)));
+    if constexpr (kBoth)
+      GB_CHECK((launch_x_fused<R, NX, KIND, BZ, 2>(c, ins, outs, rows)));
   } else if (KIND == X_C2R && xw_plain_ok(c)) {
     GB_CHECK(launch_xw_c2r(c, in, out));
   } else if (KIND == X_R2C && xw_plain_ok(c)) {

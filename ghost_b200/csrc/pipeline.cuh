@@ -19,6 +19,11 @@ namespace gb {
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// The first 1024-byte boundary in dynamic shared memory.  Pointer arithmetic
+// only: rounding the address as an integer hides from the compiler that it is
+// shared memory, and every access becomes a generic load or store.
+__device__ __forceinline__ unsigned char *align1024(unsigned char *p) { return p + ((1024u - (smem_u32(p) & 1023u)) & 1023u); }
+
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }
@@ -64,6 +69,11 @@ __device__ __forceinline__ void tma_store_3d(const CUtensorMap *map, const void 
   asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];\n" ::"l"(
                    reinterpret_cast<uint64_t>(map)),
                "r"(smem_u32(src)), "r"(c0), "r"(c1), "r"(c2)
+               : "memory");
+}
+// Bulk store of bytes (a multiple of 16, both addresses 16-byte aligned).
+__device__ __forceinline__ void bulk_s2g(void *dst, const void *src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n" ::"l"(dst), "r"(smem_u32(src)), "r"(bytes)
                : "memory");
 }
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;\n" ::: "memory"); }

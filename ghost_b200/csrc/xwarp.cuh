@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(256, 2) xwarp_r2c_kernel(const __grid_constant
   constexpr int M = NX / 2, E = 8, T = 32, BZ = G::BZ;
   static_assert(M == E * T, "one warp per line: NX = 512");
   extern __shared__ unsigned char smem_raw[];
-  unsigned char *sm = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  unsigned char *sm = align1024(smem_raw);
   unsigned char *obuf = sm + STAGES * G::r2c_in;
   const int tid = threadIdx.x, lane = tid & 31, l = tid >> 5;
   XWRing rg(obuf + 2 * G::out_bytes, M, NX, STAGES, l);
@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(256, 2) xwarp_c2r_kernel(const __grid_constant
   constexpr int M = NX / 2, E = 8, T = 32, BZ = G::BZ;
   static_assert(M == E * T, "one warp per line: NX = 512");
   extern __shared__ unsigned char smem_raw[];
-  unsigned char *sm = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  unsigned char *sm = align1024(smem_raw);
   const int tid = threadIdx.x, lane = tid & 31, l = tid >> 5;
   XWRing rg(sm + STAGES * G::c2r_in, M, NX, STAGES, l);
   const int nzb = nz / BZ, ntiles = nzb * ny;

@@ -772,6 +772,33 @@ def test_bouss_fp32_with_512_point_x_lines(shape):
             assert all(torch.equal(a, b) for a, b in zip(V + [TH], first)), cfg
 
 
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("shape", [(64, 16, 16), (128, 16, 32), (256, 32, 16), (1024, 16, 32), (64, 256, 64)])
+def test_warp_line_x_pass(prec, shape):
+    """The fused X pass at every line length it keeps inside a warp, HD and
+    Boussinesq, one and several tiles per y, full (first substep, modes outside
+    the truncation) and zero-pruned substeps: two steps against the oracle."""
+    box = dict(Lx=1, Ly=1, Lz=0.5, arbsize=True)
+    o, ob = Oracle(*shape), Oracle(*shape, **box)
+    cd = np.complex128 if prec == "fp64" else np.complex64
+    tol = 1e-12 if prec == "fp64" else 1e-5
+    v0 = [x + 0.01 * rand_spectral(o, 70 + q) for q, x in enumerate(o.random_solenoidal(71, 1.0, 8.0, 1, 1.0)[0])]
+    th0 = rand_spectral(o, 75, 0.1)
+    g = ghost(*shape, precision=prec)
+    V = [to_dev(x.astype(cd)) for x in v0]
+    g.hd_run(2, 2, 1e-3, 2e-3, *V)
+    assert rel_l2([to_host(x) for x in V], o.hd_run(2, 2, 1e-3, 2e-3, v0)) <= tol
+    gb = ghost(*shape, precision=prec, **box)
+    V, TH = [to_dev(x.astype(cd)) for x in v0], to_dev(th0.astype(cd))
+    args = (2, 2.5e-4, 5e-4, 5e-4, 0.5, 8.0, 8.0)
+    gb.bouss_run(2, *args, *V, TH)
+    rv, rt = ob.bouss_run(2, *args, v0, th0)
+    assert rel_l2([to_host(x) for x in V] + [to_host(TH)], list(rv) + [rt]) <= tol
+    # maxabs through the fused passes
+    for kin in (0, 1, 2):
+        assert g.maxabs(*[to_dev(x.astype(cd)) for x in v0], kin) == pytest.approx(o.maxabs(*v0, kin), rel=1e-12 if prec == "fp64" else 2e-6)
+
+
 # ------------------------------------------------ rand = 2 forcing update
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])
 def test_forcing_slow_matches_oracle(prec):
