@@ -82,6 +82,8 @@ PipeCtl pipe_ctl(ghost_ctx *c);
 // kx rows, 0 for all)
 bool xnl_takes(const ghost_ctx *c);
 int launch_xnl(ghost_ctx *c, bool bouss, const void *const *ins, void *const *outs, int rows);
+// the Y pass with lines kept inside a warp (FP32, lines of 256 points or more; ywarp.cuh)
+template <int S> int launch_ywarp(ghost_ctx *c, const Fields<float> &f, int nf, const Prune &pr);
 // FP64 partial sums owned by the context, grown on demand
 int partials(ghost_ctx *c, size_t n, double **out);
 // per-kernel timers around a launch (kind GHOST_TIMER_*)

@@ -55,6 +55,10 @@ int launch_y_cfg(ghost_ctx *c, const Fields<R> &f, int nf, const Prune &pr) {
 
 // tiles 8 z-lines wide, or 16 with tile variant bit 0
 template <typename R, int N, int S> int launch_y_n(ghost_ctx *c, const Fields<R> &f, int nf, const Prune &pr) {
+  // FP32 lines of 256 points or more: the warp-line kernel, whatever the tile
+  // variant (its y bits choose between kernels of other line lengths)
+  if constexpr (sizeof(R) == 4 && N >= 256) return launch_ywarp<S>(c, f, nf, pr);
+  else {
   // the 16-wide tile needs two stages of 16 lines in shared memory; where
   // that does not fit (FP64, long lines) the variant falls back to 8
   constexpr int E = N < 8 ? N : 8, T = N / E;
@@ -63,23 +67,13 @@ template <typename R, int N, int S> int launch_y_n(ghost_ctx *c, const Fields<R>
   if constexpr (fits16) {
     if ((c->tile_cfg & 1) && c->nz >= 16) return launch_y_cfg<R, N, S, 16>(c, f, nf, pr);
   }
-  // bit 4 (FP32, lines of 256 points or more): 16 values per thread, two
-  // radix-8 butterflies per stage, half the threads per line
-  if constexpr (sizeof(R) == 4 && N >= 256) {
-    if (c->tile_cfg & 16) {
-      // bit 6 with bit 3: the inverse pass in tiles of 4 z-lines, four CTAs per SM
-      if constexpr (S > 0)
-        if ((c->tile_cfg & 72) == 72) return launch_y_cfg<R, N, S, 4, true, 16>(c, f, nf, pr);
-      if (c->tile_cfg & 8) return launch_y_cfg<R, N, S, 8, true, 16>(c, f, nf, pr);
-      return launch_y_cfg<R, N, S, 8, false, 16>(c, f, nf, pr);
-    }
-  }
   // bit 3: two stages and a second exchange buffer (one barrier per exchange)
   constexpr bool fits_dual = YGeom<R, N, E, 8, true>::smem_bytes(2) <= 113 * 1024;
   if constexpr (N >= 256 && fits_dual) {
     if (c->tile_cfg & 8) return launch_y_cfg<R, N, S, 8, true>(c, f, nf, pr);
   }
   return launch_y_cfg<R, N, S, 8>(c, f, nf, pr);
+  }
 }
 
 template <typename R, int S> int launch_y(ghost_ctx *c, const Fields<R> &f, int nf, const Prune &pr) {
