@@ -16,7 +16,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libghost_b200.so")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
-SOURCES = ["api.cu", "passes_x.cu", "passes_y.cu", "passes_z32.cu", "passes_z64.cu", "xnl.cu", "ywarp.cu", "reduce.cu", "mlp.cu", "les.cu", "io.cu", "ic_host.cpp"]
+SOURCES = ["api.cu", "passes_x.cu", "passes_y.cu", "passes_z32.cu", "passes_z64.cu", "xnl.cu", "xplain.cu", "ywarp.cu", "reduce.cu", "mlp.cu", "les.cu", "io.cu", "ic_host.cpp"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC",
               "-Xptxas", "-warn-spills"]

@@ -82,6 +82,13 @@ PipeCtl pipe_ctl(ghost_ctx *c);
 // kx rows, 0 for all)
 bool xnl_takes(const ghost_ctx *c);
 int launch_xnl(ghost_ctx *c, bool bouss, const void *const *ins, void *const *outs, int rows);
+// plain x transforms with lines kept inside a warp (xplain.cuh): whether they
+// take this grid, and their launches
+bool xline_takes(const ghost_ctx *c);
+int launch_xline_r2c(ghost_ctx *c, const void *in, void *out);
+int launch_xline_c2r(ghost_ctx *c, const void *in, void *out);
+bool xline_features_takes(const ghost_ctx *c, const void *x);
+int launch_xline_features(ghost_ctx *c, const void *const *spec, float *x, float gs, float delta);
 // the Y pass with lines kept inside a warp (FP32, lines of 256 points or more; ywarp.cuh)
 template <int S> int launch_ywarp(ghost_ctx *c, const Fields<float> &f, int nf, const Prune &pr);
 // FP64 partial sums owned by the context, grown on demand

@@ -132,6 +132,10 @@ template <typename R, int NX, int KIND> int launch_x_n(ghost_ctx *c, const void 
     GB_CHECK(launch_xw_c2r(c, in, out));
   } else if (KIND == X_R2C && xw_plain_ok(c)) {
     GB_CHECK(launch_xw_r2c(c, in, out));
+  } else if (KIND == X_C2R && xline_takes(c)) {
+    GB_CHECK(launch_xline_c2r(c, in, out));
+  } else if (KIND == X_R2C && xline_takes(c)) {
+    GB_CHECK(launch_xline_r2c(c, in, out));
   } else if (KIND == X_C2R) {
     const size_t smem = (size_t)(NX + (M + 1) * BZ + M * BZ) * sizeof(C);
     auto kern = xpass_c2r_kernel<R, NX, E, BZ>;
@@ -192,6 +196,12 @@ int grad9_features_dev(ghost_ctx *c, const void *const v[3], void *const spec[9]
   Fields<R> fy{};
   for (int q = 0; q < 9; ++q) fy.p[q] = (cx<R> *)spec[q];
   GB_CHECK((launch_y<R, +1>(c, fy, 9)));
+  if (xline_features_takes(c, x)) {
+    const int ts = timer_begin(c, GHOST_TIMER_X_C2R);
+    GB_CHECK(launch_xline_features(c, (const void *const *)spec, x, gs, delta));
+    timer_end(c, ts);
+    return post_launch(c);
+  }
   switch (c->nx) {
     case 16: return grad9_features_n<R, 16>(c, spec, x, gs, delta);
     case 32: return grad9_features_n<R, 32>(c, spec, x, gs, delta);

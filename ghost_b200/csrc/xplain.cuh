@@ -1,0 +1,234 @@
+// xplain.cuh -- plain x transforms and the LES closure's inputs with the
+// warp-line tools of xnl.cuh (fftp3d_real_to_complex / fftp3d_complex_to_real,
+// the x stage of fftp-3/fftp3D.fpp).
+//
+// A tile is BZ z-lines at one y; a line of NX real values is held by T lanes
+// of one warp as M = NX/2 complex ones.  Persistent groups stream tiles through
+// a ring of bulk copies; a slot is refilled by the last warp to read it.
+//   r2c       real lines come in as they lie (line-major), the half spectrum
+//             goes out by TMA from a swizzled kx-row tile;
+//   c2r       kx-row tiles in, each lane stores its real pairs;
+//   features  the nine gradients of a tile in turn, collected as the closure's
+//             rows x[point][10] in shared memory and sent out line by line.
+// Against one tile per block, real data scattered through shared memory and
+// (features) rows written four bytes at a time: 256 x 128 x 64 FP64 r2c 16.5
+// -> 8 us, inputs of a 128^3 closure 137 -> 53 us.
+#pragma once
+#include "xnl.cuh"
+
+namespace gb {
+
+template <typename R, int NX, int E, int BZ> struct XPlainGeom {
+  using G = XnlGeom<R, NX, E, BZ, E>;
+  // real lines: a phase's two lines (FP32, T < 32) or four (T = 4) start on other banks
+  static constexpr int PITCH = G::M * G::ES + (sizeof(R) == 8 ? 16 : (G::T < 32 ? 64 : 0));
+  static constexpr size_t line_tile = ((size_t)BZ * PITCH + 127) / 128 * 128;
+  static constexpr size_t tables = G::NW * G::xch + (size_t)(G::M + G::TW2 + G::TW3) * G::ES + 256 + 1024;
+  static constexpr size_t r2c(int st) { return st * line_tile + 2 * G::tile + tables; }
+  static constexpr size_t c2r(int st) { return st * G::tile + tables; }
+  static constexpr int ROWF = NX * 10 + 4;  // floats of a line's closure inputs
+  static constexpr size_t feat(int st) { return st * G::tile + (size_t)BZ * ROWF * 4 + tables; }
+};
+
+// Ring bookkeeping of a group: bounded waits, refills by the last reader.
+template <int STAGES, int NW> struct XRing {
+  uint64_t *full, *never;
+  unsigned *cnt;
+  __device__ __forceinline__ XRing(void *at, int tid) {
+    full = reinterpret_cast<uint64_t *>(at);
+    never = full + STAGES;
+    cnt = reinterpret_cast<unsigned *>(never + 1);
+    if (tid == 0) {
+      mbar_init(never, 1);
+      for (int q = 0; q < STAGES; ++q) {
+        mbar_init(&full[q], 1);
+        cnt[q] = 0;
+      }
+      fence_barrier_init();
+    }
+  }
+  __device__ __forceinline__ void wait(int L, int lane, const PipeCtl &ctl) const {
+    const uint32_t par = (uint32_t)(L / STAGES) & 1u;
+    uint64_t *bar = &full[L % STAGES];
+    const bool got = (!ctl.stall || L > 0 || injected_stall_wait(never, ctl.cap)) && mbar_wait(bar, par, ctl.cap);
+    if (!got) {
+      if (lane == 0) record_timeout(ctl.status);
+      mbar_wait(bar, par, kDrainPolls);
+    }
+  }
+  // every lane has read the slot of load L; true in one lane of the group, which refills it
+  __device__ __forceinline__ bool read(int L, int lane) const {
+    __syncwarp();
+    if (lane != 0) return false;
+    __threadfence_block();
+    if (NW > 1 && atomicAdd(&cnt[L % STAGES], 1u) % NW != NW - 1) return false;
+    __threadfence_block();
+    return true;
+  }
+};
+
+template <typename R, int NX, int E, int BZ, int STAGES>
+__global__ void __launch_bounds__(XnlGeom<R, NX, E, BZ, E>::NT)
+    xline_r2c_kernel(const R *__restrict__ in, const __grid_constant__ CUtensorMap cmap, const cx<R> *__restrict__ twg,
+                     int ny, int nz, int nbox, int rb, PipeCtl ctl) {
+  using C = cx<R>;
+  using G = XnlGeom<R, NX, E, BZ, E>;
+  using P = XPlainGeom<R, NX, E, BZ>;
+  constexpr int M = G::M, T = G::T, RB = G::RB, U = G::ES / 8;
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char *sm = align1024(smem_raw);
+  unsigned char *obuf = sm, *ibuf = sm + 2 * G::tile;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const XLine<R, NX, E, BZ> ln(tid, reinterpret_cast<C *>(ibuf + STAGES * P::line_tile), twg);
+  const XRing<STAGES, G::NW> ring(ln.tw3 + G::TW3, tid);
+  __syncthreads();
+  const int nzb = nz / BZ, ntiles = nzb * ny, bstep = rb & ~7;
+  auto issue = [&](int k) {
+    const int tile = blockIdx.x + k * gridDim.x;
+    if (tile >= ntiles) return;
+    const int s = k % STAGES;
+    fence_proxy_async();
+    mbar_arrive_expect_tx(&ring.full[s], BZ * NX * (uint32_t)sizeof(R));
+    for (int z = 0; z < BZ; ++z)
+      bulk_g2s(ibuf + s * P::line_tile + (size_t)z * P::PITCH,
+               in + (size_t)NX * ((size_t)(tile / nzb) + (size_t)ny * ((tile % nzb) * BZ + z)), NX * (uint32_t)sizeof(R),
+               &ring.full[s]);
+  };
+  if (tid == 0)
+    for (int k = 0; k < STAGES; ++k) issue(k);
+  for (int k = 0;; ++k) {
+    const int tile = blockIdx.x + k * gridDim.x;
+    if (tile >= ntiles) break;
+    ring.wait(k, lane, ctl);
+    const C *src = reinterpret_cast<const C *>(ibuf + (k % STAGES) * P::line_tile + (size_t)ln.z * P::PITCH) + ln.t;
+    C x[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) x[e] = src[T * e];
+    if (ring.read(k, lane)) issue(k + STAGES);
+    ln.template fft<-1>(x);
+#pragma unroll
+    for (int e = 0; e < E; ++e) x[e] = mul2(x[e], both((R)0.5));  // store_unpacked gives twice the spectrum
+    unsigned char *ob = obuf + (size_t)(k & 1) * G::tile;
+    ln.template store_unpacked<E>(x, ob);
+    fence_proxy_async();                 // the tile's generic writes, before the store reads them
+    if (tid == 0) bulk_wait_read_all();  // the store before this one has read its buffer
+    __syncthreads();
+    if (tid == 0) {
+      for (int q = 0; q < nbox; ++q) {
+        const int r0 = min(q * bstep, M + 1 - rb);
+        tma_store_3d(&cmap, ob + (size_t)r0 * RB, (tile % nzb) * BZ * U, tile / nzb, r0);
+      }
+      bulk_commit();
+    }
+  }
+  if (tid == 0) bulk_wait_all();
+}
+
+template <typename R, int NX, int E, int BZ, int STAGES>
+__global__ void __launch_bounds__(XnlGeom<R, NX, E, BZ, E>::NT)
+    xline_c2r_kernel(const __grid_constant__ CUtensorMap cmap, R *__restrict__ out, const cx<R> *__restrict__ twg, int ny,
+                     int nz, int nbox, int rb, PipeCtl ctl) {
+  using C = cx<R>;
+  using G = XnlGeom<R, NX, E, BZ, E>;
+  constexpr int M = G::M, T = G::T, RB = G::RB, U = G::ES / 8;
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char *sm = align1024(smem_raw);
+  const int tid = threadIdx.x, lane = tid & 31;
+  const XLine<R, NX, E, BZ> ln(tid, reinterpret_cast<C *>(sm + STAGES * G::tile), twg);
+  const XRing<STAGES, G::NW> ring(ln.tw3 + G::TW3, tid);
+  __syncthreads();
+  const int nzb = nz / BZ, ntiles = nzb * ny, bstep = rb & ~7;
+  auto issue = [&](int k) {
+    const int tile = blockIdx.x + k * gridDim.x;
+    if (tile >= ntiles) return;
+    const int s = k % STAGES;
+    fence_proxy_async();
+    mbar_arrive_expect_tx(&ring.full[s], (uint32_t)(nbox * rb) * RB);
+    for (int q = 0; q < nbox; ++q) {
+      const int r0 = min(q * bstep, M + 1 - rb);
+      tma_load_3d(sm + s * G::tile + (size_t)r0 * RB, &cmap, (tile % nzb) * BZ * U, tile / nzb, r0, &ring.full[s]);
+    }
+  };
+  if (tid == 0)
+    for (int k = 0; k < STAGES; ++k) issue(k);
+  for (int k = 0;; ++k) {
+    const int tile = blockIdx.x + k * gridDim.x;
+    if (tile >= ntiles) break;
+    ring.wait(k, lane, ctl);
+    C x[E];
+    ln.template load_packed<E>(x, sm + (k % STAGES) * G::tile);
+    if (ring.read(k, lane)) issue(k + STAGES);
+    ln.template fft<+1>(x);
+    C *row = reinterpret_cast<C *>(out + (size_t)NX * ((size_t)(tile / nzb) + (size_t)ny * ((tile % nzb) * BZ + ln.z))) + ln.t;
+#pragma unroll
+    for (int e = 0; e < E; ++e) row[T * e] = x[e];
+  }
+}
+
+// x[q][3a+b] = (real value / (nx ny nz)) * gs of the nine fields, x[q][9] = delta
+template <typename R, int NX, int E, int BZ, int STAGES>
+__global__ void __launch_bounds__(XnlGeom<R, NX, E, BZ, E>::NT)
+    xline_features_kernel(const __grid_constant__ FieldMaps maps, float *__restrict__ xrows,
+                          const cx<R> *__restrict__ twg, int ny, int nz, int nbox, int rb, R inv_n, float gs, float delta,
+                          PipeCtl ctl) {
+  using C = cx<R>;
+  using G = XnlGeom<R, NX, E, BZ, E>;
+  using P = XPlainGeom<R, NX, E, BZ>;
+  constexpr int M = G::M, T = G::T, RB = G::RB, U = G::ES / 8;
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char *sm = align1024(smem_raw);
+  float *st = reinterpret_cast<float *>(sm + STAGES * G::tile);
+  const int tid = threadIdx.x, lane = tid & 31;
+  const XLine<R, NX, E, BZ> ln(tid, reinterpret_cast<C *>(st + BZ * P::ROWF), twg);
+  const XRing<STAGES, G::NW> ring(ln.tw3 + G::TW3, tid);
+  for (int q = tid; q < BZ * NX; q += G::NT) st[(q / NX) * P::ROWF + (q % NX) * 10 + 9] = delta;  // stays from tile to tile
+  __syncthreads();
+  const int nzb = nz / BZ, ntiles = nzb * ny, bstep = rb & ~7;
+  auto issue = [&](int L) {
+    const int k = L / 9, f = L - 9 * k, tile = blockIdx.x + k * gridDim.x;
+    if (tile >= ntiles) return;
+    const int s = L % STAGES;
+    fence_proxy_async();
+    mbar_arrive_expect_tx(&ring.full[s], (uint32_t)(nbox * rb) * RB);
+    for (int q = 0; q < nbox; ++q) {
+      const int r0 = min(q * bstep, M + 1 - rb);
+      tma_load_3d(sm + s * G::tile + (size_t)r0 * RB, &maps.m[f], (tile % nzb) * BZ * U, tile / nzb, r0, &ring.full[s]);
+    }
+  };
+  if (tid == 0)
+    for (int L = 0; L < STAGES; ++L) issue(L);
+  float *mine = st + ln.z * P::ROWF + 20 * ln.t;
+  for (int k = 0;; ++k) {
+    const int tile = blockIdx.x + k * gridDim.x;
+    if (tile >= ntiles) break;
+#pragma unroll 1
+    for (int f = 0; f < 9; ++f) {
+      const int L = 9 * k + f;
+      ring.wait(L, lane, ctl);
+      C x[E];
+      ln.template load_packed<E>(x, sm + (L % STAGES) * G::tile);
+      if (ring.read(L, lane)) issue(L + STAGES);
+      ln.template fft<+1>(x);
+      if (f == 0) {  // the last tile's rows have left shared memory
+        if (tid == 0) bulk_wait_read_all();
+        __syncthreads();
+      }
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        mine[20 * T * e + f] = (float)(x[e].x * inv_n) * gs;
+        mine[20 * T * e + 10 + f] = (float)(x[e].y * inv_n) * gs;
+      }
+    }
+    fence_proxy_async();
+    __syncthreads();
+    if (tid == 0) {
+      for (int z = 0; z < BZ; ++z)
+        bulk_s2g(xrows + (size_t)10 * NX * ((size_t)(tile / nzb) + (size_t)ny * ((tile % nzb) * BZ + z)), st + z * P::ROWF,
+                 NX * 40);
+      bulk_commit();
+    }
+  }
+  if (tid == 0) bulk_wait_all();
+}
+
+}  // namespace gb

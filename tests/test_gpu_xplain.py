@@ -49,6 +49,29 @@ def test_plain_c2r_warp_lines(shape):
     assert bool((cin == keep).all())
 
 
+LINES = [("fp32", n) for n in (32, 64, 128, 256, 1024)] + [("fp64", n) for n in (32, 64, 128, 256, 512, 1024)]
+
+
+@pytest.mark.parametrize("prec,nx", LINES)
+def test_plain_lines_of_every_length(prec, nx):
+    """Both plain transforms at every other line length, on non-cubic grids
+    with one and with several tiles per y, against the oracle."""
+    from ghost_b200 import GHOST_COMPLEX_TO_REAL, GHOST_REAL_TO_COMPLEX
+    from tests.helpers import rand_real, rand_spectral
+    for ny, nz in ((16, 16), (32, 64)):
+        o = Oracle(nx, ny, nz)
+        g = ghost(nx, ny, nz, precision=prec)
+        tol = 1e-13 if prec == "fp64" else 2e-6
+        r, c = rand_real(o, 5), rand_spectral(o, 6)
+        fwd = g.fftp3d_create_plan((nx, ny, nz), GHOST_REAL_TO_COMPLEX)
+        inv = g.fftp3d_create_plan((nx, ny, nz), GHOST_COMPLEX_TO_REAL)
+        out, real = g.czeros(), g.rzeros()
+        g.fftp3d_real_to_complex(fwd, to_dev(r.astype(g.rdtype_np)), out)
+        assert rel_l2(to_host(out), o.fftp3d_real_to_complex(r)) < tol
+        g.fftp3d_complex_to_real(inv, to_dev(c.astype(g.cdtype_np)), real)
+        assert rel_l2(to_host(real), o.fftp3d_complex_to_real(c)) < tol
+
+
 def test_plain_timeout_reports_and_recovers():
     """With the stall injected the warp-line transforms record
     GHOST_ERR_TIMEOUT and finish; the context then works normally."""
