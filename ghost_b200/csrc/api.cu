@@ -983,31 +983,27 @@ template <typename R> int scale3_impl(ghost_ctx *c, void *x, void *y, void *z, d
   return post_launch(c);
 }
 
+// maxabs in three passes, its real fields never in memory (the separate
+// operators and transforms moved 33 fields, this 15)
 template <typename R> int maxabs_impl(ghost_ctx *c, const void *a, const void *b, const void *cc, double *d, int kin) {
-  // scratch 0: the complex-to-real intermediate; 1..3: spectral fields
-  // whose real-space norm is wanted; 4..6: their real-space values
-  void *w[7];
-  GB_CHECK(scratch(c, 7, w));
-  if (kin == 0) {
-    GB_CHECK(rotor3_impl<R>(c, b, cc, w[1], 1));
-    GB_CHECK(rotor3_impl<R>(c, a, cc, w[2], 2));
-    GB_CHECK(rotor3_impl<R>(c, a, b, w[3], 3));
-  } else if (kin == 1) {
-    GB_CHECK(laplak3_impl<R>(c, a, w[1]));
-    GB_CHECK(laplak3_impl<R>(c, b, w[2]));
-    GB_CHECK(laplak3_impl<R>(c, cc, w[3]));
-  } else {
-    GB_CUDA(cudaMemcpyAsync(w[1], a, c->cbytes, cudaMemcpyDeviceToDevice, c->stream));
-    GB_CUDA(cudaMemcpyAsync(w[2], b, c->cbytes, cudaMemcpyDeviceToDevice, c->stream));
-    GB_CUDA(cudaMemcpyAsync(w[3], cc, c->cbytes, cudaMemcpyDeviceToDevice, c->stream));
+  void *w[3];
+  GB_CHECK(scratch(c, 3, w));
+  ZNorm<R> zn{};
+  const void *in[3] = {a, b, cc};
+  Fields<R> fy{};
+  for (int q = 0; q < 3; ++q) {
+    zn.v.p[q] = (const cx<R> *)in[q];
+    fy.p[q] = zn.w.p[q] = (cx<R> *)w[q];
   }
-  for (int q = 0; q < 3; ++q) GB_CHECK(c2r_dev<R>(c, w[1 + q], w[4 + q]));
+  zn.kp = kparams<R>(c);
+  zn.kin = kin;
+  GB_CHECK(launch_z<R>(c, zn));
+  GB_CHECK((launch_y<R, +1>(c, fy, 3)));
   double *part;
   GB_CHECK(partials(c, 1, &part));
   GB_CUDA(cudaMemsetAsync(part, 0, sizeof(double), c->stream));
-  maxnorm_kernel<R><<<grid1d(c->nreal), 256, 0, c->stream>>>((const R *)w[4], (const R *)w[5], (const R *)w[6], c->nreal,
-                                                               (unsigned long long *)part);
-  GB_CHECK(post_launch(c));
+  void *out[1] = {part};
+  GB_CHECK((launch_x<R, X_NORM>(c, nullptr, nullptr, (const void *const *)w, out)));
   double m;
   GB_CUDA(cudaMemcpyAsync(&m, part, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   GB_CUDA(cudaStreamSynchronize(c->stream));

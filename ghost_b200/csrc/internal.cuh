@@ -51,7 +51,7 @@ struct Prune {
 };
 
 // X pass kinds
-enum XKind { X_HD = 0, X_C2R = 1, X_R2C = 2, X_BOUSS = 3, X_MHD = 4 };
+enum XKind { X_HD = 0, X_C2R = 1, X_R2C = 2, X_BOUSS = 3, X_MHD = 4, X_NORM = 5 };
 
 // the passes: Op of passes.cuh over z-lines; nf fields along y (in place);
 // an X pass of kind KIND (in, out: the plain transforms; ins, outs: the fused

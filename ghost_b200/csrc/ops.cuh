@@ -487,24 +487,4 @@ __global__ void __launch_bounds__(256) zprof_kernel(ZProfArgs<R> za, int op, siz
   if (threadIdx.x == 0) partials[(size_t)k * gridDim.y + blockIdx.y] = s;
 }
 
-// max over real space of sqrt(r1^2+r2^2+r3^2) (maxabs); non-negative
-// floats order like their bit patterns, so an integer max is exact.
-template <typename R>
-__global__ void maxnorm_kernel(const R *__restrict__ r1, const R *__restrict__ r2, const R *__restrict__ r3, size_t n,
-                               unsigned long long *out) {
-  R m = 0;
-  for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x) {
-    const R s = sqrt(r1[p] * r1[p] + r2[p] * r2[p] + r3[p] * r3[p]);
-    m = s > m ? s : m;
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    const R q = __shfl_down_sync(0xffffffffu, m, o);
-    m = q > m ? q : m;
-  }
-  if ((threadIdx.x & 31) == 0) {
-    const double md = (double)m;
-    atomicMax(out, (unsigned long long)__double_as_longlong(md));
-  }
-}
-
 }  // namespace gb

@@ -236,6 +236,50 @@ template <typename R, int PHYS> struct ZInv {
   }
 };
 
+// Inverse prologue of maxabs (pseudospec3D_hd.f90:939-1020): per mode the
+// field whose real-space norm is wanted, kin 0: curl v (rotor3), 1: laplak3 of
+// v, 2: v, with its inverse z transform.
+template <typename R> struct ZNorm {
+  using C = cx<R>;
+  static constexpr int NLOAD = 3;
+  CFields<R> v;  // 3
+  Fields<R> w;   // 3 outputs
+  KParams<R> kp;
+  int kin;
+  __device__ __forceinline__ const C *load_src(int f) const { return v.p[f]; }
+  template <int N, int E, class Buf, class Sync, class In>
+  __device__ __forceinline__ void body(long line, bool act, int t, const C *tw, Buf buf, Sync sync, In src) const {
+    constexpr int T = N / E;
+    const int j = (int)(line % kp.ny), i = (int)(line / kp.ny) % kp.nxh + kp.i0;
+    const R kx = kx_of(kp, i), ky = ky_of(kp, j);
+#pragma unroll
+    for (int f = 0; f < 3; ++f) {
+      C x[E];
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const int k = t + T * e;
+        if (kin == 0) {
+          const R kz = kz_of(kp, k), ka = f == 0 ? ky : (f == 1 ? kz : kx), kb = f == 0 ? kz : (f == 1 ? kx : ky);
+          const C a = src((f + 2) % 3)[k], b = src((f + 1) % 3)[k];  // i ka a - i kb b
+          x[e] = mk((-ka * a.y) - (-kb * b.y), (ka * a.x) - (kb * b.x));
+        } else {
+          x[e] = src(f)[k];
+          if (kin == 1) {
+            const R kk2 = kk2_of(kp, i, j, k);
+            x[e] = mk(-kk2 * x[e].x, -kk2 * x[e].y);
+          }
+        }
+      }
+      line_fft<C, N, E, +1>(x, t, tw, buf, sync);
+      if (act) {
+        C *dst = w.p[f] + (size_t)line * N;
+#pragma unroll
+        for (int e = 0; e < E; ++e) dst[t + T * e] = x[e];
+      }
+    }
+  }
+};
+
 // Inverse prologue of the MHD substep (include/mhd_rkstep2.f90): from v and
 // the vector potential a, per mode and with rotor3's operation order,
 //   w[0..2] = v, w[3..5] = curl v, w[6..8] = b = curl a, w[9..11] = curl b,
@@ -855,6 +899,9 @@ template <typename C> __device__ __forceinline__ C r2c_unpack(C zk, C zm, C w) {
 //   PHYS 2 (MHD):   in v, curl v, b, curl b (12)
 //                   -> out v x b (3), w x v - j x b (3) (vector3, and nonlin3's
 //                   difference of the two prodre3, pseudospec3D_mhd.f90:22-227)
+//   PHYS 3 (norm):  in three fields -> the largest |r| = sqrt(r1^2 + r2^2 + r3^2),
+//                   as the bits of a double, by atomicMax on out.p[0] (non-negative
+//                   doubles order like their bits, so the result is exact)
 // A persistent CTA walks (z-block, y) tiles.  Every input field of a tile
 // is one TMA tensor load (nbox boxes of rb kx-rows x BZ z-values) into a
 // STAGES-deep ring, so the next fields (and the next tile) stream in while
@@ -889,7 +936,7 @@ __device__ __forceinline__ void xpipe_nl_body(int vb, int nvb, const FieldMaps &
   using G = XGeom<R, NX, BZ, YB>;
   constexpr int M = NX / 2, T = M / E, NT = YB * BZ * T;
   constexpr int LW = YB * BZ;  // lines of a tile: (y, z) with z fastest
-  constexpr int NIN = PHYS == 0 ? 6 : (PHYS == 1 ? 9 : 12), NOUT = PHYS == 1 ? 4 : 3;
+  constexpr int NIN = PHYS == 0 ? 6 : (PHYS == 1 ? 9 : (PHYS == 2 ? 12 : 3)), NOUT = PHYS == 1 ? 4 : (PHYS == 3 ? 1 : 3);
   extern __shared__ __align__(128) unsigned char smem_raw[];
   C *stage = reinterpret_cast<C *>(smem_raw);
   C *tw = stage + STAGES * G::stage_elems;
@@ -925,11 +972,11 @@ __device__ __forceinline__ void xpipe_nl_body(int vb, int nvb, const FieldMaps &
   int ph = 0;
   auto buf = dual_buf<C>([xb, lw](int idx, int h) -> C & { return xb[(size_t)h * (M * LW) + idx * LW + lw]; }, &ph);
   auto sync = [] { __syncthreads(); };
+  R most = 0;  // PHYS 3
   for (int k = 0;; ++k) {
     const int tile = vb + k * nvb;
     if (tile >= ntiles) break;
-    C V[3][E], P[NOUT][E], B[PHYS == 2 ? 3 : 1][E], Q[PHYS == 2 ? 3 : 1][E];
-    bool failed = false;
+    C V[3][E], P[NOUT][E];
     // forward: the real-to-complex line of a product, written to output c
     auto emit = [&](C(&x)[E], int c) {
       line_fft<C, M, E, -1, 2>(x, t, tw, buf, sync);
@@ -947,14 +994,14 @@ __device__ __forceinline__ void xpipe_nl_body(int vb, int nvb, const FieldMaps &
       }
       buf.flip();  // the next write goes to the other half
     };
-#pragma unroll
-    for (int f = 0; f < NIN; ++f) {
+    // inverse: the complex-to-real line of input f, x[e] = (r_{2m}, r_{2m+1})
+    // at m = t + T*e; false when its wait timed out (the whole CTA agrees)
+    auto inverse = [&](int f, C(&x)[E]) -> bool {
       const int L = k * NIN + f;
       issue(L + STAGES - 1);
       const bool ok = (!ctl.stall || L > 0 || injected_stall_wait(&bars[STAGES], ctl.cap)) &&
                       mbar_wait(&bars[L % STAGES], (uint32_t)(L / STAGES) & 1u, ctl.cap);
       const C *sb = stage + (size_t)(L % STAGES) * G::stage_elems;
-      C x[E];
 #pragma unroll
       for (int e = 0; e < E; ++e) x[e] = c2r_pack(sb, LW, lw, t + T * e, M, rows, tw);
       // The CTA agrees on the wait at the transform's first exchange barrier,
@@ -973,41 +1020,81 @@ __device__ __forceinline__ void xpipe_nl_body(int vb, int nvb, const FieldMaps &
         for (int LL = L; LL < L + STAGES; ++LL)
           if (vb + (LL / NIN) * nvb < ntiles)
             mbar_wait(&bars[LL % STAGES], (uint32_t)(LL / STAGES) & 1u, kDrainPolls);
-        failed = true;
-        break;
       }
-      // x[e] = (r_{2m}, r_{2m+1}) at m = t + T*e
-      if (f < 3) {
+      return !bad;
+    };
+    // PHYS 2 loops where the live registers allow it: its eighteen lines
+    // unrolled are more code than the instruction cache holds
+    constexpr int UV = PHYS == 2 ? 1 : 3;
+#pragma unroll UV
+    for (int f = 0; f < 3; ++f) {
+      C x[E];
+      if (!inverse(f, x)) return;
 #pragma unroll
-        for (int e = 0; e < E; ++e) V[f][e] = x[e];
-      } else if (f == 3) {  // wx: (w x v)_y = wz vx - vz wx ; (w x v)_z = wx vy - vx wy
+      for (int e = 0; e < E; ++e) {
+        if constexpr (PHYS == 3) {
+          const C q = mk(x[e].x * x[e].x, x[e].y * x[e].y);
+          P[0][e] = f == 0 ? q : mk(P[0][e].x + q.x, P[0][e].y + q.y);
+          if (f == 2) {
+            const R a = sqrt(P[0][e].x), b = sqrt(P[0][e].y);
+            most = a > most ? a : most;
+            most = b > most ? b : most;
+          }
+        } else {
+          if (f == 0) V[0][e] = x[e];
+          else if (f == 1) V[1][e] = x[e];
+          else V[2][e] = x[e];
+        }
+      }
+    }
+    if constexpr (PHYS != 3) {
+#pragma unroll
+      for (int f = 0; f < 3; ++f) {
+        C x[E];
+        if (!inverse(3 + f, x)) return;
 #pragma unroll
         for (int e = 0; e < E; ++e) {
-          P[1][e] = mk(-(V[2][e].x * x[e].x), -(V[2][e].y * x[e].y));
-          P[2][e] = mk(x[e].x * V[1][e].x, x[e].y * V[1][e].y);
+          if (f == 0) {  // wx: (w x v)_y = wz vx - vz wx ; (w x v)_z = wx vy - vx wy
+            P[1][e] = mk(-(V[2][e].x * x[e].x), -(V[2][e].y * x[e].y));
+            P[2][e] = mk(x[e].x * V[1][e].x, x[e].y * V[1][e].y);
+          } else if (f == 1) {  // wy: (w x v)_x = wy vz - vy wz
+            P[0][e] = mk(x[e].x * V[2][e].x, x[e].y * V[2][e].y);
+            P[2][e] = mk(P[2][e].x - V[0][e].x * x[e].x, P[2][e].y - V[0][e].y * x[e].y);
+          } else {  // wz
+            P[0][e] = mk((P[0][e].x - V[1][e].x * x[e].x) * scale, (P[0][e].y - V[1][e].y * x[e].y) * scale);
+            P[1][e] = mk((x[e].x * V[0][e].x + P[1][e].x) * scale, (x[e].y * V[0][e].y + P[1][e].y) * scale);
+            P[2][e] = mk(P[2][e].x * scale, P[2][e].y * scale);
+          }
         }
-      } else if (f == 4) {  // wy: (w x v)_x = wy vz - vy wz
+      }
+      if constexpr (PHYS == 1) {
+        // advect3 accumulates vx th_x + vy th_y + vz th_z, then times -1/(nx ny nz)^2
 #pragma unroll
-        for (int e = 0; e < E; ++e) {
-          P[0][e] = mk(x[e].x * V[2][e].x, x[e].y * V[2][e].y);
-          P[2][e] = mk(P[2][e].x - V[0][e].x * x[e].x, P[2][e].y - V[0][e].y * x[e].y);
-        }
-      } else if (f == 5) {  // wz
-#pragma unroll
-        for (int e = 0; e < E; ++e) {
-          P[0][e] = mk((P[0][e].x - V[1][e].x * x[e].x) * scale, (P[0][e].y - V[1][e].y * x[e].y) * scale);
-          P[1][e] = mk((x[e].x * V[0][e].x + P[1][e].x) * scale, (x[e].y * V[0][e].y + P[1][e].y) * scale);
-          P[2][e] = mk(P[2][e].x * scale, P[2][e].y * scale);
-        }
-      } else if constexpr (PHYS == 2) {
-        if (f < 9) {  // v x b, sent out before curl b comes in
+        for (int f = 0; f < 3; ++f) {
+          C x[E];
+          if (!inverse(6 + f, x)) return;
 #pragma unroll
           for (int e = 0; e < E; ++e) {
-            B[f - 6][e] = x[e];
-            if (f == 6) {
+            C &q = P[NOUT - 1][e];
+            if (f == 0) q = mk(V[0][e].x * x[e].x, V[0][e].y * x[e].y);
+            else if (f == 1) q = mk(q.x + V[1][e].x * x[e].x, q.y + V[1][e].y * x[e].y);
+            else q = mk((q.x + V[2][e].x * x[e].x) * -scale, (q.y + V[2][e].y * x[e].y) * -scale);
+          }
+        }
+      }
+      if constexpr (PHYS == 2) {
+        C B[3][E], Q[3][E];
+#pragma unroll
+        for (int f = 0; f < 3; ++f) {  // v x b
+          C x[E];
+          if (!inverse(6 + f, x)) return;
+#pragma unroll
+          for (int e = 0; e < E; ++e) {
+            B[f][e] = x[e];
+            if (f == 0) {
               Q[1][e] = mk(V[2][e].x * x[e].x, V[2][e].y * x[e].y);
               Q[2][e] = mk(-(V[1][e].x * x[e].x), -(V[1][e].y * x[e].y));
-            } else if (f == 7) {
+            } else if (f == 1) {
               Q[0][e] = mk(-(V[2][e].x * x[e].x), -(V[2][e].y * x[e].y));
               Q[2][e] = mk((Q[2][e].x + V[0][e].x * x[e].x) * scale, (Q[2][e].y + V[0][e].y * x[e].y) * scale);
             } else {
@@ -1015,12 +1102,25 @@ __device__ __forceinline__ void xpipe_nl_body(int vb, int nvb, const FieldMaps &
               Q[1][e] = mk((Q[1][e].x - V[0][e].x * x[e].x) * scale, (Q[1][e].y - V[0][e].y * x[e].y) * scale);
             }
           }
-          if (f == 8)
+        }
+        // sent out before curl b comes in
+#pragma unroll 1
+        for (int c = 0; c < 3; ++c) {
+          C y[E];
 #pragma unroll
-            for (int c = 0; c < 3; ++c) emit(Q[c], c);
-        } else {
-          // minus j x b: (j x b)_c = j_{c+1} b_{c+2} - j_{c+2} b_{c+1}
-          const int c1 = (f - 9 + 2) % 3, c2 = (f - 9 + 1) % 3;  // j_d enters (j x b)_{d+2} with b_{d+1} and (j x b)_{d+1} with -b_{d+2}
+          for (int e = 0; e < E; ++e) {
+            y[e] = Q[0][e];
+            Q[0][e] = Q[1][e];
+            Q[1][e] = Q[2][e];
+          }
+          emit(y, c);
+        }
+        // minus j x b: j_d enters (j x b)_{d+2} with b_{d+1} and (j x b)_{d+1} with -b_{d+2}
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          const int c1 = (d + 2) % 3, c2 = (d + 1) % 3;
+          C x[E];
+          if (!inverse(9 + d, x)) return;
 #pragma unroll
           for (int e = 0; e < E; ++e) {
             const C y = mk(x[e].x * scale, x[e].y * scale);
@@ -1028,26 +1128,30 @@ __device__ __forceinline__ void xpipe_nl_body(int vb, int nvb, const FieldMaps &
             P[c2][e] = mk(P[c2][e].x + y.x * B[c1][e].x, P[c2][e].y + y.y * B[c1][e].y);
           }
         }
-      } else if constexpr (PHYS == 1) {
-        // advect3 accumulates vx th_x + vy th_y + vz th_z, then times -1/(nx ny nz)^2
-        if (f == 6) {
+#pragma unroll 1
+        for (int c = 0; c < 3; ++c) {
+          C y[E];
 #pragma unroll
-          for (int e = 0; e < E; ++e) P[NOUT - 1][e] = mk(V[0][e].x * x[e].x, V[0][e].y * x[e].y);
-        } else if (f == 7) {
-#pragma unroll
-          for (int e = 0; e < E; ++e)
-            P[NOUT - 1][e] = mk(P[NOUT - 1][e].x + V[1][e].x * x[e].x, P[NOUT - 1][e].y + V[1][e].y * x[e].y);
-        } else {
-#pragma unroll
-          for (int e = 0; e < E; ++e)
-            P[NOUT - 1][e] = mk((P[NOUT - 1][e].x + V[2][e].x * x[e].x) * -scale,
-                                (P[NOUT - 1][e].y + V[2][e].y * x[e].y) * -scale);
+          for (int e = 0; e < E; ++e) {
+            y[e] = P[0][e];
+            P[0][e] = P[1][e];
+            P[1][e] = P[2][e];
+          }
+          emit(y, 3 + c);
         }
+      } else {
+#pragma unroll
+        for (int c = 0; c < NOUT; ++c) emit(P[c], c);
       }
     }
-    if (failed) return;
-#pragma unroll
-    for (int c = 0; c < NOUT; ++c) emit(P[c], PHYS == 2 ? 3 + c : c);
+  }
+  if constexpr (PHYS == 3) {
+    for (int o = 16; o > 0; o >>= 1) {
+      const R q = __shfl_down_sync(0xffffffffu, most, o);
+      most = q > most ? q : most;
+    }
+    if ((tid & 31) == 0)
+      atomicMax(reinterpret_cast<unsigned long long *>(out.p[0]), (unsigned long long)__double_as_longlong((double)most));
   }
 }
 

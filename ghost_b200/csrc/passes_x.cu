@@ -22,8 +22,10 @@ int launch_x_fused(ghost_ctx *c, const void *const *ins, void *const *outs, int 
   if (c->ny % YB != 0) return fail(GHOST_ERR_SIZE, "ny=%d not a multiple of the x tile's %d rows", c->ny, YB);
   constexpr int M = NX / 2, T = M / E, NT = YB * BZ * T;
   typedef cx<R> C;
-  constexpr int PHYS = KIND == X_HD ? 0 : (KIND == X_BOUSS ? 1 : 2);
-  constexpr int NIN = PHYS == 0 ? 6 : (PHYS == 1 ? 9 : 12), NOUT = PHYS == 0 ? 3 : (PHYS == 1 ? 4 : 6);
+  constexpr int PHYS = KIND == X_HD ? 0 : (KIND == X_BOUSS ? 1 : (KIND == X_MHD ? 2 : 3));
+  constexpr int NIN = PHYS == 0 ? 6 : (PHYS == 1 ? 9 : (PHYS == 2 ? 12 : 3));
+  constexpr int NOUT = PHYS == 0 ? 3 : (PHYS == 1 ? 4 : (PHYS == 2 ? 6 : 1));
+  const int nruns = KIND == X_NORM ? 1 : c->nruns;  // maxabs is of the first run's field
   using G = XGeom<R, NX, BZ, YB>;
   constexpr size_t cap = 220 * 1024 / MINB;  // four stages while MINB CTAs fit an SM
   constexpr int STAGES = G::smem_bytes(4) <= cap ? 4 : (G::smem_bytes(3) <= 200 * 1024 ? 3 : 2);
@@ -42,9 +44,9 @@ int launch_x_fused(ghost_ctx *c, const void *const *ins, void *const *outs, int 
   const unsigned U = sizeof(R) == 4 ? 1 : 2;
   FieldMaps maps;
   for (int q = 0; q < NIN; ++q) GB_CHECK(field_map(c, ins[q], BZ * U, YB, rb, &maps.m[q]));
-  const int pgrid = persistent_grid(c, kern, NT, smem, (long)(c->nz / BZ) * (c->ny / YB) * c->nruns);
+  const int pgrid = persistent_grid(c, kern, NT, smem, (long)(c->nz / BZ) * (c->ny / YB) * nruns);
   kern<<<pgrid, NT, smem, c->stream>>>(maps, fo, (const C *)c->tw_x, c->ny, c->nz, (R)1 / (nn * nn), nrows, nbox, rb,
-                                       c->nruns, c->nxh, pipe_ctl(c));
+                                       nruns, c->nxh, pipe_ctl(c));
   return GHOST_OK;
 }
 
@@ -108,8 +110,10 @@ template <typename R, int NX, int KIND> int launch_x_n(ghost_ctx *c, const void 
   typedef cx<R> C;
   dim3 grid(c->nz / BZ, c->ny);
   const C *tw = (const C *)c->tw_x;
-  const int ts = timer_begin(c, KIND == X_C2R ? GHOST_TIMER_X_C2R : (KIND == X_R2C ? GHOST_TIMER_X_R2C : GHOST_TIMER_X_NL));
-  if constexpr (KIND == X_MHD) {
+  const int ts = timer_begin(c, KIND == X_C2R || KIND == X_NORM ? GHOST_TIMER_X_C2R : (KIND == X_R2C ? GHOST_TIMER_X_R2C : GHOST_TIMER_X_NL));
+  if constexpr (KIND == X_NORM) {
+    GB_CHECK((launch_x_fused<R, NX, KIND, BZ, 2>(c, ins, outs, rows)));
+  } else if constexpr (KIND == X_MHD) {
     // v, b and both products of a line live in registers: 255 a thread
     constexpr int YB = x_yb<R, NX, BZ>();
     GB_CHECK((launch_x_fused<R, NX, KIND, BZ, (YB * NT <= 128 ? 2 : 1)>(c, ins, outs, rows)));
@@ -218,6 +222,7 @@ int grad9_features_dev(ghost_ctx *c, const void *const v[3], void *const spec[9]
   template int launch_x<R, X_HD>(ghost_ctx *, const void *, void *, const void *const *, void *const *, int);       \
   template int launch_x<R, X_BOUSS>(ghost_ctx *, const void *, void *, const void *const *, void *const *, int);    \
   template int launch_x<R, X_MHD>(ghost_ctx *, const void *, void *, const void *const *, void *const *, int);      \
+  template int launch_x<R, X_NORM>(ghost_ctx *, const void *, void *, const void *const *, void *const *, int);     \
   template int launch_x<R, X_C2R>(ghost_ctx *, const void *, void *, const void *const *, void *const *, int);      \
   template int launch_x<R, X_R2C>(ghost_ctx *, const void *, void *, const void *const *, void *const *, int);      \
   template int grad9_features_dev<R>(ghost_ctx *, const void *const[3], void *const[9], float *, float, float);

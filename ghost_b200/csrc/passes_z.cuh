@@ -11,6 +11,7 @@ template <class Op> struct ZKind;
 template <typename R, int S, int NF> struct ZKind<ZC2C<R, S, NF>> { static constexpr int value = GHOST_TIMER_Z_C2C; };
 template <typename R, int P> struct ZKind<ZInv<R, P>> { static constexpr int value = GHOST_TIMER_Z_INV; };
 template <typename R> struct ZKind<ZGrad<R>> { static constexpr int value = GHOST_TIMER_Z_INV; };
+template <typename R> struct ZKind<ZNorm<R>> { static constexpr int value = GHOST_TIMER_Z_INV; };
 template <typename R> struct ZKind<ZInvMhd<R>> { static constexpr int value = GHOST_TIMER_Z_INV; };
 template <typename R> struct ZKind<ZFwdMhd<R>> { static constexpr int value = GHOST_TIMER_Z_FWD; };
 template <typename R> struct ZKind<ZFwdHD<R>> { static constexpr int value = GHOST_TIMER_Z_FWD; };
@@ -74,6 +75,7 @@ template <typename R, class Op> int launch_z(ghost_ctx *c, const Op &op, const P
   template int launch_z<R, ZGrad<R>>(ghost_ctx *, const ZGrad<R> &, const Prune &);       \
   template int launch_z<R, ZFwdHD<R>>(ghost_ctx *, const ZFwdHD<R> &, const Prune &);     \
   template int launch_z<R, ZFwdBouss<R>>(ghost_ctx *, const ZFwdBouss<R> &, const Prune &); \
+  template int launch_z<R, ZNorm<R>>(ghost_ctx *, const ZNorm<R> &, const Prune &);       \
   template int launch_z<R, ZInvMhd<R>>(ghost_ctx *, const ZInvMhd<R> &, const Prune &);   \
   template int launch_z<R, ZFwdMhd<R>>(ghost_ctx *, const ZFwdMhd<R> &, const Prune &);   \
   template int launch_z<R, ZC2C<R, -1, 1>>(ghost_ctx *, const ZC2C<R, -1, 1> &, const Prune &); \
