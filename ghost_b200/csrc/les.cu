@@ -146,9 +146,14 @@ __global__ void tau_force_kernel(KParams<R> kp, Spec6<R> T, Spec3<R> f, Spec3w<R
 // (nu + tve(ki)) times the Laplacian); tve 1-based in GHOST, tve[ki-1] here.
 // With tvh (heli = 1) the helicity eddy diffusivity adds tvh(ki) w_a, w =
 // curl v formed as rotor3 does (:25-27, the C5, C6, C19 of the update).
+// With ef it also keeps Eden (and with hf Hden) of include/edqnmhd_rkstep2.f90
+// :8-17, which vcorrect needs after the update: (|vx|^2+|vy|^2+|vz|^2) rmp per
+// mode, rmp = 1/n^6, and 2 rmp times kz (Re vx Im vy - Re vy Im vx) + ky (Re vz
+// Im vx - Re vx Im vz) + kx (Re vy Im vz - Re vz Im vy).
 template <typename R>
 __global__ void eddy_force_kernel(KParams<R> kp, Spec3<R> v, Spec3<R> f, Spec3w<R> o, const double *__restrict__ tve,
-                                  const double *__restrict__ tvh, int ntve, size_t total) {
+                                  const double *__restrict__ tvh, int ntve, size_t total, R *__restrict__ ef = nullptr,
+                                  R *__restrict__ hf = nullptr, R rmp = (R)0) {
   for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < total; p += (size_t)gridDim.x * blockDim.x) {
     const int k = (int)(p % kp.nz), j = (int)((p / kp.nz) % kp.ny), i = (int)(p / ((size_t)kp.nz * kp.ny));
     const R kn2 = kn2_of(kp, i, j, k);
@@ -161,6 +166,13 @@ __global__ void eddy_force_kernel(KParams<R> kp, Spec3<R> v, Spec3<R> f, Spec3w<
       nuh = (in && tvh) ? (R)tvh[ki - 1] : (R)0;
     }
     const cx<R> vx = v.p[0][p], vy = v.p[1][p], vz = v.p[2][p];
+    if (ef) ef[p] = (vx.x * vx.x + vx.y * vx.y + vy.x * vy.x + vy.y * vy.y + vz.x * vz.x + vz.y * vz.y) * rmp;
+    if (hf) {
+      const R t1 = kz_of(kp, k) * (vx.x * vy.y - vy.x * vx.y);
+      const R t2 = ky_of(kp, j) * (vz.x * vx.y - vx.x * vz.y);
+      const R t3 = kx_of(kp, i) * (vy.x * vz.y - vz.x * vy.y);
+      hf[p] = (R)2 * rmp * (t1 + t2 + t3);
+    }
     cx<R> w[3] = {};
     if (nuh != (R)0) {
       const R kx = kx_of(kp, i), ky = ky_of(kp, j), kz = kz_of(kp, k);
@@ -250,7 +262,7 @@ __device__ static void vc_phase(double r, double im, double eps, double *c, doub
   const double pi = 3.14159265358979323846;
   *c = r / (sqrt(r * r + im * im) + eps);
   *s = im / (sqrt(r * r + im * im) + eps);
-  *t = *s > 0. ? acos(*c) : 2.0 * pi - acos(*c);
+  if (t) *t = *s > 0. ? acos(*c) : 2.0 * pi - acos(*c);
 }
 /* the common energy ratio of the first branches */
 __device__ static double vc_ratio(double E, double H, double v2, double w2, double kk2) {
@@ -279,8 +291,7 @@ __device__ static void vc_rebuild3(double *v, double mx, double my, double mz, d
 }
 
 __device__ static void vc_vcorr_general(double kx, double ky, double kz, double kk2, double E, double H, double v2, double w2,
-                            double cx, double sx, double cy, double sy, double cz, double sz, double txy, double tzx,
-                            double tyz, double *v);
+                            double cx, double sx, double cy, double sy, double cz, double sz, double *v);
 
 /* One mode.  zx/zy/zz: the wavenumber component is zero (index 1 in the
  * Fortran).  kx..kz and kk2 are the GP tables; E and H as above. */
@@ -373,11 +384,13 @@ __device__ static void vc_vcorr_mode(int zx, int zy, int zz, double kx, double k
       }
     }
   } else {                   /* three components */
-    vc_phase(v[0], v[1], eps, &cx, &sx, &tx);
-    vc_phase(v[2], v[3], eps, &cy, &sy, &ty);
-    vc_phase(v[4], v[5], eps, &cz, &sz, &tz);
-    const double txy = ty - tx, tzx = tx - tz, tyz = tz - ty;
-    if (zx || zy || zz) {
+    // the angles enter where a component of k vanishes only
+    const bool angles = zx || zy || zz;
+    vc_phase(v[0], v[1], eps, &cx, &sx, angles ? &tx : nullptr);
+    vc_phase(v[2], v[3], eps, &cy, &sy, angles ? &ty : nullptr);
+    vc_phase(v[4], v[5], eps, &cz, &sz, angles ? &tz : nullptr);
+    if (angles) {
+      const double txy = ty - tx, tzx = tx - tz, tyz = tz - ty;
       /* one vanishing component of k (vcorr_x0ynzn, vcorr_xny0zn, vcorr_xnynz0):
        * the mode along that axis takes its share of E, the other two split
        * the rest in proportion to the other axes' k^2 */
@@ -439,15 +452,14 @@ __device__ static void vc_vcorr_mode(int zx, int zy, int zz, double kx, double k
         }
       }
     } else {
-      vc_vcorr_general(kx, ky, kz, kk2, E, H, v2, w2, cx, sx, cy, sy, cz, sz, txy, tzx, tyz, v);
+      vc_vcorr_general(kx, ky, kz, kk2, E, H, v2, w2, cx, sx, cy, sy, cz, sz, v);
     }
   }
 }
 
 // vcorr_xnynzn (:1377-1629): all components of k non-zero
 __device__ static void vc_vcorr_general(double kx, double ky, double kz, double kk2, double E, double H, double v2, double w2,
-                            double cx, double sx, double cy, double sy, double cz, double sz, double txy, double tzx,
-                            double tyz, double *v) {
+                            double cx, double sx, double cy, double sy, double cz, double sz, double *v) {
   const double kx2 = kx * kx, ky2 = ky * ky, kz2 = kz * kz;
   const double fx = 1. - kx2 / kk2, fy = 1. - ky2 / kk2, fz = 1. - kz2 / kk2;
   const double tmq = vc_ratio(E, H, v2, w2, kk2);
@@ -495,28 +507,8 @@ __device__ static void vc_vcorr_general(double kx, double ky, double kz, double 
                  my >= mx && my >= mz, mz >= mx && mz >= my);
     }
   }
-  (void)txy; (void)tzx; (void)tyz;
 }
 
-
-// Eden of include/edqnmhd_rkstep2.f90:8-10: (|vx|^2+|vy|^2+|vz|^2)/n^6 per
-// mode; with hf (heli = 1) also Hden of :11-17, 2/n^6 times
-// kz (Re vx Im vy - Re vy Im vx) + ky (Re vz Im vx - Re vx Im vz)
-// + kx (Re vy Im vz - Re vz Im vy)
-template <typename R>
-__global__ void eden_kernel(KParams<R> kp, Spec3<R> v, R *__restrict__ ef, R *__restrict__ hf, size_t total, R rmp) {
-  for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < total; p += (size_t)gridDim.x * blockDim.x) {
-    const cx<R> a = v.p[0][p], b = v.p[1][p], c = v.p[2][p];
-    ef[p] = (a.x * a.x + a.y * a.y + b.x * b.x + b.y * b.y + c.x * c.x + c.y * c.y) * rmp;
-    if (hf) {
-      const int k = (int)(p % kp.nz), j = (int)((p / kp.nz) % kp.ny), i = (int)(p / ((size_t)kp.nz * kp.ny));
-      const R t1 = kz_of(kp, k) * (a.x * b.y - b.x * a.y);
-      const R t2 = ky_of(kp, j) * (c.x * a.y - a.x * c.y);
-      const R t3 = kx_of(kp, i) * (b.x * c.y - c.x * b.y);
-      hf[p] = (R)2 * rmp * (t1 + t2 + t3);
-    }
-  }
-}
 
 // vcorrect over every resolved mode but the origin: tepq and eold are the
 // shell arrays of the substep's start (1-based shells stored at k-1), ef its
@@ -840,38 +832,144 @@ static void evedqnm_h(int n, R kmax, R kolmo, const double *Eold, const double *
   }
 }
 
-// Device: one thread fits the spectra and forms mu (go: 0 no closure, 1
+// spec_fit by one block: the logarithms and the extrapolated shells one
+// thread each, the sums by thread 0 in spec_fit's order, so the fit is the
+// same.  buf: 2 (n/2 + 1) values; power and ddelta come out in every thread.
+template <typename R>
+__device__ void spec_fit_block(int n, R kmax, const double *__restrict__ Ein, R delk, double *Efit, R *power_out,
+                               R *ddelta_out, R *buf) {
+  __shared__ R sh[4];  // power, ddelta, expo, which form
+  const R tinyf = (R)1e-15 < (R)0.1 / ((R)n * (R)n) ? (R)1e-15 : (R)0.1 / ((R)n * (R)n);
+  const int kc = (int)msqrt(kmax);
+  const int ktot = 3 * kc, ksup = kc;
+  const int kinf = (int)((R)kc - delk);
+  const int nfit = 3 * (n / 2 + 1);
+  const int tid = threadIdx.x, nt = blockDim.x;
+  R *li = buf, *le = buf + (n / 2 + 1);
+  const bool any = !(Ein[ksup - 1] <= (double)tinyf);
+  for (int k = tid; k < nfit; k += nt) Efit[k] = 0;
+  if (any)
+    for (int i = kinf + tid; i <= ksup; i += nt) {
+      li[i - kinf] = mlog((R)i);
+      le[i - kinf] = (R)mlog(Ein[i - 1] + (double)tinyf);
+    }
+  __syncthreads();
+  if (tid == 0) {
+    R power = -1, ddelta = -1, expo = 0, form = 0;
+    if (any) {
+      R x = 0, y = 0, z = 0, v = 0, w = 0, m = 0, nn = 0, o = 0, p = 0;
+      for (int i = kinf; i <= ksup; ++i) {
+        const R ii = (R)i, l = li[i - kinf], e = le[i - kinf];
+        x = x + (R)1;
+        y = y + l;
+        z = z + e;
+        v = v + l * e;
+        w = w + l * l;
+        m = m + ii;
+        nn = nn + ii * l;
+        o = o + ii * e;
+        p = p + ii * ii;
+      }
+      R pden = (w * p - nn * nn) * (x * nn - y * m) - (y * nn - w * m) * (y * p - m * nn);
+      R pnum = ((z * nn - v * m) * (y * p - m * nn) - (v * p - o * nn) * (x * nn - y * m));
+      R dden = x * nn - y * m;
+      if (pden != 0 && dden != 0) {
+        power = pnum / pden;
+        expo = ((z * nn - v * m) - power * (w * m - y * nn)) / dden;
+        ddelta = expo * x / m - power * y / m - z / m;
+      }
+      form = 1;  // the resolved shells as they are
+      if (power >= 0 && ddelta >= 0) {
+        expo = mexp(expo);
+        form = 2;  // and expo k^-power exp(-ddelta k) beyond
+      } else {
+        pden = y * y - w * x;
+        pnum = (v * x - y * z);
+        dden = x * y;
+        if (pden != 0 && dden != 0) {
+          power = pnum / pden;
+          expo = mexp((y * z + power * y * y) / dden);
+          form = 3;  // and expo k^-power beyond
+        }
+      }
+    }
+    sh[0] = power;
+    sh[1] = ddelta;
+    sh[2] = expo;
+    sh[3] = form;
+  }
+  __syncthreads();
+  const R power = sh[0], ddelta = sh[1], expo = sh[2], form = sh[3];
+  if (form >= 1)
+    for (int k = 1 + tid; k <= ksup; k += nt) Efit[k - 1] = Ein[k - 1];
+  if (form >= 2)
+    for (int k = ksup + 1 + tid; k <= ktot; k += nt) {
+      const R kk = (R)k;
+      Efit[k - 1] = form == 2 ? (double)(expo * mpow(kk, -power) * mexp(-ddelta * kk)) : (double)(expo * mpow(kk, -power) + tinyf);
+    }
+  *power_out = power;
+  *ddelta_out = ddelta;
+  __syncthreads();
+}
+
+// cusp_mu (half: full_cusp_prep) by one block: the running sums by thread 0
+// in order, the roots one thread each.
+template <typename R>
+__device__ bool cusp_mu_block(R kmax, R kolmo, double *Ext, double *Hxt, R *mu, bool half) {
+  const R lambda = (R)0.218f * mpow(kolmo, (R)1.5);
+  const int kc = (int)msqrt(kmax);
+  const int ktot = 3 * kc;
+  const bool go = Ext[kc] != 0.0;  // Ext(kc+1)
+  __syncthreads();
+  if (!go) return false;
+  if (half)
+    for (int k = 1 + (int)threadIdx.x; k <= ktot; k += (int)blockDim.x) {
+      Ext[k - 1] = 0.5 * Ext[k - 1];
+      Hxt[k - 1] = 0.5 * Hxt[k - 1];
+    }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    R en = 0;
+    mu[0] = 0;
+    for (int k = 1; k <= ktot; ++k) {
+      const R tmp = (R)(float)(k * k);
+      en = (R)((double)en + (double)tmp * Ext[k - 1]);
+      mu[k] = en;
+    }
+  }
+  __syncthreads();
+  for (int k = 1 + (int)threadIdx.x; k <= ktot; k += (int)blockDim.x) mu[k] = lambda * msqrt(mu[k]);
+  return true;
+}
+
+// Device: one block fits the spectra and forms mu (go: 0 no closure, 1
 // cusp, 2 full_cusp); then one block per shell k, its threads sharing the
 // p, partial sums combined in thread order.  Hold, thpq, tvh, Hxt are only
-// touched for hel = 1.
+// touched for hel = 1.  The fit is a chain of dependent operations: with the
+// logarithms, powers and roots spread over the block it is no
+// longer the substep's longest kernel; by one thread it took 21 us at 33 shells.
 template <typename R>
 __global__ void __launch_bounds__(128) edqnm_fit_kernel(int n, R kmax, R kolmo, const double *__restrict__ Eold,
                                                         const double *__restrict__ Hold, int hel, double *tepq,
                                                         double *thpq, double *tve, double *tvh, double *Ext,
                                                         double *Hxt, R *mu, int *go) {
+  extern __shared__ double fit_raw[];  // 2 (n/2 + 1) values
+  R *buf = reinterpret_cast<R *>(fit_raw);
   const int nb = n / 2 + 1, kc = (int)msqrt(kmax);
   for (int k = threadIdx.x; k < nb; k += blockDim.x) {
     tve[k] = tepq[k] = 0;
     if (hel == 1) thpq[k] = tvh[k] = 0;
   }
-  if (threadIdx.x == 0) {
-    const R delk = (R)3 * (R)kc / (R)4;
-    R power, ddelta;
-    if (hel == 1) {
-      R hpower, hddelta;
-      spec_fit<R>(n, kmax, Eold, delk - (R)2, Ext, &power, &ddelta);
-      spec_fit<R>(n, kmax, Hold, delk, Hxt, &hpower, &hddelta);
-      if (!(power > 0))
-        *go = 0;
-      else if (hpower > 0)
-        *go = full_cusp_prep<R>(kmax, kolmo, Ext, Hxt, mu) ? 2 : 0;
-      else
-        *go = cusp_mu<R>(kmax, kolmo, Ext, mu) ? 1 : 0;
-    } else {
-      spec_fit<R>(n, kmax, Eold, delk, Ext, &power, &ddelta);
-      *go = (power > 0) && cusp_mu<R>(kmax, kolmo, Ext, mu) ? 1 : 0;
-    }
+  const R delk = (R)3 * (R)kc / (R)4;
+  R power, ddelta, hpower = 0, hddelta;
+  spec_fit_block<R>(n, kmax, Eold, hel == 1 ? delk - (R)2 : delk, Ext, &power, &ddelta, buf);
+  if (hel == 1) spec_fit_block<R>(n, kmax, Hold, delk, Hxt, &hpower, &hddelta, buf);
+  int g = 0;
+  if (power > 0) {
+    const bool full = hel == 1 && hpower > 0;
+    if (cusp_mu_block<R>(kmax, kolmo, Ext, Hxt, mu, full)) g = full ? 2 : 1;
   }
+  if (threadIdx.x == 0) *go = g;
 }
 
 template <typename R>
@@ -1041,13 +1139,13 @@ static int tau_force_dev(ghost_les *L, const float *tau, float ts, const void *c
 // EDQNM closure on the device: kinetic spectrum -> evedqnm (one block) ->
 // eddy-viscous force; the host is not involved, so a substep does not wait
 template <typename R>
-static int eddy_force_dev(ghost_les *L, const void *const v[3], const void *const f[3], void *const o[3]) {
+static int eddy_force_dev(ghost_les *L, const void *const v[3], const void *const f[3], void *const o[3], bool eden) {
   ghost_ctx *c = L->c;
   const int nb = c->nx / 2 + 1;
   const int hel = L->heli;
   GB_CHECK(shells_dev<R>(c, 1u << RED_ENERGY_KIND, v[0], v[1], v[2], nullptr, nullptr, nullptr, L->Ek_dev, (R)0.501f));
   if (hel == 1) GB_CHECK(shells_dev<R>(c, 1u << RED_HELICITY_KIND, v[0], v[1], v[2], nullptr, nullptr, nullptr, L->Hk_dev, (R)0.501f));
-  edqnm_fit_kernel<R><<<1, 128, 0, c->stream>>>(c->nx, (R)c->kmax, (R)L->kolmo, L->Ek_dev, L->Hk_dev, hel,
+  edqnm_fit_kernel<R><<<1, 128, 2 * sizeof(R) * nb, c->stream>>>(c->nx, (R)c->kmax, (R)L->kolmo, L->Ek_dev, L->Hk_dev, hel,
                                                 L->tepq_dev, L->thpq_dev, L->tve_dev, L->tvh_dev, L->Ext_dev,
                                                 L->Hxt_dev, (R *)L->mu_dev, L->go_dev);
   GB_CHECK(post_launch(c));
@@ -1063,8 +1161,10 @@ static int eddy_force_dev(ghost_les *L, const void *const v[3], const void *cons
     fs.p[a] = f ? (const cx<R> *)f[a] : nullptr;
     os.p[a] = (cx<R> *)o[a];
   }
-  eddy_force_kernel<R><<<blocks(c->nspec), 256, 0, c->stream>>>(kparams<R>(c), vs, fs, os, L->tve_dev,
-                                                                  hel == 1 ? L->tvh_dev : nullptr, nb, c->nspec);
+  const R n3 = (R)c->nx * (R)c->ny * (R)c->nz;
+  eddy_force_kernel<R><<<blocks(c->nspec), 256, 0, c->stream>>>(
+      kparams<R>(c), vs, fs, os, L->tve_dev, hel == 1 ? L->tvh_dev : nullptr, nb, c->nspec, eden ? (R *)L->ef : nullptr,
+      eden && hel == 1 ? (R *)L->hf : nullptr, (R)1 / (n3 * n3));
   return post_launch(c);
 }
 
@@ -1093,9 +1193,11 @@ static int spectral_force_dev(ghost_les *L, const void *const v[3], const void *
   return post_launch(c);
 }
 
-// closure force of the selected model for the velocity v: o = f + F(v)
+// closure force of the selected model for the velocity v: o = f + F(v); eden:
+// EDQNM also keeps the per-mode energies (helicities) that vcorrect needs
 template <typename R>
-static int closure_force_dev(ghost_les *L, const void *const v[3], const void *const f[3], void *const o[3]) {
+static int closure_force_dev(ghost_les *L, const void *const v[3], const void *const f[3], void *const o[3],
+                             bool eden = false) {
   ghost_ctx *c = L->c;
   switch (L->model) {
     case GHOST_LES_MLP: {
@@ -1105,7 +1207,7 @@ static int closure_force_dev(ghost_les *L, const void *const v[3], const void *c
       return tau_force_dev<R>(L, L->y, L->ts, f, o);
     }
     case GHOST_LES_EDQNM:
-      return eddy_force_dev<R>(L, v, f, o);
+      return eddy_force_dev<R>(L, v, f, o, eden);
     case GHOST_LES_MLP_SPECTRAL:
       return spectral_force_dev<R>(L, v, f, o);
     default: {
@@ -1134,14 +1236,9 @@ static int les_run_dev(ghost_les *L, int nsteps, int ord, double dt, double nu, 
   // of the substep's start (edqnmhd_rkstep2.f90:8-10,63)
   const int nb = c->nx / 2 + 1;
   const R n3 = (R)c->nx * (R)c->ny * (R)c->nz;
-  const R rmp = (R)1 / (n3 * n3);
   const R tinyf = (R)1e-15 < (R)0.1 / ((R)c->nmax * (R)c->nmax) ? (R)1e-15 : (R)0.1 / ((R)c->nmax * (R)c->nmax);
-  Spec3<R> vr;
   Spec3w<R> vw;
-  for (int a = 0; a < 3; ++a) {
-    vr.p[a] = (const cx<R> *)v[a];
-    vw.p[a] = (cx<R> *)v[a];
-  }
+  for (int a = 0; a < 3; ++a) vw.p[a] = (cx<R> *)v[a];
   // the learned closure's fallback: each step starts from a saved copy, and a
   // step that ends non-finite or with <|v|^2> above blowup times its value at
   // the start of the call is redone with GHOST's EDQNM closure, which then
@@ -1157,13 +1254,8 @@ static int les_run_dev(ghost_les *L, int nsteps, int ord, double dt, double nu, 
         GB_CUDA(cudaMemcpyAsync(L->save[a], v[a], c->cbytes, cudaMemcpyDeviceToDevice, c->stream));
     const bool vcorr_step = L->model == GHOST_LES_EDQNM;
     for (int o = ord; o >= 1; --o) {
-      GB_CHECK(closure_force_dev<R>(L, v, f, L->force));
+      GB_CHECK(closure_force_dev<R>(L, v, f, L->force, vcorr_step));
       const int hel = vcorr_step ? L->heli : 0;
-      if (vcorr_step) {
-        eden_kernel<R><<<blocks(c->nspec), 256, 0, c->stream>>>(kparams<R>(c), vr, (R *)L->ef,
-                                                                hel == 1 ? (R *)L->hf : nullptr, c->nspec, rmp);
-        GB_CHECK(post_launch(c));
-      }
       GB_CHECK(hd_substep_dev<R>(c, o, dt, nu, v, L->rk, L->force, o == ord ? 1 : 0, !first));
       if (vcorr_step) {
         vcorrect_kernel<R><<<blocks(c->nspec), 256, 0, c->stream>>>(
