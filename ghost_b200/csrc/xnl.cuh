@@ -562,13 +562,22 @@ __device__ __forceinline__ void xnl_body(int vb, int nvb, int g, unsigned char *
         }
       }
     }
+    // The FP32 pass of six loads is short enough to keep its three emissions
+    // unrolled (128^3: 117 -> 111 us a step); with nine loads that was 22.7 -> 27.7 ms
+    // at 1024 x 1024 x 256.
+    if constexpr (PHYS == 0 && sizeof(R) == 4) {
+      emit(P[0], tile, 0);
+      emit(P[1], tile, 1);
+      emit(P[2], tile, 2);
+    } else {
 #pragma unroll 1
-    for (int c = 0; c < 3; ++c) {
-      emit(P[0], tile, c);
+      for (int c = 0; c < 3; ++c) {
+        emit(P[0], tile, c);
 #pragma unroll
-      for (int e = 0; e < E; ++e) {
-        P[0][e] = P[1][e];
-        P[1][e] = P[2][e];
+        for (int e = 0; e < E; ++e) {
+          P[0][e] = P[1][e];
+          P[1][e] = P[2][e];
+        }
       }
     }
   }
