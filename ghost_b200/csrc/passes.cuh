@@ -79,6 +79,7 @@ __device__ __forceinline__ void zpipe_body(int vb, int nvb, const Op &op, const 
   uint64_t *bars = reinterpret_cast<uint64_t *>(xb + 2 * LPB * NP);
   const int tid = threadIdx.x, lq = tid / T, t = tid - lq * T;
   const int ntiles = (nlines + LPB - 1) / LPB;
+  dep_go();
   if (tid == 0) {
     for (int q = 0; q <= STAGES; ++q) mbar_init(&bars[q], 1);  // bars[STAGES]: never completed
     fence_barrier_init();
@@ -108,6 +109,7 @@ __device__ __forceinline__ void zpipe_body(int vb, int nvb, const Op &op, const 
                  N * (uint32_t)sizeof(C), &bars[s]);
     }
   };
+  dep_wait();
   for (int k = 0; k < STAGES - 1; ++k) issue(k);
   C *mine = xb + lq * NP;
   int ph = 0;
@@ -681,6 +683,7 @@ __device__ __forceinline__ void ypipe_body(int vb, int nvb, const FieldMaps &map
   const int nzb = nz / BZ;
   const int nig = (ni + KB - 1) / KB;  // groups of KB kx indices
   const int ntiles = nzb * nig * nruns * nf;
+  dep_go();
   if (tid == 0) {
     for (int q = 0; q <= STAGES; ++q) mbar_init(&bars[q], 1);  // bars[STAGES]: never completed
     fence_barrier_init();
@@ -741,6 +744,7 @@ __device__ __forceinline__ void ypipe_body(int vb, int nvb, const FieldMaps &map
       }
     }
   };
+  dep_wait();
   for (int k = 0; k < STAGES - 1; ++k) issue(k);
   auto sync = [] { __syncthreads(); };
   for (int k = 0;; ++k) {
@@ -948,6 +952,7 @@ __device__ __forceinline__ void xpipe_nl_body(int vb, int nvb, const FieldMaps &
   const int nzb = nz / BZ, nyg = ny / YB;
   const int ntiles = nzb * nyg * nruns;
   const size_t rowstride = (size_t)nz * ny;
+  dep_go();
   if (tid == 0) {
     for (int q = 0; q <= STAGES; ++q) mbar_init(&bars[q], 1);  // bars[STAGES]: never completed
     fence_barrier_init();
@@ -968,6 +973,7 @@ __device__ __forceinline__ void xpipe_nl_body(int vb, int nvb, const FieldMaps &
       tma_load_3d(dst + (size_t)q * rb * LW, &maps.m[f], (tile % nzb) * BZ * U, ((tile / nzb) % nyg) * YB,
                   (tile / nzb / nyg) * nxh + q * rb, &bars[s]);
   };
+  dep_wait();
   for (int L = 0; L < STAGES - 1; ++L) issue(L);
   int ph = 0;
   auto buf = dual_buf<C>([xb, lw](int idx, int h) -> C & { return xb[(size_t)h * (M * LW) + idx * LW + lw]; }, &ph);

@@ -45,8 +45,8 @@ int launch_x_fused(ghost_ctx *c, const void *const *ins, void *const *outs, int 
   FieldMaps maps;
   for (int q = 0; q < NIN; ++q) GB_CHECK(field_map(c, ins[q], BZ * U, YB, rb, &maps.m[q]));
   const int pgrid = persistent_grid(c, kern, NT, smem, (long)(c->nz / BZ) * (c->ny / YB) * nruns);
-  kern<<<pgrid, NT, smem, c->stream>>>(maps, fo, (const C *)c->tw_x, c->ny, c->nz, (R)1 / (nn * nn), nrows, nbox, rb,
-                                       nruns, c->nxh, pipe_ctl(c));
+  GB_CHECK(launch_dep(c, NIN, kern, pgrid, NT, smem, maps, fo, (const C *)c->tw_x, c->ny, c->nz, (R)1 / (nn * nn), nrows,
+                      nbox, rb, nruns, c->nxh, pipe_ctl(c)));
   return GHOST_OK;
 }
 
@@ -81,7 +81,7 @@ static int launch_xw_r2c(ghost_ctx *c, const void *in, void *out) {
   GB_CHECK(real_map(c, in, &rm));
   GB_CHECK(field_map(c, out, 8, 1, rb, &cm, CU_TENSOR_MAP_SWIZZLE_64B));
   const int grid = persistent_grid(c, kern, 256, G::r2c_bytes, (long)(c->nz / 8) * c->ny);
-  kern<<<grid, 256, G::r2c_bytes, c->stream>>>(rm, cm, (const float2 *)c->tw_x, c->ny, c->nz, rb, pipe_ctl(c));
+  GB_CHECK(launch_dep(c, 1, kern, grid, 256, G::r2c_bytes, rm, cm, (const float2 *)c->tw_x, c->ny, c->nz, rb, pipe_ctl(c)));
   return GHOST_OK;
 }
 static int launch_xw_c2r(ghost_ctx *c, const void *in, void *out) {
@@ -94,8 +94,7 @@ static int launch_xw_c2r(ghost_ctx *c, const void *in, void *out) {
   CUtensorMap m;
   GB_CHECK(field_map(c, in, 8, 1, rb, &m, CU_TENSOR_MAP_SWIZZLE_64B));
   const int grid = persistent_grid(c, kern, 256, G::c2r_bytes, (long)(c->nz / 8) * c->ny);
-  kern<<<grid, 256, G::c2r_bytes, c->stream>>>(m, (float *)out, (const float2 *)c->tw_x, c->ny, c->nz, nbox, rb,
-                                               pipe_ctl(c));
+  GB_CHECK(launch_dep(c, 1, kern, grid, 256, G::c2r_bytes, m, (float *)out, (const float2 *)c->tw_x, c->ny, c->nz, nbox, rb, pipe_ctl(c)));
   return GHOST_OK;
 }
 

@@ -47,8 +47,7 @@ int launch_y_cfg(ghost_ctx *c, const Fields<R> &f, int nf, const Prune &pr) {
   if (DUAL)
     for (int q = 0; q < nf; ++q) GB_CHECK(field_map(c, f.p[q], BZ * U, rbo, 1, &omaps.m[q]));
   const int ts = timer_begin(c, S > 0 ? GHOST_TIMER_Y_INV : GHOST_TIMER_Y_FWD);
-  kern<<<grid, KB * BZ * T, smem, c->stream>>>(maps, DUAL ? omaps : maps, f, (const cx<R> *)c->tw_y, c->nz, ni, nf,
-                                          c->nruns, c->nxh, pr.jpos, pr.jneg, rb, rbo, pipe_ctl(c));
+  GB_CHECK(launch_dep(c, nf, kern, grid, KB * BZ * T, smem, maps, DUAL ? omaps : maps, f, (const cx<R> *)c->tw_y, c->nz, ni, nf, c->nruns, c->nxh, pr.jpos, pr.jneg, rb, rbo, pipe_ctl(c)));
   timer_end(c, ts);
   return post_launch(c);
 }

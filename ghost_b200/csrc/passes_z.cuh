@@ -28,14 +28,11 @@ int launch_z_cfg(ghost_ctx *c, const Op &op, const Prune &pr) {
   GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int grid = persistent_grid(c, kern, LPB * T, smem, (nlines + LPB - 1) / LPB);
   const int ts = timer_begin(c, ZKind<Op>::value);
-  kern<<<grid, LPB * T, smem, c->stream>>>(op, (const cx<R> *)c->tw_z, pr.lines, nlines, pipe_ctl(c));
+  GB_CHECK(launch_dep(c, Op::NLOAD, kern, grid, LPB * T, smem, op, (const cx<R> *)c->tw_z, pr.lines, nlines, pipe_ctl(c)));
   timer_end(c, ts);
   return post_launch(c);
 }
 
-// CTAs of 256 threads; with tile variant bit 1 of 128 threads; with bits 1
-// and 2 of 128 threads with a two-stage ring and at most 170 registers, so
-// that three CTAs share an SM (lines of 256 points or more)
 // lines per CTA, halved from want until a two-stage ring of NL fields fits
 template <typename R, int N, int NL> constexpr int fit_lines(int want) {
   int lpb = want;
@@ -44,13 +41,34 @@ template <typename R, int N, int NL> constexpr int fit_lines(int want) {
   return lpb;
 }
 
+// whether the one-stage ring with four CTAs per SM is an Op's better one
+// (512^3 FP32: z_fwd 0.649 -> 0.596 ms, z_inv 0.569 -> 0.562; 1024 x 1024 x 256
+// Boussinesq: 2.10 -> 1.91 and 1.77 -> 1.56).  Not for the plain transforms
+// (0.178 -> 0.199 ms at 512^3 FP32) and the FP64 inverse (0.235 -> 0.238 at 256^3).
+template <class Op> struct OneStage { static constexpr bool value = true; };
+template <typename R, int S, int NF> struct OneStage<ZC2C<R, S, NF>> { static constexpr bool value = false; };
+template <int P> struct OneStage<ZInv<double, P>> { static constexpr bool value = false; };
+
+// CTAs of 256 threads; with tile variant bit 1 of 128 threads; with bits 1
+// and 2, for lines of 256 points or more, of 128 threads with a two-stage ring
+// and at most 170 registers, so that three CTAs share an SM; with bit 5 too
+// with a one-stage ring and four CTAs.  Passes of few lines take smaller CTAs,
+// so that every SM has work: 64 threads below two tiles of 128 per SM (a 64^3
+// FP64 step: 740 live lines were 47 CTAs of 256 threads).
 template <typename R, int N, class Op> int launch_z_n(ghost_ctx *c, const Op &op, const Prune &pr) {
   constexpr int E = zE<R>() < N ? zE<R>() : N, T = N / E;
   constexpr int L256 = fit_lines<R, N, Op::NLOAD>(256 / T > 0 ? 256 / T : 1);
   constexpr int L128 = fit_lines<R, N, Op::NLOAD>(128 / T > 0 ? 128 / T : 1);
+  constexpr int L64 = fit_lines<R, N, Op::NLOAD>(64 / T > 0 ? 64 / T : 1);
   if constexpr (N >= 256 && L128 != L256) {
-    if ((c->tile_cfg & 38) == 38) return launch_z_cfg<R, N, L128, 1, 4>(c, op, pr);
+    if constexpr (OneStage<Op>::value)
+      if ((c->tile_cfg & 38) == 38) return launch_z_cfg<R, N, L128, 1, 4>(c, op, pr);
     if ((c->tile_cfg & 6) == 6) return launch_z_cfg<R, N, L128, 2, 3>(c, op, pr);
+  }
+  if constexpr (N < 256 && L64 != L128) {
+    const int nlines = pr.lines ? pr.nlines : c->ny * c->nxh * c->nruns;
+    if (nlines < 2 * L128 * sm_count(c)) return launch_z_cfg<R, N, L64, 3, 1>(c, op, pr);
+    if (nlines < 2 * L256 * sm_count(c)) return launch_z_cfg<R, N, L128, 3, 1>(c, op, pr);
   }
   if ((c->tile_cfg & 2) && L128 != L256) return launch_z_cfg<R, N, L128, 3, 1>(c, op, pr);
   return launch_z_cfg<R, N, L256, 3, 1>(c, op, pr);

@@ -82,6 +82,13 @@ __device__ __forceinline__ void bulk_wait_read_all() { asm volatile("cp.async.bu
 // ... and have completed
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory"); }
 
+// A pass launched with launch_dep starts while the pass before it ends:
+// dep_wait() returns once every grid before this one has completed and its
+// memory operations are visible (every thread calls it before it touches a
+// field), dep_go() lets the next pass start its own prologue.
+__device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+__device__ __forceinline__ void dep_go() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+
 // Hint: bring the 32-byte sector holding p into L2.
 __device__ __forceinline__ void prefetch_l2(const void *p) {
   asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p));

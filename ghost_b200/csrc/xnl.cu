@@ -24,8 +24,8 @@ static int launch(ghost_ctx *c, const void *const *ins, void *const *outs, int r
   for (int q = 0; q < NOUT; ++q) GB_CHECK(field_map(c, outs[q], BZ * U, 1, bx.rb, &omaps.m[q], swz));
   const R nn = (R)c->nx * (R)c->ny * (R)c->nz_glob;
   const int grid = persistent_grid(c, kern, G::NT, smem, (long)(c->nz / BZ) * c->ny * c->nruns);
-  kern<<<grid, G::NT, smem, c->stream>>>(maps, omaps, (const cx<R> *)c->tw_x, c->ny, c->nz, (R)1 / (nn * nn), rows,
-                                         bx.nbox, bx.rb, c->nruns, c->nxh, pipe_ctl(c));
+  GB_CHECK(launch_dep(c, NIN, kern, grid, G::NT, smem, maps, omaps, (const cx<R> *)c->tw_x, c->ny, c->nz, (R)1 / (nn * nn),
+                      rows, bx.nbox, bx.rb, c->nruns, c->nxh, pipe_ctl(c)));
   return GHOST_OK;
 }
 

@@ -435,6 +435,7 @@ __device__ __forceinline__ void xnl_body(int vb, int nvb, int g, unsigned char *
     else named_sync(1 + g, NT);
   };
   const int nzb = nz / BZ, ntiles = nzb * ny * nruns;
+  dep_go();
   if (tid == 0) {
     mbar_init(never, 1);
     for (int q = 0; q < STAGES; ++q) {
@@ -466,6 +467,7 @@ __device__ __forceinline__ void xnl_body(int vb, int nvb, int g, unsigned char *
                   (tile / nzb / ny) * nxh + r0, &full[s]);
     }
   };
+  dep_wait();
   if (tid == 0)
     for (int L = 0; L < STAGES; ++L) issue(L);
   int nout = 0;

@@ -30,8 +30,7 @@ template <typename R, int NX, int E, int BZ> static int r2c(ghost_ctx *c, const 
   CUtensorMap m;
   GB_CHECK(field_map(c, out, BZ * G::ES / 8, 1, bx.rb, &m, swizzle_of(G::RB)));
   const int grid = persistent_grid(c, kern, G::NT, smem, (long)(c->nz / BZ) * c->ny);
-  kern<<<grid, G::NT, smem, c->stream>>>((const R *)in, m, (const cx<R> *)c->tw_x, c->ny, c->nz, bx.nbox, bx.rb,
-                                         pipe_ctl(c));
+  GB_CHECK(launch_dep(c, 1, kern, grid, G::NT, smem, (const R *)in, m, (const cx<R> *)c->tw_x, c->ny, c->nz, bx.nbox, bx.rb, pipe_ctl(c)));
   return GHOST_OK;
 }
 
@@ -46,7 +45,7 @@ template <typename R, int NX, int E, int BZ> static int c2r(ghost_ctx *c, const 
   CUtensorMap m;
   GB_CHECK(field_map(c, in, BZ * G::ES / 8, 1, bx.rb, &m, swizzle_of(G::RB)));
   const int grid = persistent_grid(c, kern, G::NT, smem, (long)(c->nz / BZ) * c->ny);
-  kern<<<grid, G::NT, smem, c->stream>>>(m, (R *)out, (const cx<R> *)c->tw_x, c->ny, c->nz, bx.nbox, bx.rb, pipe_ctl(c));
+  GB_CHECK(launch_dep(c, 1, kern, grid, G::NT, smem, m, (R *)out, (const cx<R> *)c->tw_x, c->ny, c->nz, bx.nbox, bx.rb, pipe_ctl(c)));
   return GHOST_OK;
 }
 
@@ -63,8 +62,7 @@ static int features(ghost_ctx *c, const void *const *spec, float *x, float gs, f
   FieldMaps maps;
   for (int q = 0; q < 9; ++q) GB_CHECK(field_map(c, spec[q], BZ * G::ES / 8, 1, bx.rb, &maps.m[q], swizzle_of(G::RB)));
   const int grid = persistent_grid(c, kern, G::NT, smem, (long)(c->nz / BZ) * c->ny);
-  kern<<<grid, G::NT, smem, c->stream>>>(maps, x, (const cx<R> *)c->tw_x, c->ny, c->nz, bx.nbox, bx.rb,
-                                         (R)(1.0 / (double)c->nreal), gs, delta, pipe_ctl(c));
+  GB_CHECK(launch_dep(c, 3, kern, grid, G::NT, smem, maps, x, (const cx<R> *)c->tw_x, c->ny, c->nz, bx.nbox, bx.rb, (R)(1.0 / (double)c->nreal), gs, delta, pipe_ctl(c)));
   return GHOST_OK;
 }
 

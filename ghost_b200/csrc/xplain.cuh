@@ -79,6 +79,7 @@ __global__ void __launch_bounds__(XnlGeom<R, NX, E, BZ, E>::NT)
   unsigned char *sm = align1024(smem_raw);
   unsigned char *obuf = sm, *ibuf = sm + 2 * G::tile;
   const int tid = threadIdx.x, lane = tid & 31;
+  dep_go();
   const XLine<R, NX, E, BZ> ln(tid, reinterpret_cast<C *>(ibuf + STAGES * P::line_tile), twg);
   const XRing<STAGES, G::NW> ring(ln.tw3 + G::TW3, tid);
   __syncthreads();
@@ -94,6 +95,7 @@ __global__ void __launch_bounds__(XnlGeom<R, NX, E, BZ, E>::NT)
                in + (size_t)NX * ((size_t)(tile / nzb) + (size_t)ny * ((tile % nzb) * BZ + z)), NX * (uint32_t)sizeof(R),
                &ring.full[s]);
   };
+  dep_wait();
   if (tid == 0)
     for (int k = 0; k < STAGES; ++k) issue(k);
   for (int k = 0;; ++k) {
@@ -134,6 +136,7 @@ __global__ void __launch_bounds__(XnlGeom<R, NX, E, BZ, E>::NT)
   extern __shared__ unsigned char smem_raw[];
   unsigned char *sm = align1024(smem_raw);
   const int tid = threadIdx.x, lane = tid & 31;
+  dep_go();
   const XLine<R, NX, E, BZ> ln(tid, reinterpret_cast<C *>(sm + STAGES * G::tile), twg);
   const XRing<STAGES, G::NW> ring(ln.tw3 + G::TW3, tid);
   __syncthreads();
@@ -149,6 +152,7 @@ __global__ void __launch_bounds__(XnlGeom<R, NX, E, BZ, E>::NT)
       tma_load_3d(sm + s * G::tile + (size_t)r0 * RB, &cmap, (tile % nzb) * BZ * U, tile / nzb, r0, &ring.full[s]);
     }
   };
+  dep_wait();
   if (tid == 0)
     for (int k = 0; k < STAGES; ++k) issue(k);
   for (int k = 0;; ++k) {
@@ -179,6 +183,7 @@ __global__ void __launch_bounds__(XnlGeom<R, NX, E, BZ, E>::NT)
   unsigned char *sm = align1024(smem_raw);
   float *st = reinterpret_cast<float *>(sm + STAGES * G::tile);
   const int tid = threadIdx.x, lane = tid & 31;
+  dep_go();
   const XLine<R, NX, E, BZ> ln(tid, reinterpret_cast<C *>(st + BZ * P::ROWF), twg);
   const XRing<STAGES, G::NW> ring(ln.tw3 + G::TW3, tid);
   for (int q = tid; q < BZ * NX; q += G::NT) st[(q / NX) * P::ROWF + (q % NX) * 10 + 9] = delta;  // stays from tile to tile
@@ -195,6 +200,7 @@ __global__ void __launch_bounds__(XnlGeom<R, NX, E, BZ, E>::NT)
       tma_load_3d(sm + s * G::tile + (size_t)r0 * RB, &maps.m[f], (tile % nzb) * BZ * U, tile / nzb, r0, &ring.full[s]);
     }
   };
+  dep_wait();
   if (tid == 0)
     for (int L = 0; L < STAGES; ++L) issue(L);
   float *mine = st + ln.z * P::ROWF + 20 * ln.t;

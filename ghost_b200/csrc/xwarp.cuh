@@ -121,6 +121,7 @@ __global__ void __launch_bounds__(256, 2) xwarp_r2c_kernel(const __grid_constant
   const int tid = threadIdx.x, lane = tid & 31, l = tid >> 5;
   XWRing rg(obuf + 2 * G::out_bytes, M, NX, STAGES, l);
   const int nzb = nz / BZ, ntiles = nzb * ny;
+  dep_go();
   if (tid == 0) {
     mbar_init(rg.never, 1);
     for (int q = 0; q < STAGES; ++q) {
@@ -139,6 +140,7 @@ __global__ void __launch_bounds__(256, 2) xwarp_r2c_kernel(const __grid_constant
     mbar_arrive_expect_tx(&rg.full[s], (uint32_t)G::r2c_in);
     tma_load_3d(sm + (size_t)s * G::r2c_in, &rmap, 0, tile / nzb, (tile % nzb) * BZ, &rg.full[s]);
   };
+  dep_wait();
   if (tid == 0)
     for (int k = 0; k < STAGES; ++k) issue(k);
   float2 *xw = rg.xw;
@@ -197,6 +199,7 @@ __global__ void __launch_bounds__(256, 2) xwarp_c2r_kernel(const __grid_constant
   const int tid = threadIdx.x, lane = tid & 31, l = tid >> 5;
   XWRing rg(sm + STAGES * G::c2r_in, M, NX, STAGES, l);
   const int nzb = nz / BZ, ntiles = nzb * ny;
+  dep_go();
   if (tid == 0) {
     mbar_init(rg.never, 1);
     for (int q = 0; q < STAGES; ++q) {
@@ -217,6 +220,7 @@ __global__ void __launch_bounds__(256, 2) xwarp_c2r_kernel(const __grid_constant
     for (int q = 0; q < nbox; ++q)
       tma_load_3d(dst + (size_t)q * rb * 64, &cmap, (tile % nzb) * BZ, tile / nzb, q * rb, &rg.full[s]);
   };
+  dep_wait();
   if (tid == 0)
     for (int k = 0; k < STAGES; ++k) issue(k);
   float2 *xw = rg.xw;

@@ -22,8 +22,7 @@ static int launch(ghost_ctx *c, const Fields<float> &f, int nf, const Prune &pr)
     GB_CHECK(field_map(c, f.p[q], BZ, rbo, 1, &omaps.m[q], swz));
   }
   const int ts = timer_begin(c, S > 0 ? GHOST_TIMER_Y_INV : GHOST_TIMER_Y_FWD);
-  kern<<<grid, G::NT, G::smem, c->stream>>>(maps, omaps, (const float2 *)c->tw_y, c->nz / BZ, ni, nf, c->nruns, c->nxh,
-                                            pr.jpos, pr.jneg, rb, rbo, pipe_ctl(c));
+  GB_CHECK(launch_dep(c, nf, kern, grid, G::NT, G::smem, maps, omaps, (const float2 *)c->tw_y, c->nz / BZ, ni, nf, c->nruns, c->nxh, pr.jpos, pr.jneg, rb, rbo, pipe_ctl(c)));
   timer_end(c, ts);
   return post_launch(c);
 }

@@ -96,6 +96,7 @@ __global__ void __launch_bounds__(YWarpGeom<N, E, BZ>::NT, N <= 256 ? 2 : 1)
   const int t = T == 32 ? lane : (lane >> 1) & (T - 1);
   const int z = T == 32 ? wp : wp * LW + (T == 16 ? lane & 1 : (lane & 1) + 2 * (lane >> 4));
   const int ntiles = nzb * ni * nruns * nf;
+  dep_go();
   if (tid == 0) {
     mbar_init(never, 1);
     for (int q = 0; q < STAGES; ++q) mbar_init(&full[q], 1);
@@ -141,6 +142,7 @@ __global__ void __launch_bounds__(YWarpGeom<N, E, BZ>::NT, N <= 256 ? 2 : 1)
       tma_load_3d(dst + (size_t)r0 * RB, &maps.m[tl.f], tl.zb * BZ, r0, tl.i, &full[s]);
     }
   };
+  dep_wait();
   if (tid == 0)
     for (int k = 0; k < STAGES - 1; ++k) issue(k);
   // off[c]: byte offset of this lane's column in row (t & 7) ^ c of an 8-row group
