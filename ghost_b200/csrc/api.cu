@@ -2699,7 +2699,7 @@ template <typename R> static int ens_substep_multi(ghost_ensemble *e, int o, dou
       P.cl[q].lines = pr[q].lines;
       P.cl[q].nlines = pr[q].lines ? pr[q].nlines : c->ny * c->nxh * c->nruns;
       P.cl[q].ctl = pipe_ctl(c);
-      const int lpb = kEnsThreads / ens_T<R>(c->nz, zE<R>());
+      const int lpb = kEnsThreads / ens_T<R>(c->nz, c->nz >= 32 ? z_warp_E<R, ZInv<R, 0>>(c->nz) : zE<R>());
       tiles[q] = (P.cl[q].nlines + lpb - 1) / lpb;
     }
     GB_CHECK((ens_launch_z<R, ZInv<R, 0>>(e, P, tiles)));
@@ -2712,11 +2712,17 @@ template <typename R> static int ens_substep_multi(ghost_ensemble *e, int o, dou
     for (int q = 0; q < nc; ++q) {
       ghost_ctx *c = e->cls[q];
       YClass<R> &k = P.cl[q];
-      const int N = c->ny, kb = ens_y_kb_of(N);
-      k.rb = (pr[q].jpos && S > 0) ? std::min(32, N / 2) : std::min(N, 256);
+      const int N = c->ny;
+      const bool wl = y_warp_line<R>(N);
+      const int kb = wl ? 1 : ens_y_kb_of(N), bz = wl ? ens_y_warp_BZ<R>() : kEnsYBZ;
+      const YWarpBoxes bx(N, pr[q].jpos != nullptr, S);
+      k.rb = wl ? bx.rb : ((pr[q].jpos && S > 0) ? std::min(32, N / 2) : std::min(N, 256));
+      k.rbo = bx.rbo;
+      const CUtensorMapSwizzle swz = wl ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE;
       for (int f = 0; f < nf; ++f) {
         k.fld.p[f] = (cx<R> *)w[q][f];
-        GB_CHECK(field_map(c, w[q][f], kEnsYBZ * U, k.rb, 1, &k.maps.m[f]));
+        GB_CHECK(field_map(c, w[q][f], bz * U, k.rb, 1, &k.maps.m[f], swz));
+        if (wl) GB_CHECK(field_map(c, w[q][f], bz * U, k.rbo, 1, &k.omaps.m[f], swz));
       }
       k.tw = (const cx<R> *)c->tw_y;
       k.nz = c->nz;
@@ -2728,7 +2734,7 @@ template <typename R> static int ens_substep_multi(ghost_ensemble *e, int o, dou
       k.jneg = pr[q].jneg;
       k.ctl = pipe_ctl(c);
       P.n[q] = N;
-      tiles[q] = (long)(c->nz / kEnsYBZ) * ((k.ni + kb - 1) / kb) * c->nruns * nf;
+      tiles[q] = (long)(c->nz / bz) * ((k.ni + kb - 1) / kb) * c->nruns * nf;
     }
     return ens_launch_y<R, S>(e, P, tiles);
   };
@@ -2791,7 +2797,7 @@ template <typename R> static int ens_substep_multi(ghost_ensemble *e, int o, dou
       P.cl[q].lines = pr[q].lines;
       P.cl[q].nlines = pr[q].lines ? pr[q].nlines : c->ny * c->nxh * c->nruns;
       P.cl[q].ctl = pipe_ctl(c);
-      const int lpb = kEnsThreads / ens_T<R>(c->nz, zE<R>());
+      const int lpb = kEnsThreads / ens_T<R>(c->nz, c->nz >= 32 ? z_warp_E<R, ZFwdHD<R>>(c->nz) : zE<R>());
       tiles[q] = (P.cl[q].nlines + lpb - 1) / lpb;
     }
     GB_CHECK((ens_launch_z<R, ZFwdHD<R>>(e, P, tiles)));

@@ -18,6 +18,8 @@
 #pragma once
 #include "passes.cuh"
 #include "xnl.cuh"
+#include "ywarp.cuh"
+#include "zwarp.cuh"
 
 namespace gb {
 
@@ -56,13 +58,21 @@ template <typename R, class Op> struct ZMulti {
 };
 template <typename R, int N, int NTH> constexpr int ens_z_lpb() { return NTH / (N / (ens_zE<R>() < N ? ens_zE<R>() : N)); }
 template <typename R, int N, class Op> constexpr size_t ens_z_smem(int stages) {
+  if constexpr (z_warp_line<R, Op>(N)) return ZWarpGeom<R, N, z_warp_E<R, Op>(N), Op::NLOAD>::smem(kEnsThreads / 32);
   constexpr int E = ens_zE<R>() < N ? ens_zE<R>() : N;
   return ZGeom<R, N, E, ens_z_lpb<R, N, kEnsThreads>(), Op::NLOAD>::smem_bytes(stages);
 }
 
 template <typename R, int N, class Op> __device__ __forceinline__ void ens_z_run(const ZClass<R, Op> &k, int vb, int nvb) {
-  constexpr int E = ens_zE<R>() < N ? ens_zE<R>() : N;
-  zpipe_body<R, N, E, ens_z_lpb<R, N, kEnsThreads>(), 2>(vb, nvb, k.op, k.tw, k.lines, k.nlines, k.ctl);
+  if constexpr (z_warp_line<R, Op>(N)) {  // as the class's own launches (zwarp.cuh)
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    constexpr int NWC = kEnsThreads / 32;
+    const int wc = (int)threadIdx.x >> 5;
+    zwarp_body<R, N, z_warp_E<R, Op>(N), NWC>(vb * NWC + wc, nvb * NWC, wc, smem_raw, k.op, k.tw, k.lines, k.nlines, k.ctl);
+  } else {
+    constexpr int E = ens_zE<R>() < N ? ens_zE<R>() : N;
+    zpipe_body<R, N, E, ens_z_lpb<R, N, kEnsThreads>(), 2>(vb, nvb, k.op, k.tw, k.lines, k.nlines, k.ctl);
+  }
 }
 
 template <typename R, class Op>
@@ -78,10 +88,10 @@ __global__ void __launch_bounds__(kEnsThreads) zmulti_kernel(const __grid_consta
 
 // ------------------------------------------------------------------ Y
 template <typename R> struct YClass {
-  FieldMaps maps;
+  FieldMaps maps, omaps;  // omaps: the warp-line body's store boxes
   Fields<R> fld;
   const cx<R> *tw;
-  int nz, ni, nf, nruns, nxh, rb;
+  int nz, ni, nf, nruns, nxh, rb, rbo;
   const int *jpos, *jneg;
   PipeCtl ctl;
 };
@@ -94,15 +104,36 @@ template <int N> constexpr int ens_y_kb() {
   constexpr int E = N < 8 ? N : 8;
   return kEnsThreads / (kEnsYBZ * (N / E));
 }
+// Lines the warp-line body takes: as many groups of its size as make up the CTA.
+template <typename R> constexpr int ens_y_warp_BZ() { return sizeof(R) == 4 ? 16 : 8; }
+constexpr int ens_y_warp_E(int N) { return N == 64 ? 8 : 16; }
+template <typename R, int N> struct EnsYWarp {
+  using G = YWarpGeom<R, N, ens_y_warp_E(N), ens_y_warp_BZ<R>()>;
+  static constexpr int groups = kEnsThreads / G::NT;
+  static constexpr size_t group = (G::smem + 1023) / 1024 * 1024;
+  static_assert(groups * G::NT == kEnsThreads, "one CTA size for all classes");
+};
 template <typename R, int N> constexpr size_t ens_y_smem() {
-  constexpr int E = N < 8 ? N : 8;
-  return YGeom<R, N, E, kEnsYBZ, false, ens_y_kb<N>()>::smem_bytes(3);
+  if constexpr (y_warp_line<R>(N)) return EnsYWarp<R, N>::groups * EnsYWarp<R, N>::group + 1024;
+  else {
+    constexpr int E = N < 8 ? N : 8;
+    return YGeom<R, N, E, kEnsYBZ, false, ens_y_kb<N>()>::smem_bytes(3);
+  }
 }
 
 template <typename R, int N, int S> __device__ __forceinline__ void ens_y_run(const YClass<R> &k, int vb, int nvb) {
-  constexpr int E = N < 8 ? N : 8;
-  ypipe_body<R, N, E, kEnsYBZ, 3, S, false, ens_y_kb<N>()>(vb, nvb, k.maps, k.maps, k.fld, k.tw, k.nz, k.ni, k.nf,
-                                                           k.nruns, k.nxh, k.jpos, k.jneg, k.rb, 0, k.ctl);
+  if constexpr (y_warp_line<R>(N)) {
+    using W = EnsYWarp<R, N>;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    const int g = (int)threadIdx.x / W::G::NT;
+    ywarp_body<R, N, ens_y_warp_E(N), ens_y_warp_BZ<R>(), S>(
+        vb * W::groups + g, nvb * W::groups, g, align1024(smem_raw) + g * W::group, k.maps, k.omaps, k.tw,
+        k.nz / ens_y_warp_BZ<R>(), k.ni, k.nf, k.nruns, k.nxh, k.jpos, k.jneg, k.rb, k.rbo, k.ctl);
+  } else {
+    constexpr int E = N < 8 ? N : 8;
+    ypipe_body<R, N, E, kEnsYBZ, 3, S, false, ens_y_kb<N>()>(vb, nvb, k.maps, k.maps, k.fld, k.tw, k.nz, k.ni, k.nf,
+                                                             k.nruns, k.nxh, k.jpos, k.jneg, k.rb, 0, k.ctl);
+  }
 }
 
 template <typename R, int S>
@@ -154,7 +185,7 @@ template <typename R, int NX> constexpr size_t ens_x_smem() {
 template <typename R, int NX> __device__ __forceinline__ void ens_x_run(const XClass<R> &k, int vb, int nvb) {
   if constexpr (ens_warp_lines(NX)) {
     using W = EnsWarp<R, NX>;
-    extern __shared__ unsigned char smem_raw[];
+    extern __shared__ __align__(128) unsigned char smem_raw[];
     const int g = (int)threadIdx.x / W::NT;
     unsigned char *sm = align1024(smem_raw) + g * W::group;
     vb = vb * W::groups + g;

@@ -114,8 +114,8 @@ int launch_xline_r2c(ghost_ctx *c, const void *in, void *out);
 int launch_xline_c2r(ghost_ctx *c, const void *in, void *out);
 bool xline_features_takes(const ghost_ctx *c, const void *x);
 int launch_xline_features(ghost_ctx *c, const void *const *spec, float *x, float gs, float delta);
-// the Y pass with lines kept inside a warp (FP32, lines of 256 points or more; ywarp.cuh)
-template <int S> int launch_ywarp(ghost_ctx *c, const Fields<float> &f, int nf, const Prune &pr);
+// the Y pass with lines kept inside a warp (ywarp.cuh)
+template <typename R, int S> int launch_ywarp(ghost_ctx *c, const Fields<R> &f, int nf, const Prune &pr);
 // FP64 partial sums owned by the context, grown on demand
 int partials(ghost_ctx *c, size_t n, double **out);
 // per-kernel timers around a launch (kind GHOST_TIMER_*)

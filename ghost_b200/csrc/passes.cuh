@@ -133,7 +133,7 @@ __device__ __forceinline__ void zpipe_body(int vb, int nvb, const Op &op, const 
     const bool act = line >= 0;
     const C *in0 = stage + ((size_t)(s * NL) * LPB + lq) * N;
     auto in = [in0](int f) -> const C * { return in0 + (size_t)f * LPB * N; };
-    op.template body<N, E>(act ? line : 0, act, t, tw, buf, sync, in);
+    op.template body<N, E>(act ? line : 0, act, t, tw, buf, sync, in, [] {});
     // the stage is refilled at the top of the next tile: the transforms'
     // exchange barriers follow every read of it, except without exchanges
     if constexpr (fft_exchanges<N, E>() == 0) __syncthreads();
@@ -147,6 +147,17 @@ __global__ void __launch_bounds__(LPB *(N / E), MINB) zpipe_kernel(Op op, const 
   zpipe_body<R, N, E, LPB, STAGES>(blockIdx.x, gridDim.x, op, twg, lines, nlines, ctl);
 }
 
+// An operation's line transform: by the CTA's threads, or (zwarp.cuh) by the
+// lanes of a warp, whose buffer knows how.
+template <class B> struct is_warp_line { static constexpr bool value = false; };
+template <typename C, int N, int E, int S, class Buf, class Sync>
+__device__ __forceinline__ void z_fft(C (&x)[E], int t, const C *__restrict__ tw, Buf buf, Sync sync) {
+  if constexpr (is_warp_line<Buf>::value) buf.template fft<N, E, S>(x, t);
+  else line_fft<C, N, E, S>(x, t, tw, buf, sync);
+}
+
+// An operation's body transforms one line: src(f) is its loaded field f, and
+// done() says that the body has read the last of them.
 // Plain c2c along z of NF fields (in -> out, may alias).
 template <typename R, int S, int NF> struct ZC2C {
   using C = cx<R>;
@@ -154,15 +165,17 @@ template <typename R, int S, int NF> struct ZC2C {
   CFields<R> in;
   Fields<R> out;
   __device__ __forceinline__ const C *load_src(int f) const { return in.p[f]; }
-  template <int N, int E, class Buf, class Sync, class In>
-  __device__ __forceinline__ void body(long line, bool act, int t, const C *tw, Buf buf, Sync sync, In src) const {
+  template <int N, int E, class Buf, class Sync, class In, class Done>
+  __device__ __forceinline__ void body(long line, bool act, int t, const C *tw, Buf buf, Sync sync, In src,
+                                       Done done) const {
     constexpr int T = N / E;
 #pragma unroll
     for (int f = 0; f < NF; ++f) {
       C x[E];
 #pragma unroll
       for (int e = 0; e < E; ++e) x[e] = src(f)[t + T * e];
-      line_fft<C, N, E, S>(x, t, tw, buf, sync);
+      if (f == NF - 1) done();
+      z_fft<C, N, E, S>(x, t, tw, buf, sync);
       if (act) {
         C *dst = out.p[f] + (size_t)line * N;
 #pragma unroll
@@ -190,8 +203,9 @@ template <typename R, int PHYS> struct ZInv {
   KParams<R> kp;
   int copy;
   __device__ __forceinline__ const C *load_src(int f) const { return v.p[f]; }
-  template <int N, int E, class Buf, class Sync, class In>
-  __device__ __forceinline__ void body(long line, bool act, int t, const C *tw, Buf buf, Sync sync, In src) const {
+  template <int N, int E, class Buf, class Sync, class In, class Done>
+  __device__ __forceinline__ void body(long line, bool act, int t, const C *tw, Buf buf, Sync sync, In src,
+                                       Done done) const {
     constexpr int T = N / E;
     const int j = (int)(line % kp.ny), ir = (int)(line / kp.ny), i = ir % kp.nxh + kp.i0;
     const R kx = kx_of(kp, i), ky = ky_of(kp, j);
@@ -228,7 +242,8 @@ template <typename R, int PHYS> struct ZInv {
           x[e] = mk(-(kd * th.y), kd * th.x);
         }
       }
-      line_fft<C, N, E, +1>(x, t, tw, buf, sync);
+      if (f == NOUT - 1) done();
+      z_fft<C, N, E, +1>(x, t, tw, buf, sync);
       if (act) {
         C *dst = w.p[f] + (size_t)line * N;
 #pragma unroll
@@ -249,8 +264,9 @@ template <typename R> struct ZNorm {
   KParams<R> kp;
   int kin;
   __device__ __forceinline__ const C *load_src(int f) const { return v.p[f]; }
-  template <int N, int E, class Buf, class Sync, class In>
-  __device__ __forceinline__ void body(long line, bool act, int t, const C *tw, Buf buf, Sync sync, In src) const {
+  template <int N, int E, class Buf, class Sync, class In, class Done>
+  __device__ __forceinline__ void body(long line, bool act, int t, const C *tw, Buf buf, Sync sync, In src,
+                                       Done done) const {
     constexpr int T = N / E;
     const int j = (int)(line % kp.ny), i = (int)(line / kp.ny) % kp.nxh + kp.i0;
     const R kx = kx_of(kp, i), ky = ky_of(kp, j);
@@ -272,7 +288,8 @@ template <typename R> struct ZNorm {
           }
         }
       }
-      line_fft<C, N, E, +1>(x, t, tw, buf, sync);
+      if (f == 2) done();
+      z_fft<C, N, E, +1>(x, t, tw, buf, sync);
       if (act) {
         C *dst = w.p[f] + (size_t)line * N;
 #pragma unroll
@@ -301,8 +318,9 @@ template <typename R> struct ZInvMhd {
     if (d == 1) return mk((-kz * x.y) - (-kx * z.y), (kz * x.x) - (kx * z.x));
     return mk((-kx * y.y) - (-ky * x.y), (kx * y.x) - (ky * x.x));
   }
-  template <int N, int E, class Buf, class Sync, class In>
-  __device__ __forceinline__ void body(long line, bool act, int t, const C *tw, Buf buf, Sync sync, In src) const {
+  template <int N, int E, class Buf, class Sync, class In, class Done>
+  __device__ __forceinline__ void body(long line, bool act, int t, const C *tw, Buf buf, Sync sync, In src,
+                                       Done done) const {
     constexpr int T = N / E;
     const int j = (int)(line % kp.ny), i = (int)(line / kp.ny) % kp.nxh + kp.i0;
     const R kx = kx_of(kp, i), ky = ky_of(kp, j);
@@ -336,7 +354,8 @@ template <typename R> struct ZInvMhd {
           }
         }
       }
-      line_fft<C, N, E, +1>(x, t, tw, buf, sync);
+      if (f == 11) done();
+      z_fft<C, N, E, +1>(x, t, tw, buf, sync);
       if (act) {
         C *dst = w.p[f] + (size_t)line * N;
 #pragma unroll
@@ -356,8 +375,9 @@ template <typename R> struct ZGrad {
   Fields<R> w;   // 9 outputs
   KParams<R> kp;
   __device__ __forceinline__ const C *load_src(int f) const { return v.p[f]; }
-  template <int N, int E, class Buf, class Sync, class In>
-  __device__ __forceinline__ void body(long line, bool act, int t, const C *tw, Buf buf, Sync sync, In src) const {
+  template <int N, int E, class Buf, class Sync, class In, class Done>
+  __device__ __forceinline__ void body(long line, bool act, int t, const C *tw, Buf buf, Sync sync, In src,
+                                       Done done) const {
     constexpr int T = N / E;
     const int j = (int)(line % kp.ny), i = (int)(line / kp.ny) % kp.nxh + kp.i0;
     const R kx = kx_of(kp, i), ky = ky_of(kp, j);
@@ -372,7 +392,8 @@ template <typename R> struct ZGrad {
         const C u = src(a)[k];
         x[e] = mk(-(kd * u.y), kd * u.x);
       }
-      line_fft<C, N, E, +1>(x, t, tw, buf, sync);
+      if (f == 8) done();
+      z_fft<C, N, E, +1>(x, t, tw, buf, sync);
       if (act) {
         C *dst = w.p[f] + (size_t)line * N;
 #pragma unroll
@@ -387,9 +408,9 @@ template <typename R> struct ZGrad {
 // GAUGE: its negative, gauge3 of pseudospec3D_mhd.f90:230-336), then
 // v = C + dt (nu laplak3(v) + x + f)/o on the kept modes, 0 elsewhere
 // (include/hd_rkstep2.f90:18-38).
-template <typename R, int N, int E, bool GAUGE, int OFF, class Buf, class Sync, class In>
+template <typename R, int N, int E, bool GAUGE, int OFF, class Buf, class Sync, class In, class Done>
 __device__ __forceinline__ void fwd_update(const KParams<R> &kp, long line, bool act, int i, int j, R kx, R ky, int t,
-                                           const cx<R> *tw, Buf buf, Sync sync, In src, const Fields<R> &v,
+                                           const cx<R> *tw, Buf buf, Sync sync, In src, Done done, const Fields<R> &v,
                                            const CFields<R> &c0, const CFields<R> &f, R dt, R nuv, R rmp) {
   using C = cx<R>;
   constexpr int T = N / E;
@@ -421,7 +442,8 @@ __device__ __forceinline__ void fwd_update(const KParams<R> &kp, long line, bool
   for (int c = 0; c < 3; ++c) {
 #pragma unroll
     for (int e = 0; e < E; ++e) g[c][e] = src(OFF + c)[t + T * e];
-    line_fft<C, N, E, -1>(g[c], t, tw, buf, sync);
+    if (c == 2) done();
+    z_fft<C, N, E, -1>(g[c], t, tw, buf, sync);
   }
   if (!act) return;
   // The projected nonlinear term replaces g in place; then, component by
@@ -448,32 +470,38 @@ __device__ __forceinline__ void fwd_update(const KParams<R> &kp, long line, bool
     }
   }
   const size_t base = (size_t)line * N + t;
+  // (in chunks of 8 elements, 4 in FP64, which the registers hold)
+  constexpr int EC = E < 32 / (int)sizeof(R) ? E : 32 / (int)sizeof(R);
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    C vv[E], ff[E], cc0[E];
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
-      vv[e] = mk((R)0, (R)0);
-      ff[e] = mk((R)0, (R)0);
-      cc0[e] = mk((R)0, (R)0);
-      if (keep[e]) {
-        const size_t p = base + (size_t)T * e;
-        vv[e] = v.p[OFF + c][p];
-        cc0[e] = c0.p[OFF + c][p];
-        if (forced) ff[e] = f.p[OFF + c][p];
+    for (int e0 = 0; e0 < E; e0 += EC) {
+      C vv[EC], ff[EC], cc0[EC];
+#pragma unroll
+      for (int q = 0; q < EC; ++q) {
+        vv[q] = mk((R)0, (R)0);
+        ff[q] = mk((R)0, (R)0);
+        cc0[q] = mk((R)0, (R)0);
+        if (keep[e0 + q]) {
+          const size_t p = base + (size_t)T * (e0 + q);
+          vv[q] = v.p[OFF + c][p];
+          cc0[q] = c0.p[OFF + c][p];
+          if (forced) ff[q] = f.p[OFF + c][p];
+        }
       }
-    }
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const size_t p = base + (size_t)T * e;
-      if (keep[e]) {
-        const R kk2 = kk2e[e];
-        const C lap = mk(-kk2 * vv[e].x, -kk2 * vv[e].y);
-        C sum = mk(nuv * lap.x + g[c][e].x, nuv * lap.y + g[c][e].y);
-        if (forced) sum = mk(sum.x + ff[e].x, sum.y + ff[e].y);
-        v.p[OFF + c][p] = mk(cc0[e].x + (dt * sum.x) * rmp, cc0[e].y + (dt * sum.y) * rmp);
-      } else {
-        v.p[OFF + c][p] = mk((R)0, (R)0);
+      for (int q = 0; q < EC; ++q) {
+        const int e = e0 + q;
+        const size_t p = base + (size_t)T * e;
+        if (keep[e]) {
+          const R kk2 = kk2e[e];
+          const C lap = mk(-kk2 * vv[q].x, -kk2 * vv[q].y);
+          C sum = mk(nuv * lap.x + g[c][e].x, nuv * lap.y + g[c][e].y);
+          if (forced) sum = mk(sum.x + ff[q].x, sum.y + ff[q].y);
+          v.p[OFF + c][p] = mk(cc0[q].x + (dt * sum.x) * rmp, cc0[q].y + (dt * sum.y) * rmp);
+        } else {
+          v.p[OFF + c][p] = mk((R)0, (R)0);
+        }
       }
     }
   }
@@ -490,12 +518,13 @@ template <typename R> struct ZFwdHD {
   KParams<R> kp;
   R dt, nu, rmp;
   __device__ __forceinline__ const C *load_src(int q) const { return nl.p[q]; }
-  template <int N, int E, class Buf, class Sync, class In>
-  __device__ __forceinline__ void body(long line, bool act, int t, const C *tw, Buf buf, Sync sync, In src) const {
+  template <int N, int E, class Buf, class Sync, class In, class Done>
+  __device__ __forceinline__ void body(long line, bool act, int t, const C *tw, Buf buf, Sync sync, In src,
+                                       Done done) const {
     const int j = (int)(line % kp.ny), ir = (int)(line / kp.ny), i = ir % kp.nxh + kp.i0;
     const R kx = kx_of(kp, i), ky = ky_of(kp, j);
     const R nuv = kp.nu_run ? kp.nu_run[ir / kp.nxh] : nu;
-    fwd_update<R, N, E, false, 0>(kp, line, act, i, j, kx, ky, t, tw, buf, sync, src, v, c0, f, dt, nuv, rmp);
+    fwd_update<R, N, E, false, 0>(kp, line, act, i, j, kx, ky, t, tw, buf, sync, src, done, v, c0, f, dt, nuv, rmp);
   }
 };
 
@@ -512,12 +541,13 @@ template <typename R> struct ZFwdMhd {
   KParams<R> kp;
   R dt, nu, mu, rmp;
   __device__ __forceinline__ const C *load_src(int q) const { return nl.p[q]; }
-  template <int N, int E, class Buf, class Sync, class In>
-  __device__ __forceinline__ void body(long line, bool act, int t, const C *tw, Buf buf, Sync sync, In src) const {
+  template <int N, int E, class Buf, class Sync, class In, class Done>
+  __device__ __forceinline__ void body(long line, bool act, int t, const C *tw, Buf buf, Sync sync, In src,
+                                       Done done) const {
     const int j = (int)(line % kp.ny), i = (int)(line / kp.ny) % kp.nxh + kp.i0;
     const R kx = kx_of(kp, i), ky = ky_of(kp, j);
-    fwd_update<R, N, E, false, 0>(kp, line, act, i, j, kx, ky, t, tw, buf, sync, src, va, c0, f, dt, nu, rmp);
-    fwd_update<R, N, E, true, 3>(kp, line, act, i, j, kx, ky, t, tw, buf, sync, src, va, c0, f, dt, mu, rmp);
+    fwd_update<R, N, E, false, 0>(kp, line, act, i, j, kx, ky, t, tw, buf, sync, src, [] {}, va, c0, f, dt, nu, rmp);
+    fwd_update<R, N, E, true, 3>(kp, line, act, i, j, kx, ky, t, tw, buf, sync, src, done, va, c0, f, dt, mu, rmp);
   }
 };
 
@@ -535,8 +565,9 @@ template <typename R> struct ZFwdBouss {
   KParams<R> kp;
   R dt, nu, kappa, omegaz, xmom, xtemp, rmp;
   __device__ __forceinline__ const C *load_src(int q) const { return nl.p[q]; }
-  template <int N, int E, class Buf, class Sync, class In>
-  __device__ __forceinline__ void body(long line, bool act, int t, const C *tw, Buf buf, Sync sync, In src) const {
+  template <int N, int E, class Buf, class Sync, class In, class Done>
+  __device__ __forceinline__ void body(long line, bool act, int t, const C *tw, Buf buf, Sync sync, In src,
+                                       Done done) const {
     constexpr int T = N / E;
     const int j = (int)(line % kp.ny), i = (int)(line / kp.ny) % kp.nxh + kp.i0;
     const R kx = kx_of(kp, i), ky = ky_of(kp, j);
@@ -565,70 +596,81 @@ template <typename R> struct ZFwdBouss {
     for (int c = 0; c < 4; ++c) {
 #pragma unroll
       for (int e = 0; e < E; ++e) g[c][e] = src(c)[t + T * e];
-      line_fft<C, N, E, -1>(g[c], t, tw, buf, sync);
+      if (c == 3) done();
+      z_fft<C, N, E, -1>(g[c], t, tw, buf, sync);
     }
     if (!act) return;
     const R two_om = (R)2 * omegaz;
-    // As in ZFwdHD: all loads of a round before any store.  The velocity
+    // As in fwd_update: all loads of a round before any store.  The velocity
     // and theta values enter the projection and the Laplacians, which are
     // folded into g there, so they are dead before the update loads C and f.
-    C vv[4][E];
+    constexpr int EC = E < 32 / (int)sizeof(R) ? E : 32 / (int)sizeof(R);
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
+    for (int e0 = 0; e0 < E; e0 += EC) {
+      C vv[4][EC];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) vv[c][e] = mk((R)0, (R)0);
-      if (mode[e] == 0) {
-        const size_t p = base + (size_t)T * e;
+      for (int q = 0; q < EC; ++q) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) vv[c][e] = v.p[c][p];
+        for (int c = 0; c < 4; ++c) vv[c][q] = mk((R)0, (R)0);
+        if (mode[e0 + q] == 0) {
+          const size_t p = base + (size_t)T * (e0 + q);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) vv[c][q] = v.p[c][p];
+        }
       }
-    }
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
-      if (mode[e] != 0) continue;
-      const int k = t + T * e;
-      const R kz = kz_of(kp, k);
-      const R kk2 = kk2_of(kp, i, j, k);
-      const C a = mk(g[0][e].x - two_om * vv[1][e].x, g[0][e].y - two_om * vv[1][e].y);
-      const C b = mk(g[1][e].x + two_om * vv[0][e].x, g[1][e].y + two_om * vv[0][e].y);
-      const C cc = mk(g[2][e].x + xmom * vv[3][e].x, g[2][e].y + xmom * vv[3][e].y);
-      const C s = mk(kx * a.x + ky * b.x + kz * cc.x, kx * a.y + ky * b.y + kz * cc.y);
-      g[0][e] = (i == 0) ? mk(-a.x, -a.y) : mk(-a.x + (kx * s.x) / kk2, -a.y + (kx * s.y) / kk2);
-      g[1][e] = (j == 0) ? mk(-b.x, -b.y) : mk(-b.x + (ky * s.x) / kk2, -b.y + (ky * s.y) / kk2);
-      g[2][e] = (k == 0) ? mk(-cc.x, -cc.y) : mk(-cc.x + (kz * s.x) / kk2, -cc.y + (kz * s.y) / kk2);
-      g[3][e] = mk(g[3][e].x + xtemp * vv[2][e].x, g[3][e].y + xtemp * vv[2][e].y);
+      for (int q = 0; q < EC; ++q) {
+        const int e = e0 + q;
+        if (mode[e] != 0) continue;
+        const int k = t + T * e;
+        const R kz = kz_of(kp, k);
+        const R kk2 = kk2_of(kp, i, j, k);
+        const C a = mk(g[0][e].x - two_om * vv[1][q].x, g[0][e].y - two_om * vv[1][q].y);
+        const C b = mk(g[1][e].x + two_om * vv[0][q].x, g[1][e].y + two_om * vv[0][q].y);
+        const C cc = mk(g[2][e].x + xmom * vv[3][q].x, g[2][e].y + xmom * vv[3][q].y);
+        const C s = mk(kx * a.x + ky * b.x + kz * cc.x, kx * a.y + ky * b.y + kz * cc.y);
+        g[0][e] = (i == 0) ? mk(-a.x, -a.y) : mk(-a.x + (kx * s.x) / kk2, -a.y + (kx * s.y) / kk2);
+        g[1][e] = (j == 0) ? mk(-b.x, -b.y) : mk(-b.x + (ky * s.x) / kk2, -b.y + (ky * s.y) / kk2);
+        g[2][e] = (k == 0) ? mk(-cc.x, -cc.y) : mk(-cc.x + (kz * s.x) / kk2, -cc.y + (kz * s.y) / kk2);
+        g[3][e] = mk(g[3][e].x + xtemp * vv[2][q].x, g[3][e].y + xtemp * vv[2][q].y);
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {  // + dif * Laplacian
-        const R dif = c < 3 ? nu : kappa;
-        const C lap = mk(-kk2 * vv[c][e].x, -kk2 * vv[c][e].y);
-        g[c][e] = mk(dif * lap.x + g[c][e].x, dif * lap.y + g[c][e].y);
+        for (int c = 0; c < 4; ++c) {  // + dif * Laplacian
+          const R dif = c < 3 ? nu : kappa;
+          const C lap = mk(-kk2 * vv[c][q].x, -kk2 * vv[c][q].y);
+          g[c][e] = mk(dif * lap.x + g[c][e].x, dif * lap.y + g[c][e].y);
+        }
       }
     }
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
       const bool fc = c < 3 ? forced : sforced;
-      C ff[E], cc0[E];
 #pragma unroll
-      for (int e = 0; e < E; ++e) {
-        ff[e] = mk((R)0, (R)0);
-        cc0[e] = mk((R)0, (R)0);
-        const size_t p = base + (size_t)T * e;
-        if (mode[e] == 0) {
-          cc0[e] = c0.p[c][p];
-          if (fc) ff[e] = f.p[c][p];
-        } else if (mode[e] == 2 && c == 3) {
-          cc0[e] = c0.p[3][p];
+      for (int e0 = 0; e0 < E; e0 += EC) {
+        C ff[EC], cc0[EC];
+#pragma unroll
+        for (int q = 0; q < EC; ++q) {
+          ff[q] = mk((R)0, (R)0);
+          cc0[q] = mk((R)0, (R)0);
+          const int e = e0 + q;
+          const size_t p = base + (size_t)T * e;
+          if (mode[e] == 0) {
+            cc0[q] = c0.p[c][p];
+            if (fc) ff[q] = f.p[c][p];
+          } else if (mode[e] == 2 && c == 3) {
+            cc0[q] = c0.p[3][p];
+          }
         }
-      }
 #pragma unroll
-      for (int e = 0; e < E; ++e) {
-        const size_t p = base + (size_t)T * e;
-        if (mode[e] == 0) {
-          C sum = g[c][e];
-          if (fc) sum = mk(sum.x + ff[e].x, sum.y + ff[e].y);
-          v.p[c][p] = mk(cc0[e].x + (dt * sum.x) * rmp, cc0[e].y + (dt * sum.y) * rmp);
-        } else {
-          v.p[c][p] = (mode[e] == 2 && c == 3) ? cc0[e] : mk((R)0, (R)0);
+        for (int q = 0; q < EC; ++q) {
+          const int e = e0 + q;
+          const size_t p = base + (size_t)T * e;
+          if (mode[e] == 0) {
+            C sum = g[c][e];
+            if (fc) sum = mk(sum.x + ff[q].x, sum.y + ff[q].y);
+            v.p[c][p] = mk(cc0[q].x + (dt * sum.x) * rmp, cc0[q].y + (dt * sum.y) * rmp);
+          } else {
+            v.p[c][p] = (mode[e] == 2 && c == 3) ? cc0[q] : mk((R)0, (R)0);
+          }
         }
       }
     }

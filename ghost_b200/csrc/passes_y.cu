@@ -3,6 +3,7 @@
 #include <algorithm>
 
 #include "internal.cuh"
+#include "ywarp.cuh"
 
 namespace gb {
 
@@ -54,9 +55,9 @@ int launch_y_cfg(ghost_ctx *c, const Fields<R> &f, int nf, const Prune &pr) {
 
 // tiles 8 z-lines wide, or 16 with tile variant bit 0
 template <typename R, int N, int S> int launch_y_n(ghost_ctx *c, const Fields<R> &f, int nf, const Prune &pr) {
-  // FP32 lines of 256 points or more: the warp-line kernel, whatever the tile
-  // variant (its y bits choose between kernels of other line lengths)
-  if constexpr (sizeof(R) == 4 && N >= 256) return launch_ywarp<S>(c, f, nf, pr);
+  // lines the warp-line kernel takes, whatever the tile variant (its y bits
+  // choose between the kernels of other line lengths)
+  if constexpr (y_warp_line<R>(N)) return launch_ywarp<R, S>(c, f, nf, pr);
   else {
   // the 16-wide tile needs two stages of 16 lines in shared memory; where
   // that does not fit (FP64, long lines) the variant falls back to 8

@@ -4,6 +4,7 @@
 #include <algorithm>
 
 #include "internal.cuh"
+#include "zwarp.cuh"
 
 namespace gb {
 
@@ -49,29 +50,52 @@ template <class Op> struct OneStage { static constexpr bool value = true; };
 template <typename R, int S, int NF> struct OneStage<ZC2C<R, S, NF>> { static constexpr bool value = false; };
 template <int P> struct OneStage<ZInv<double, P>> { static constexpr bool value = false; };
 
+// CTAs of NWC warps (zwarp.cuh)
+template <typename R, int N, int E, int NWC, int MINB, class Op>
+int launch_zwarp_cfg(ghost_ctx *c, const Op &op, const Prune &pr) {
+  using G = ZWarpGeom<R, N, E, Op::NLOAD>;
+  const size_t smem = G::smem(NWC);
+  static_assert(G::smem(NWC) <= 227 * 1024, "shared memory");
+  const int nlines = pr.lines ? pr.nlines : c->ny * c->nxh * c->nruns;
+  auto kern = zwarp_kernel<R, N, E, NWC, MINB, Op>;
+  GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int grid = persistent_grid(c, kern, 32 * NWC, smem, (nlines + G::LW * NWC - 1) / (G::LW * NWC));
+  const int ts = timer_begin(c, ZKind<Op>::value);
+  GB_CHECK(launch_dep(c, Op::NLOAD, kern, grid, 32 * NWC, smem, op, (const cx<R> *)c->tw_z, pr.lines, nlines, pipe_ctl(c)));
+  timer_end(c, ts);
+  return post_launch(c);
+}
+template <typename R, int N, class Op> int launch_zwarp(ghost_ctx *c, const Op &op, const Prune &pr) {
+  constexpr int E = z_warp_E<R, Op>(N);
+  // the forward updates hold three or four components: 255 registers in FP64
+  constexpr int MINB = ZUpdate<Op>::value && sizeof(R) == 8 ? 2 : 3;
+  const int nlines = pr.lines ? pr.nlines : c->ny * c->nxh * c->nruns;
+  // few lines: one warp per CTA, so that every SM has work (a 64^3 FP64 step
+  // has 740 live lines)
+  if (nlines < 8 * ZWarpGeom<R, N, E, Op::NLOAD>::LW * sm_count(c))
+    return launch_zwarp_cfg<R, N, E, 1, 4 * MINB>(c, op, pr);
+  return launch_zwarp_cfg<R, N, E, 4, MINB>(c, op, pr);
+}
+
 // CTAs of 256 threads; with tile variant bit 1 of 128 threads; with bits 1
 // and 2, for lines of 256 points or more, of 128 threads with a two-stage ring
 // and at most 170 registers, so that three CTAs share an SM; with bit 5 too
-// with a one-stage ring and four CTAs.  Passes of few lines take smaller CTAs,
-// so that every SM has work: 64 threads below two tiles of 128 per SM (a 64^3
-// FP64 step: 740 live lines were 47 CTAs of 256 threads).
+// with a one-stage ring and four CTAs.
 template <typename R, int N, class Op> int launch_z_n(ghost_ctx *c, const Op &op, const Prune &pr) {
-  constexpr int E = zE<R>() < N ? zE<R>() : N, T = N / E;
-  constexpr int L256 = fit_lines<R, N, Op::NLOAD>(256 / T > 0 ? 256 / T : 1);
-  constexpr int L128 = fit_lines<R, N, Op::NLOAD>(128 / T > 0 ? 128 / T : 1);
-  constexpr int L64 = fit_lines<R, N, Op::NLOAD>(64 / T > 0 ? 64 / T : 1);
-  if constexpr (N >= 256 && L128 != L256) {
-    if constexpr (OneStage<Op>::value)
-      if ((c->tile_cfg & 38) == 38) return launch_z_cfg<R, N, L128, 1, 4>(c, op, pr);
-    if ((c->tile_cfg & 6) == 6) return launch_z_cfg<R, N, L128, 2, 3>(c, op, pr);
+  if constexpr (z_warp_line<R, Op>(N)) {
+    return launch_zwarp<R, N>(c, op, pr);
+  } else {
+    constexpr int E = zE<R>() < N ? zE<R>() : N, T = N / E;
+    constexpr int L256 = fit_lines<R, N, Op::NLOAD>(256 / T > 0 ? 256 / T : 1);
+    constexpr int L128 = fit_lines<R, N, Op::NLOAD>(128 / T > 0 ? 128 / T : 1);
+    if constexpr (N >= 256 && L128 != L256) {
+      if constexpr (OneStage<Op>::value)
+        if ((c->tile_cfg & 38) == 38) return launch_z_cfg<R, N, L128, 1, 4>(c, op, pr);
+      if ((c->tile_cfg & 6) == 6) return launch_z_cfg<R, N, L128, 2, 3>(c, op, pr);
+    }
+    if ((c->tile_cfg & 2) && L128 != L256) return launch_z_cfg<R, N, L128, 3, 1>(c, op, pr);
+    return launch_z_cfg<R, N, L256, 3, 1>(c, op, pr);
   }
-  if constexpr (N < 256 && L64 != L128) {
-    const int nlines = pr.lines ? pr.nlines : c->ny * c->nxh * c->nruns;
-    if (nlines < 2 * L128 * sm_count(c)) return launch_z_cfg<R, N, L64, 3, 1>(c, op, pr);
-    if (nlines < 2 * L256 * sm_count(c)) return launch_z_cfg<R, N, L128, 3, 1>(c, op, pr);
-  }
-  if ((c->tile_cfg & 2) && L128 != L256) return launch_z_cfg<R, N, L128, 3, 1>(c, op, pr);
-  return launch_z_cfg<R, N, L256, 3, 1>(c, op, pr);
 }
 
 template <typename R, class Op> int launch_z(ghost_ctx *c, const Op &op, const Prune &pr) {

@@ -30,8 +30,8 @@ namespace gb {
 
 // ------------------------------------------------------------ transforms
 // In-register DFTs on packed complex numbers, y_r = sum_m x_m exp(S 2 pi i m r / R).
-template <int S> __device__ __forceinline__ void pdft4(float2 &x0, float2 &x1, float2 &x2, float2 &x3) {
-  const float2 a0 = add2(x0, x2), a1 = sub2(x0, x2), b0 = add2(x1, x3), d = sub2(x1, x3);
+template <int S, typename C> __device__ __forceinline__ void pdft4(C &x0, C &x1, C &x2, C &x3) {
+  const C a0 = add2(x0, x2), a1 = sub2(x0, x2), b0 = add2(x1, x3), d = sub2(x1, x3);
   x0 = add2(a0, b0);
   x2 = sub2(a0, b0);
   if (S > 0) {
@@ -43,31 +43,32 @@ template <int S> __device__ __forceinline__ void pdft4(float2 &x0, float2 &x1, f
   }
 }
 // a * (c + S i s), constants
-template <int S> __device__ __forceinline__ float2 cmulk(float2 a, float c, float s) {
-  const float t = S > 0 ? s : -s;
+template <int S, typename C> __device__ __forceinline__ C cmulk(C a, double c0, double s0) {
+  typedef decltype(C{}.x) R;
+  const R c = (R)c0, t = (R)(S > 0 ? s0 : -s0);
   return mk(a.x * c - a.y * t, a.y * c + a.x * t);
 }
 // a * exp(S 2 pi i / 8) and a * exp(S 2 pi i 3/8)
-template <int S> __device__ __forceinline__ float2 mulw8(float2 a) {
-  constexpr float h = 0.70710678118654752440f;
+template <int S, typename C> __device__ __forceinline__ C mulw8(C a) {
+  const auto h = rsqrt2_of<C>::v();
   return S > 0 ? mul2(mk(a.x - a.y, a.y + a.x), both(h)) : mul2(mk(a.x + a.y, a.y - a.x), both(h));
 }
-template <int S> __device__ __forceinline__ float2 mulw83(float2 a) {
-  constexpr float h = 0.70710678118654752440f;
+template <int S, typename C> __device__ __forceinline__ C mulw83(C a) {
+  const auto h = rsqrt2_of<C>::v();
   return S > 0 ? mul2(mk(-a.x - a.y, a.x - a.y), both(h)) : mul2(mk(a.y - a.x, -a.x - a.y), both(h));
 }
-template <int S> __device__ __forceinline__ void pdft8(float2 (&v)[8]) {
-  float2 u0 = add2(v[0], v[4]), d0 = sub2(v[0], v[4]), u1 = add2(v[1], v[5]), d1 = sub2(v[1], v[5]);
-  float2 u2 = add2(v[2], v[6]), d2 = sub2(v[2], v[6]), u3 = add2(v[3], v[7]), d3 = sub2(v[3], v[7]);
-  float2 e1 = mulw8<S>(d1), e2 = mul_si<S>(d2), e3 = mulw83<S>(d3);
+template <int S, typename C> __device__ __forceinline__ void pdft8(C (&v)[8]) {
+  C u0 = add2(v[0], v[4]), d0 = sub2(v[0], v[4]), u1 = add2(v[1], v[5]), d1 = sub2(v[1], v[5]);
+  C u2 = add2(v[2], v[6]), d2 = sub2(v[2], v[6]), u3 = add2(v[3], v[7]), d3 = sub2(v[3], v[7]);
+  C e1 = mulw8<S>(d1), e2 = mul_si<S>(d2), e3 = mulw83<S>(d3);
   pdft4<S>(u0, u1, u2, u3);
   pdft4<S>(d0, e1, e2, e3);
   v[0] = u0; v[2] = u1; v[4] = u2; v[6] = u3;
   v[1] = d0; v[3] = e1; v[5] = e2; v[7] = e3;
 }
-template <int S> __device__ __forceinline__ void pdft16(float2 (&x)[16]) {
+template <int S, typename C> __device__ __forceinline__ void pdft16(C (&x)[16]) {
   // cos and sin of 2 pi/16
-  constexpr float c1 = 0.92387953251128675613f, s1 = 0.38268343236508977173f;
+  constexpr double c1 = 0.92387953251128675613, s1 = 0.38268343236508977173;
 #pragma unroll
   for (int m = 0; m < 4; ++m) pdft4<S>(x[m], x[m + 4], x[m + 8], x[m + 12]);
   // x[m + 4 r] is output r of column m: times W16^(m r)
@@ -83,7 +84,7 @@ template <int S> __device__ __forceinline__ void pdft16(float2 (&x)[16]) {
 #pragma unroll
   for (int r = 0; r < 4; ++r) pdft4<S>(x[4 * r], x[4 * r + 1], x[4 * r + 2], x[4 * r + 3]);
   // x[4 r + q] is now output r + 4 q
-  float2 y[16];
+  C y[16];
 #pragma unroll
   for (int r = 0; r < 4; ++r)
 #pragma unroll
