@@ -182,6 +182,14 @@ template <typename C, class Slot> __device__ __forceinline__ DualBuf<C, Slot> du
   return DualBuf<C, Slot>{s, ph};
 }
 
+// An exchange buffer whose slots depend on the span L of the stage that writes
+// them has at<L>(idx) instead of operator().
+template <class B> struct is_span_buf { static constexpr bool value = false; };
+template <int L, class Buf> __device__ __forceinline__ auto &slot_of(const Buf &buf, int idx) {
+  if constexpr (is_span_buf<Buf>::value) return buf.template at<L>(idx);
+  else return buf(idx);
+}
+
 // Full N-point transform of the line held in x (pattern t + T*e).
 //   buf(idx) -> C& : this thread's line slot in shared memory
 //   sync()         : barrier over every thread taking part (all lines of
@@ -195,10 +203,10 @@ __device__ __forceinline__ void line_fft(C (&x)[E], int t, const C *__restrict__
   if constexpr (LAST) {
     fft_stage<C, N, E, L, S, TWS>(x, t, tw, [](int, C) {});
   } else {
-    fft_stage<C, N, E, L, S, TWS>(x, t, tw, [&](int idx, C v) { buf(idx) = v; });
+    fft_stage<C, N, E, L, S, TWS>(x, t, tw, [&](int idx, C v) { slot_of<L>(buf, idx) = v; });
     sync();
 #pragma unroll
-    for (int e = 0; e < E; ++e) x[e] = buf(t + T * e);
+    for (int e = 0; e < E; ++e) x[e] = slot_of<L>(buf, t + T * e);
     if constexpr (is_dual_buf<Buf>::value)
       buf.flip();
     else

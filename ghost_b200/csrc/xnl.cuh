@@ -162,12 +162,11 @@ __device__ __forceinline__ void xnl_fft8(C (&x)[8], int t, C *xb, const C *tw) {
 }
 
 // E = 16 (FP32): 16 x 16, 16 x 8 or 8 x 8 x 8.  xb: the line's exchange
-// buffer, slot idx at xb[(idx + idx/PAD) STR]; t2, t3: this lane's twiddle
+// buffer (M + M/PAD slots); t2, t3: this lane's twiddle
 // pairs (see XnlGeom).
 template <int M, int S, int STR>
 __device__ __forceinline__ void xnl_fft16(float2 (&x)[16], int t, float2 *xb, const float4 *t2, const float4 *t3) {
-  constexpr int T = M / 16, PAD = M <= 256 ? 16 : 8;
-  auto slot = [&](int idx) -> float2 & { return xb[(idx + idx / PAD) * STR]; };
+  constexpr int T = M / 16;
   auto tw = [](float2 &v, float2 w) { v = twmul<S>(v, w); };
   if constexpr (M == 256) {
     pdft16<S>(x);
@@ -212,7 +211,13 @@ __device__ __forceinline__ void xnl_fft16(float2 (&x)[16], int t, float2 *xb, co
     __syncwarp();
   } else {
     static_assert(M == 512, "line length");
-    // 8 x 8 x 8, two butterflies per lane and stage: b = t, t + 32
+    // 8 x 8 x 8, two butterflies per lane and stage: b = t, t + 32.  The 16
+    // lanes of a shared-memory phase use 16 banks: the first stage writes
+    // idx = 8 b + r to slot idx + idx/16, the second 64 (b/8) + b%8 + 8 r to
+    // idx + 8 (idx/64), and both are read contiguously.  (With idx + idx/8 for
+    // both the reads took twice the phases: 22.2 -> 19.8 ms a step of 1024 x 1024 x 256
+    // Boussinesq.)
+    auto slot = [&](int st, int idx) -> float2 & { return xb[(st == 0 ? idx + idx / 16 : idx + idx / 64 * 8) * STR]; };
 #pragma unroll
     for (int st = 0; st < 3; ++st) {
 #pragma unroll
@@ -236,13 +241,13 @@ __device__ __forceinline__ void xnl_fft16(float2 (&x)[16], int t, float2 *xb, co
           const int bb = t + 32 * b;
           const int base = st == 0 ? 8 * bb : 64 * (bb / 8) + (bb & 7);
 #pragma unroll
-          for (int r = 0; r < 8; ++r) slot(base + (st == 0 ? r : 8 * r)) = v[r];
+          for (int r = 0; r < 8; ++r) slot(st, base + (st == 0 ? r : 8 * r)) = v[r];
         }
       }
       if (st < 2) {
         __syncwarp();
 #pragma unroll
-        for (int e = 0; e < 16; ++e) x[e] = slot(t + T * e);
+        for (int e = 0; e < 16; ++e) x[e] = slot(st, t + T * e);
         __syncwarp();
       }
     }

@@ -28,14 +28,15 @@ template <typename R> struct ZWriter<ZGrad<R>> { static constexpr bool value = t
 // Whether lines of N points are kept inside a warp, with z_warp_E values a lane.
 // At 256 points the FP32 inverses stay with zpipe_kernel (us a step of 1024 x
 // 1024 x 256: 6370 here, 6230 there; at 512, with 16 values a lane, 2430 and
-// 2250).  Updates take 4 values a lane where a
-// line allows it: with 8 values of every component, and 255 registers, a 128^3
-// FP64 MHD step's z_fwd took 253 us, with 4 it takes 106 (64^3 FP32: 58 and 47).
+// 2250), and so do the FP64 updates (256^3: 668 and 630), whose 4 values a lane
+// would be two warps a line.  Updates take 4 values a lane: with 8 values of
+// every component, and 255 registers, a 128^3 FP64 MHD step's z_fwd took 253
+// us, with 4 it takes 106 (64^3 FP32: 58 and 47; 128^3 FP32: 79 and 74).
 template <typename R, class Op> constexpr bool z_warp_line(int N) {
-  return N >= 32 && N <= (sizeof(R) == 4 && ZWriter<Op>::value ? 128 : 256);
+  return N >= 32 && N <= ((sizeof(R) == 4 ? ZWriter<Op>::value : ZUpdate<Op>::value) ? 128 : 256);
 }
 template <typename R, class Op> constexpr int z_warp_E(int N) {
-  return ZUpdate<Op>::value && N <= (sizeof(R) == 8 ? 128 : 64) ? 4 : 8;
+  return ZUpdate<Op>::value && N <= 128 ? 4 : 8;
 }
 
 template <typename R, int N, int E, int NL> struct ZWarpGeom {
@@ -43,7 +44,7 @@ template <typename R, int N, int E, int NL> struct ZWarpGeom {
   // a line of the stage starts T values' worth of banks after the one before
   // it, where a shared-memory phase covers several lines
   static constexpr int PITCH = N * ES + (T * ES < 128 ? T * ES : 0);
-  static constexpr int PADL = N + N / 8;  // exchange slots of a line: idx + idx/8
+  static constexpr int PADL = N + N / E;  // exchange slots of a line (zw_slot)
   static constexpr size_t warp = (size_t)NL * LW * PITCH + (size_t)LW * PADL * ES;
   static constexpr int tw_count(int L) {
     int n = 0;
@@ -54,6 +55,15 @@ template <typename R, int N, int E, int NL> struct ZWarpGeom {
   static constexpr size_t smem(int nw) { return nw * warp + (size_t)TW * ES + 16 * nw + 16; }
   static_assert(T >= 4 && T <= 32 && E >= 4 && E <= 8, "a line is 4 to 32 lanes of a warp");
 };
+
+// Exchange slot of value idx after the stage of span L: the lanes of a shared
+// memory phase (16 values of FP32, 8 of FP64, from one line or several) write
+// and read different banks.  The first stage writes idx = E b + r, the ones
+// after it E L (b/L) + b%L + L r; all are read contiguously.
+template <typename C, int T, int E, int L> __device__ __forceinline__ constexpr int zw_slot(int idx) {
+  constexpr int P = sizeof(C) == 8 && T >= 16 ? 16 : 8;
+  return L == 1 ? idx + idx / P : idx + idx / (E * E) * E;
+}
 
 // Stages of radix E and a last one of radix E or less, from span L on; tw: powers 1..Q-1 of the stage's
 // twiddles, L of each.
@@ -78,7 +88,7 @@ __device__ __forceinline__ void zw_fft(C (&x)[E], int t, C *xb, const C *tw) {
       if (LAST) y[q + NB * r] = v[r];
       else {
         const int idx = (b / L) * L * Q + k + r * L;
-        xb[idx + idx / 8] = v[r];
+        xb[zw_slot<C, T, E, L>(idx)] = v[r];
       }
     }
   }
@@ -90,7 +100,7 @@ __device__ __forceinline__ void zw_fft(C (&x)[E], int t, C *xb, const C *tw) {
 #pragma unroll
     for (int e = 0; e < E; ++e) {
       const int idx = t + T * e;
-      x[e] = xb[idx + idx / 8];
+      x[e] = xb[zw_slot<C, T, E, L>(idx)];
     }
     __syncwarp();
     zw_fft<N, E, S, L * Q>(x, t, xb, tw + (L > 1 ? (Q - 1) * L : 0));
