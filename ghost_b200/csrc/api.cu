@@ -1139,9 +1139,8 @@ int ghost_ctx_create(int nx, int ny, int nz, double Lx, double Ly, double Lz, in
   c->nz_glob = nz;
   // the fastest variants measured for long lines (ghost_hd_autotune
   // re-measures): one-stage z ring with four CTAs per SM where the operation
-  // allows it (passes_z.cuh), else two stages and three, and a two-stage y ring
-  // with a second exchange buffer
-  c->tile_cfg = (nz >= 256 ? 38 : 0) | (ny >= 256 ? 8 : 0);
+  // allows it (passes_z.cuh), else two stages and three
+  c->tile_cfg = nz >= 256 ? 38 : 0;
   const size_t rs = precision == GHOST_SINGLE ? 4 : 8;
   c->cbytes = c->nspec * 2 * rs;
   c->rbytes = c->nreal * rs;
@@ -2182,11 +2181,10 @@ int ghost_hd_run(ghost_ctx *c, int nsteps, int ord, double dt, double nu, void *
 
 // Tile variants tried by the autotuners (bit 0: y tiles 16 z-lines wide;
 // bit 1: z CTAs of 128 threads; bits 1 and 2: two-stage z ring, three CTAs
-// per SM; bit 3: two-stage y ring with a second exchange buffer; bits 1, 2 and
-// 5: one-stage z ring, four CTAs per SM, for lines of 256 points or more).
-// Bits 4 and 6 chose FP32 y kernels that the warp-line pass has replaced; they
-// are accepted and change nothing.
-static const int kTileCfgs[] = {0, 1, 2, 3, 6, 7, 8, 14, 38, 46};
+// per SM; bits 1, 2 and 5: one-stage z ring, four CTAs per SM, for lines of 256
+// points or more).  Bits 3, 4 and 6 chose y kernels that the warp-line pass has
+// replaced; they are accepted and change nothing.
+static const int kTileCfgs[] = {0, 1, 2, 3, 6, 7, 38};
 
 // a variant with bit 5 runs the same kernels as without it on z lines
 // shorter than 256 points: the autotuners skip it there

@@ -117,7 +117,7 @@ template <typename R, int N> constexpr size_t ens_y_smem() {
   if constexpr (y_warp_line<R>(N)) return EnsYWarp<R, N>::groups * EnsYWarp<R, N>::group + 1024;
   else {
     constexpr int E = N < 8 ? N : 8;
-    return YGeom<R, N, E, kEnsYBZ, false, ens_y_kb<N>()>::smem_bytes(3);
+    return YGeom<R, N, E, kEnsYBZ, ens_y_kb<N>()>::smem_bytes(3);
   }
 }
 
@@ -131,8 +131,8 @@ template <typename R, int N, int S> __device__ __forceinline__ void ens_y_run(co
         k.nz / ens_y_warp_BZ<R>(), k.ni, k.nf, k.nruns, k.nxh, k.jpos, k.jneg, k.rb, k.rbo, k.ctl);
   } else {
     constexpr int E = N < 8 ? N : 8;
-    ypipe_body<R, N, E, kEnsYBZ, 3, S, false, ens_y_kb<N>()>(vb, nvb, k.maps, k.maps, k.fld, k.tw, k.nz, k.ni, k.nf,
-                                                             k.nruns, k.nxh, k.jpos, k.jneg, k.rb, 0, k.ctl);
+    ypipe_body<R, N, E, kEnsYBZ, 3, S, ens_y_kb<N>()>(vb, nvb, k.maps, k.fld, k.tw, k.nz, k.ni, k.nf, k.nruns, k.nxh,
+                                                      k.jpos, k.jneg, k.rb, k.ctl);
   }
 }
 

@@ -706,38 +706,29 @@ template <typename R> struct ZFwdBouss {
 // can be non-zero: the inverse pass loads only those, the forward pass
 // writes only those (the rest are never read).
 // ====================================================================
-// DUAL: the exchanges alternate between a second buffer of the same size
-// and the tile's own stage buffer, one barrier per exchange and none other
-// than the tile's first (the stage refill is issued after it).  The tile's
-// result then leaves by TMA tensor stores (omaps, boxes of rbo rows) from
-// whichever of the two buffers the last exchange did not use; one thread
-// issues them and, before the next tile's first barrier, waits until they
-// have read shared memory.
-// KB > 1 (short lines, and only without DUAL): a tile holds BZ z-lines of
+// KB > 1 (short lines): a tile holds BZ z-lines of
 // KB consecutive kx indices, one block of BZ x N per kx, so that a CTA of
 // KB BZ N/E threads has enough threads; thread (l, t, kb) with l fastest.
-template <typename R, int N, int E, int BZ, bool DUAL = false, int KB = 1> struct YGeom {
+template <typename R, int N, int E, int BZ, int KB = 1> struct YGeom {
   static constexpr int T = N / E;
   static constexpr int NT = KB * BZ * T;
   static constexpr size_t stage_elems = (size_t)KB * BZ * N;
   static constexpr size_t smem_bytes(int stages) {
-    return ((stages + (DUAL ? 1 : 0)) * stage_elems + N) * sizeof(cx<R>) + 8 * (stages + 1);
+    return (stages * stage_elems + N) * sizeof(cx<R>) + 8 * (stages + 1);
   }
 };
 
-template <typename R, int N, int E, int BZ, int STAGES, int S, bool DUAL = false, int KB = 1>
-__device__ __forceinline__ void ypipe_body(int vb, int nvb, const FieldMaps &maps, const FieldMaps &omaps,
+template <typename R, int N, int E, int BZ, int STAGES, int S, int KB = 1>
+__device__ __forceinline__ void ypipe_body(int vb, int nvb, const FieldMaps &maps,
                                            const Fields<R> &fld, const cx<R> *__restrict__ twg, int nz, int ni,
                                            int nf, int nruns, int nxh, const int *__restrict__ jpos,
-                                           const int *__restrict__ jneg, int rb, int rbo, PipeCtl ctl) {
-  static_assert(KB == 1 || !DUAL, "several kx per tile only without the second buffer");
+                                           const int *__restrict__ jneg, int rb, PipeCtl ctl) {
   using C = cx<R>;
-  using G = YGeom<R, N, E, BZ, DUAL, KB>;
+  using G = YGeom<R, N, E, BZ, KB>;
   constexpr int T = G::T, NT = G::NT;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   C *stage = reinterpret_cast<C *>(smem_raw);
-  C *xb = stage + STAGES * G::stage_elems;  // second exchange buffer (DUAL)
-  C *tw = xb + (DUAL ? G::stage_elems : 0);
+  C *tw = stage + STAGES * G::stage_elems;
   uint64_t *bars = reinterpret_cast<uint64_t *>(tw + N);
   // with one kx per tile the kx offset is the constant 0 and every line is live
   const int tid = threadIdx.x, l = tid % BZ, t = KB == 1 ? tid / BZ : (tid / BZ) % T;
@@ -812,24 +803,16 @@ __device__ __forceinline__ void ypipe_body(int vb, int nvb, const FieldMaps &map
   for (int k = 0;; ++k) {
     const int tile = vb + k * nvb;
     if (tile >= ntiles) break;
-    // DUAL: the refill of the previous tile's slot waits for this tile's
-    // first barrier, which follows every read of that slot (so no barrier
-    // closes a tile)
-    if constexpr (!DUAL) issue(k + STAGES - 1);
+    issue(k + STAGES - 1);
     const int s = k % STAGES;
     const bool ok = (!ctl.stall || injected_stall_wait(&bars[STAGES], ctl.cap)) &&
                     mbar_wait(&bars[s], (uint32_t)(k / STAGES) & 1u, ctl.cap);
-    // DUAL: the previous tile's stores have read their buffer before anyone
-    // writes it again (this barrier orders every later write)
-    if (DUAL && tid == 0) bulk_wait_read_all();
     if (__syncthreads_or(!ok)) {
       if (tid == 0) record_timeout(ctl.status);
-      for (int kk = k; kk < k + STAGES - (DUAL ? 1 : 0); ++kk)
+      for (int kk = k; kk < k + STAGES; ++kk)
         if (vb + kk * nvb < ntiles) mbar_wait(&bars[kk % STAGES], (uint32_t)(kk / STAGES) & 1u, kDrainPolls);
-      if (DUAL && tid == 0) bulk_wait_all();
       return;
     }
-    if constexpr (DUAL) issue(k + STAGES - 1);
     const Tile tl = tile_of(tile);
     // this thread's kx: beyond the last one (a short last group) its line is
     // transformed from zeros and not stored
@@ -847,64 +830,28 @@ __device__ __forceinline__ void ypipe_body(int vb, int nvb, const FieldMaps &map
       const bool live = act && ((S < 0) || jj < jp || jj >= N - jn);
       x[e] = live ? sb[jj * BZ + l] : mk((R)0, (R)0);
     }
-    if constexpr (DUAL) {
-      // The exchanges alternate between the second buffer (half 1, first) and
-      // this tile's stage buffer (half 0): the first exchange barrier follows
-      // every thread's reads of the stage, so the second exchange may write
-      // it, and the second buffer's last reads come before the next tile's
-      // first barrier.
-      int ph = 1;
-      auto buf = dual_buf<C>([sb, xb, l](int idx, int h) -> C & { return (h ? xb : sb)[idx * BZ + l]; }, &ph);
-      line_fft<C, N, E, S>(x, t, tw, buf, sync);
-      // the exchanges used xb, sb, xb, ...: the result goes to the buffer the
-      // last one did not use (its last reads came before that exchange's barrier)
-      C *ob = (fft_exchanges<N, E>() % 2 == 1) ? sb : xb;
+    __syncthreads();  // every read of the stage before the exchanges overwrite it
+    auto buf = [sb, l](int idx) -> C & { return sb[idx * BZ + l]; };
+    line_fft<C, N, E, S>(x, t, tw, buf, sync);
+    C *base = fld.p[tl.f] + (size_t)tl.zb * BZ + l + (size_t)nz * N * (tl.i + kb);
 #pragma unroll
-      for (int e = 0; e < E; ++e) ob[(t + T * e) * BZ + l] = x[e];
-      fence_proxy_async();
-      __syncthreads();
-      if (tid == 0) {
-        // rows written: all of them, or (pruned forward pass) boxes covering
-        // the live rows; the extra rows of a box hold the transform's own
-        // values, in rows nothing reads
-        if (S > 0 || (jp == N && jn == 0)) {
-          for (int r0 = 0; r0 < N; r0 += rbo) tma_store_3d(&omaps.m[tl.f], ob + (size_t)r0 * BZ, tl.zb * BZ * U, r0, tl.i);
-        } else {
-          for (int r0 = 0; r0 < jp; r0 += rbo) tma_store_3d(&omaps.m[tl.f], ob + (size_t)r0 * BZ, tl.zb * BZ * U, r0, tl.i);
-          for (int q = 0; q * rbo < jn; ++q) {
-            const int r0 = N - (q + 1) * rbo;
-            tma_store_3d(&omaps.m[tl.f], ob + (size_t)r0 * BZ, tl.zb * BZ * U, r0, tl.i);
-          }
-        }
-        bulk_commit();
-      }
-    } else {
-      __syncthreads();  // every read of the stage before the exchanges overwrite it
-      auto buf = [sb, l](int idx) -> C & { return sb[idx * BZ + l]; };
-      line_fft<C, N, E, S>(x, t, tw, buf, sync);
-      C *base = fld.p[tl.f] + (size_t)tl.zb * BZ + l + (size_t)nz * N * (tl.i + kb);
-#pragma unroll
-      for (int e = 0; e < E; ++e) {
-        const int jj = t + T * e;
-        if (act && (S > 0 || jj < jp || jj >= N - jn)) base[(size_t)nz * jj] = x[e];
-      }
-      __syncthreads();  // the stage is read before the next refill
+    for (int e = 0; e < E; ++e) {
+      const int jj = t + T * e;
+      if (act && (S > 0 || jj < jp || jj >= N - jn)) base[(size_t)nz * jj] = x[e];
     }
+    __syncthreads();  // the stage is read before the next refill
   }
-  if (DUAL && tid == 0) bulk_wait_all();
 }
 
-template <typename R, int N, int E, int BZ, int STAGES, int S, bool DUAL = false, int KB = 1>
+template <typename R, int N, int E, int BZ, int STAGES, int S, int KB = 1>
 __global__ void __launch_bounds__(KB *BZ *(N / E), 2) ypipe_kernel(const __grid_constant__ FieldMaps maps,
-                                                                 const __grid_constant__ FieldMaps omaps,
                                                                  const __grid_constant__ Fields<R> fld,
                                                                  const cx<R> *__restrict__ twg, int nz, int ni,
                                                                  int nf, int nruns, int nxh,
                                                                  const int *__restrict__ jpos,
-                                                                 const int *__restrict__ jneg, int rb, int rbo,
-                                                                 PipeCtl ctl) {
-  ypipe_body<R, N, E, BZ, STAGES, S, DUAL, KB>(blockIdx.x, gridDim.x, maps, omaps, fld, twg, nz, ni, nf, nruns, nxh,
-                                                jpos, jneg, rb, rbo, ctl);
+                                                                 const int *__restrict__ jneg, int rb, PipeCtl ctl) {
+  ypipe_body<R, N, E, BZ, STAGES, S, KB>(blockIdx.x, gridDim.x, maps, fld, twg, nz, ni, nf, nruns, nxh, jpos, jneg,
+                                         rb, ctl);
 }
 
 // ====================================================================

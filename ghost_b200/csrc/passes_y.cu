@@ -17,62 +17,53 @@ template <typename R, int N, int BZ0> constexpr int y_tile_width() {
 }
 
 // kx indices per y tile: short lines put several kx in one tile so that a
-// CTA has at least 128 threads (not with the second exchange buffer)
-template <int N, int E, int BZ, bool DUAL> constexpr int y_kb() {
-  return (DUAL || BZ * (N / E) >= 128) ? 1 : 128 / (BZ * (N / E));
+// CTA has at least 128 threads
+template <int N, int E, int BZ> constexpr int y_kb() {
+  return BZ * (N / E) >= 128 ? 1 : 128 / (BZ * (N / E));
 }
 
-template <typename R, int N, int S, int BZ0, bool DUAL = false, int E0 = 8>
+template <typename R, int N, int S, int BZ0>
 int launch_y_cfg(ghost_ctx *c, const Fields<R> &f, int nf, const Prune &pr) {
-  constexpr int E = N < E0 ? N : E0, T = N / E;
+  constexpr int E = N < 8 ? N : 8, T = N / E;
   constexpr int BZ = y_tile_width<R, N, BZ0>();
-  constexpr int KB = y_kb<N, E, BZ, DUAL>();
-  using G = YGeom<R, N, E, BZ, DUAL, KB>;
-  constexpr int STAGES = DUAL ? 2 : (G::smem_bytes(3) <= 200 * 1024 ? 3 : 2);
+  constexpr int KB = y_kb<N, E, BZ>();
+  using G = YGeom<R, N, E, BZ, KB>;
+  constexpr int STAGES = G::smem_bytes(3) <= 200 * 1024 ? 3 : 2;
   if (c->nz < BZ) return fail(GHOST_ERR_SIZE, "nz=%d below the y-pass tile width %d", c->nz, BZ);
   const size_t smem = G::smem_bytes(STAGES);
-  auto kern = ypipe_kernel<R, N, E, BZ, STAGES, S, DUAL, KB>;
+  auto kern = ypipe_kernel<R, N, E, BZ, STAGES, S, KB>;
   GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int ni = pr.jpos ? pr.ni : c->nxh;
   const long ntiles = (long)(c->nz / BZ) * ((ni + KB - 1) / KB) * c->nruns * nf;
   const int grid = persistent_grid(c, kern, KB * BZ * T, smem, ntiles);
   // box rows: 32 (or N/2) for the pruned inverse, whole halves otherwise
   const int rb = (pr.jpos && S > 0) ? std::min(32, N / 2) : std::min(N, 256);
-  // store boxes of the dual-buffer variant (TMA stores): whole halves for the
-  // inverse, 32 rows for the forward pass, whose pruned tiles store the live
-  // rows only; both divide N
-  const int rbo = S > 0 ? std::min(N, 256) : std::min(N, 32);
   const unsigned U = sizeof(R) == 4 ? 1 : 2;
-  FieldMaps maps, omaps;
+  FieldMaps maps;
   for (int q = 0; q < nf; ++q) GB_CHECK(field_map(c, f.p[q], BZ * U, rb, 1, &maps.m[q]));
-  if (DUAL)
-    for (int q = 0; q < nf; ++q) GB_CHECK(field_map(c, f.p[q], BZ * U, rbo, 1, &omaps.m[q]));
   const int ts = timer_begin(c, S > 0 ? GHOST_TIMER_Y_INV : GHOST_TIMER_Y_FWD);
-  GB_CHECK(launch_dep(c, nf, kern, grid, KB * BZ * T, smem, maps, DUAL ? omaps : maps, f, (const cx<R> *)c->tw_y, c->nz, ni, nf, c->nruns, c->nxh, pr.jpos, pr.jneg, rb, rbo, pipe_ctl(c)));
+  GB_CHECK(launch_dep(c, nf, kern, grid, KB * BZ * T, smem, maps, f, (const cx<R> *)c->tw_y, c->nz, ni, nf, c->nruns,
+                      c->nxh, pr.jpos, pr.jneg, rb, pipe_ctl(c)));
   timer_end(c, ts);
   return post_launch(c);
 }
 
 // tiles 8 z-lines wide, or 16 with tile variant bit 0
 template <typename R, int N, int S> int launch_y_n(ghost_ctx *c, const Fields<R> &f, int nf, const Prune &pr) {
-  // lines the warp-line kernel takes, whatever the tile variant (its y bits
-  // choose between the kernels of other line lengths)
-  if constexpr (y_warp_line<R>(N)) return launch_ywarp<R, S>(c, f, nf, pr);
-  else {
-  // the 16-wide tile needs two stages of 16 lines in shared memory; where
-  // that does not fit (FP64, long lines) the variant falls back to 8
-  constexpr int E = N < 8 ? N : 8, T = N / E;
-  constexpr int BZ16 = 16 * T <= 1024 ? 16 : 1024 / T;
-  constexpr bool fits16 = YGeom<R, N, E, BZ16>::smem_bytes(2) <= 227 * 1024;
-  if constexpr (fits16) {
-    if ((c->tile_cfg & 1) && c->nz >= 16) return launch_y_cfg<R, N, S, 16>(c, f, nf, pr);
-  }
-  // bit 3: two stages and a second exchange buffer (one barrier per exchange)
-  constexpr bool fits_dual = YGeom<R, N, E, 8, true>::smem_bytes(2) <= 113 * 1024;
-  if constexpr (N >= 256 && fits_dual) {
-    if (c->tile_cfg & 8) return launch_y_cfg<R, N, S, 8, true>(c, f, nf, pr);
-  }
-  return launch_y_cfg<R, N, S, 8>(c, f, nf, pr);
+  // lines the warp-line kernel takes, whatever the tile variant (its y bit
+  // chooses between the tiles of other line lengths)
+  if constexpr (y_warp_line<R>(N)) {
+    return launch_ywarp<R, S>(c, f, nf, pr);
+  } else {
+    // the 16-wide tile needs two stages of 16 lines in shared memory; where
+    // that does not fit (FP64, long lines) the variant falls back to 8
+    constexpr int E = N < 8 ? N : 8, T = N / E;
+    constexpr int BZ16 = 16 * T <= 1024 ? 16 : 1024 / T;
+    constexpr bool fits16 = YGeom<R, N, E, BZ16>::smem_bytes(2) <= 227 * 1024;
+    if constexpr (fits16) {
+      if ((c->tile_cfg & 1) && c->nz >= 16) return launch_y_cfg<R, N, S, 16>(c, f, nf, pr);
+    }
+    return launch_y_cfg<R, N, S, 8>(c, f, nf, pr);
   }
 }
 

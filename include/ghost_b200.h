@@ -94,13 +94,12 @@ int ghost_ctx_set_kmax(ghost_ctx *ctx, double kmax);
  * plays this role in fftp-3/fftp3D.fpp:92-107), for the line lengths that
  * are not kept inside a warp: bit 0 y tiles 16 z-lines wide instead of 8; bit
  * 1 z-pass CTAs of 128 threads instead of 256; bits 1 and 2 together a
- * two-stage z ring with three CTAs per SM; bit 3 a two-stage y ring with a
- * second exchange buffer; bits 1, 2 and 5 (z lines of 256 points or more) a
- * one-stage z ring with four CTAs per SM.  The other bits are accepted; bit 8
- * picks the fused x pass of FP32 1024-point lines that is not kept inside a
- * warp, bits 4, 6 and 7 change nothing.  Results do not depend on the variant
- * (0..511).  Default: bits 1, 2 and 5 for z lines of 256 points or more, bit 3
- * for such y lines. */
+ * two-stage z ring with three CTAs per SM; bits 1, 2 and 5 (z lines of 256
+ * points or more) a one-stage z ring with four CTAs per SM.  The other bits
+ * are accepted; bit 8 picks the fused x pass of FP32 1024-point lines that is
+ * not kept inside a warp, bits 3, 4, 6 and 7 change nothing.  Results do not
+ * depend on the variant (0..511).  Default: bits 1, 2 and 5 for z lines of 256
+ * points or more. */
 int ghost_ctx_set_tile_cfg(ghost_ctx *ctx, int cfg);
 int ghost_ctx_get_tile_cfg(const ghost_ctx *ctx, int *cfg);
 /* Times one RK step of every tile variant on a copy of v (device arrays;
