@@ -661,9 +661,17 @@ template <typename R> int c2r_dev(ghost_ctx *c, const void *in, void *out) {
 }
 
 // Six real fields to spectra at once (the stresses of the LES closure):
-// x r2c per field, then one y and one z pass over all six.
+// one pass of each axis over all six (x one by one where the warp-line
+// transform does not take the grid).
 template <typename R> int r2c6_dev(ghost_ctx *c, const void *const in[6], void *const out[6]) {
-  for (int q = 0; q < 6; ++q) GB_CHECK((launch_x<R, X_R2C>(c, in[q], out[q])));
+  if (xline_takes(c)) {
+    const int ts = timer_begin(c, GHOST_TIMER_X_R2C);
+    GB_CHECK(launch_xline_r2c(c, in, out, 6));
+    timer_end(c, ts);
+    GB_CHECK(post_launch(c));
+  } else {
+    for (int q = 0; q < 6; ++q) GB_CHECK((launch_x<R, X_R2C>(c, in[q], out[q])));
+  }
   Fields<R> f{};
   for (int q = 0; q < 6; ++q) f.p[q] = (cx<R> *)out[q];
   GB_CHECK((launch_y<R, -1>(c, f, 6)));

@@ -110,7 +110,7 @@ int launch_xnl(ghost_ctx *c, bool bouss, const void *const *ins, void *const *ou
 // plain x transforms with lines kept inside a warp (xplain.cuh): whether they
 // take this grid, and their launches
 bool xline_takes(const ghost_ctx *c);
-int launch_xline_r2c(ghost_ctx *c, const void *in, void *out);
+int launch_xline_r2c(ghost_ctx *c, const void *const *in, void *const *out, int nf);  // nf <= 12 fields
 int launch_xline_c2r(ghost_ctx *c, const void *in, void *out);
 bool xline_features_takes(const ghost_ctx *c, const void *x);
 int launch_xline_features(ghost_ctx *c, const void *const *spec, float *x, float gs, float delta);

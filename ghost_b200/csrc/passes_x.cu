@@ -138,7 +138,7 @@ template <typename R, int NX, int KIND> int launch_x_n(ghost_ctx *c, const void 
   } else if (KIND == X_C2R && xline_takes(c)) {
     GB_CHECK(launch_xline_c2r(c, in, out));
   } else if (KIND == X_R2C && xline_takes(c)) {
-    GB_CHECK(launch_xline_r2c(c, in, out));
+    GB_CHECK(launch_xline_r2c(c, &in, &out, 1));
   } else if (KIND == X_C2R) {
     const size_t smem = (size_t)(NX + (M + 1) * BZ + M * BZ) * sizeof(C);
     auto kern = xpass_c2r_kernel<R, NX, E, BZ>;

@@ -18,7 +18,7 @@ static CUtensorMapSwizzle swizzle_of(int row_bytes) {
   return row_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
 }
 
-template <typename R, int NX, int E, int BZ> static int r2c(ghost_ctx *c, const void *in, void *out) {
+template <typename R, int NX, int E, int BZ> static int r2c(ghost_ctx *c, const void *const *in, void *const *out, int nf) {
   using G = XnlGeom<R, NX, E, BZ, E>;
   using P = XPlainGeom<R, NX, E, BZ>;
   constexpr int STAGES = P::r2c(3) <= 110 * 1024 ? 3 : 2;
@@ -27,10 +27,15 @@ template <typename R, int NX, int E, int BZ> static int r2c(ghost_ctx *c, const 
   static_assert(smem <= 227 * 1024, "shared memory");
   GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const XnlBoxes bx(G::M + 1);
-  CUtensorMap m;
-  GB_CHECK(field_map(c, out, BZ * G::ES / 8, 1, bx.rb, &m, swizzle_of(G::RB)));
-  const int grid = persistent_grid(c, kern, G::NT, smem, (long)(c->nz / BZ) * c->ny);
-  GB_CHECK(launch_dep(c, 1, kern, grid, G::NT, smem, (const R *)in, m, (const cx<R> *)c->tw_x, c->ny, c->nz, bx.nbox, bx.rb, pipe_ctl(c)));
+  CFields<R> f{};
+  FieldMaps maps;
+  for (int q = 0; q < nf; ++q) {
+    f.p[q] = (const cx<R> *)in[q];
+    GB_CHECK(field_map(c, out[q], BZ * G::ES / 8, 1, bx.rb, &maps.m[q], swizzle_of(G::RB)));
+  }
+  const int grid = persistent_grid(c, kern, G::NT, smem, (long)(c->nz / BZ) * c->ny * nf);
+  GB_CHECK(launch_dep(c, nf, kern, grid, G::NT, smem, f, maps, (const cx<R> *)c->tw_x, c->ny, c->nz, nf, bx.nbox, bx.rb,
+                      pipe_ctl(c)));
   return GHOST_OK;
 }
 
@@ -84,7 +89,7 @@ static int features(ghost_ctx *c, const void *const *spec, float *x, float gs, f
   }                                                                   \
   return fail(GHOST_ERR_SIZE, "nx=%d has no warp-line x transform", c->nx);
 
-int launch_xline_r2c(ghost_ctx *c, const void *in, void *out) { GB_LINES(r2c, in, out) }
+int launch_xline_r2c(ghost_ctx *c, const void *const *in, void *const *out, int nf) { GB_LINES(r2c, in, out, nf) }
 int launch_xline_c2r(ghost_ctx *c, const void *in, void *out) { GB_LINES(c2r, in, out) }
 
 // the closure's rows of a tile fit shared memory up to 128-point lines, and
