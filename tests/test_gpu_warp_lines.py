@@ -54,3 +54,22 @@ def test_warp_line_y_and_z_passes(prec, shape):
     gb.bouss_run(2, *args, *V, TH)
     rv, rt = ob.bouss_run(2, *args, v, th)
     assert rel_l2(host(V) + [to_host(TH)], list(rv) + [rt]) <= tol
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("n", [32, 64, 128])
+def test_stresses_through_one_x_pass(prec, n):
+    """The six stresses of the closure as spectra: x one by one below 64
+    points, in one launch from there on.  The rows are float32, so the error is
+    that of six transforms, a sum of three of them and a projection."""
+    from ghost_b200 import Ghost
+    from ghost_b200.les import LES
+    from oracle import les_oracle
+    co, gc = Oracle(n), Ghost(n, precision=prec)
+    kc = n // 3
+    co.set_kmax(float(kc * kc))
+    les = LES(gc, kc)
+    tau = np.random.default_rng(n).standard_normal((n ** 3, 6)).astype(np.float32)
+    F = les.tau_force(to_dev(tau), 0.25)
+    ref = les_oracle.tau_force(co, tau.astype(np.float64), 0.25)
+    assert rel_l2([to_host(x) for x in F], ref) <= (1e-13 if prec == "fp64" else 2e-6)
