@@ -73,8 +73,10 @@ template <typename R, int N, class Op> int launch_zwarp(ghost_ctx *c, const Op &
   // few lines: one warp per CTA, so that every SM has work (a 64^3 FP64 step
   // has 740 live lines)
   if (nlines < 8 * ZWarpGeom<R, N, E, Op::NLOAD>::LW * sm_count(c))
-    return launch_zwarp_cfg<R, N, E, 1, 4 * MINB>(c, op, pr);
-  return launch_zwarp_cfg<R, N, E, 4, MINB>(c, op, pr);
+    return launch_zwarp_cfg<R, N, E, 1, (N == 512 ? 6 : 4 * MINB)>(c, op, pr);
+  // 512 points: three warps and their lines of three fields are half an SM's shared memory
+  if constexpr (N == 512) return launch_zwarp_cfg<R, N, E, 3, 2>(c, op, pr);
+  else return launch_zwarp_cfg<R, N, E, 4, MINB>(c, op, pr);
 }
 
 // CTAs of 256 threads; with tile variant bit 1 of 128 threads; with bits 1

@@ -32,11 +32,15 @@ template <typename R> struct ZWriter<ZGrad<R>> { static constexpr bool value = t
 // would be two warps a line.  Updates take 4 values a lane: with 8 values of
 // every component, and 255 registers, a 128^3 FP64 MHD step's z_fwd took 253
 // us, with 4 it takes 106 (64^3 FP32: 58 and 47; 128^3 FP32: 79 and 74).
+// FP64 operations of up to three loads take 512 points too, 16 values a lane:
+// CTA-wide, 4 values a thread were four exchanges (512^3 z_inv 6180 -> 3380 us a
+// step, 256 x 256 x 512 plain transforms 398 -> 202 us a pair).
 template <typename R, class Op> constexpr bool z_warp_line(int N) {
-  return N >= 32 && N <= ((sizeof(R) == 4 ? ZWriter<Op>::value : ZUpdate<Op>::value) ? 128 : 256);
+  if (sizeof(R) == 4) return N >= 32 && N <= (ZWriter<Op>::value ? 128 : 256);
+  return N >= 32 && N <= (ZUpdate<Op>::value ? 128 : (Op::NLOAD <= 3 ? 512 : 256));
 }
 template <typename R, class Op> constexpr int z_warp_E(int N) {
-  return ZUpdate<Op>::value && N <= 128 ? 4 : 8;
+  return N == 512 ? 16 : (ZUpdate<Op>::value && N <= 128 ? 4 : 8);
 }
 
 template <typename R, int N, int E, int NL> struct ZWarpGeom {
@@ -44,32 +48,34 @@ template <typename R, int N, int E, int NL> struct ZWarpGeom {
   // a line of the stage starts T values' worth of banks after the one before
   // it, where a shared-memory phase covers several lines
   static constexpr int PITCH = N * ES + (T * ES < 128 ? T * ES : 0);
-  static constexpr int PADL = N + N / E;  // exchange slots of a line (zw_slot)
+  static constexpr int RX = E < 8 ? E : 8;  // radix of the stages
+  static constexpr int PADL = N + N / RX;   // exchange slots of a line (zw_slot)
   static constexpr size_t warp = (size_t)NL * LW * PITCH + (size_t)LW * PADL * ES;
   static constexpr int tw_count(int L) {
     int n = 0;
-    for (; L < N; L *= E) n += (N / L < E ? N / L - 1 : E - 1) * L;
+    for (; L < N; L *= RX) n += (N / L < RX ? N / L - 1 : RX - 1) * L;
     return n;
   }
-  static constexpr int TW = tw_count(E);
+  static constexpr int TW = tw_count(RX);
   static constexpr size_t smem(int nw) { return nw * warp + (size_t)TW * ES + 16 * nw + 16; }
-  static_assert(T >= 4 && T <= 32 && E >= 4 && E <= 8, "a line is 4 to 32 lanes of a warp");
+  static_assert(T >= 4 && T <= 32 && E >= 4 && E <= 16, "a line is 4 to 32 lanes of a warp");
 };
 
 // Exchange slot of value idx after the stage of span L: the lanes of a shared
 // memory phase (16 values of FP32, 8 of FP64, from one line or several) write
-// and read different banks.  The first stage writes idx = E b + r, the ones
-// after it E L (b/L) + b%L + L r; all are read contiguously.
-template <typename C, int T, int E, int L> __device__ __forceinline__ constexpr int zw_slot(int idx) {
+// and read different banks.  The first stage writes idx = RX b + r, the
+// ones after it RX L (b/L) + b%L + L r; all are read contiguously.
+template <typename C, int T, int RX, int L> __device__ __forceinline__ constexpr int zw_slot(int idx) {
   constexpr int P = sizeof(C) == 8 && T >= 16 ? 16 : 8;
-  return L == 1 ? idx + idx / P : idx + idx / (E * E) * E;
+  return L == 1 ? idx + idx / P : idx + idx / (RX * RX) * RX;
 }
 
-// Stages of radix E and a last one of radix E or less, from span L on; tw: powers 1..Q-1 of the stage's
+// Stages of radix 8 (4 where a lane holds 4 values) and a last one of that or
+// less, from span L on; tw: powers 1..Q-1 of the stage's
 // twiddles, L of each.
 template <int N, int E, int S, int L, typename C>
 __device__ __forceinline__ void zw_fft(C (&x)[E], int t, C *xb, const C *tw) {
-  constexpr int T = N / E, Q = N / L < E ? N / L : E, NB = E / Q;
+  constexpr int T = N / E, RX = E < 8 ? E : 8, Q = N / L < RX ? N / L : RX, NB = E / Q;
   constexpr bool LAST = L * Q == N;
   C y[E];
 #pragma unroll
@@ -88,7 +94,7 @@ __device__ __forceinline__ void zw_fft(C (&x)[E], int t, C *xb, const C *tw) {
       if (LAST) y[q + NB * r] = v[r];
       else {
         const int idx = (b / L) * L * Q + k + r * L;
-        xb[zw_slot<C, T, E, L>(idx)] = v[r];
+        xb[zw_slot<C, T, RX, L>(idx)] = v[r];
       }
     }
   }
@@ -100,7 +106,7 @@ __device__ __forceinline__ void zw_fft(C (&x)[E], int t, C *xb, const C *tw) {
 #pragma unroll
     for (int e = 0; e < E; ++e) {
       const int idx = t + T * e;
-      x[e] = xb[zw_slot<C, T, E, L>(idx)];
+      x[e] = xb[zw_slot<C, T, RX, L>(idx)];
     }
     __syncwarp();
     zw_fft<N, E, S, L * Q>(x, t, xb, tw + (L > 1 ? (Q - 1) * L : 0));
@@ -138,8 +144,8 @@ __device__ __forceinline__ void zwarp_body(int w, int nw, int wc, unsigned char 
   {
     int o = 0;
 #pragma unroll
-    for (int L = E; L < N; L *= E) {
-      const int Q = N / L < E ? N / L : E;
+    for (int L = G::RX; L < N; L *= G::RX) {
+      const int Q = N / L < G::RX ? N / L : G::RX;
       for (int q = threadIdx.x; q < (Q - 1) * L; q += 32 * NWC) tw[o + q] = twg[(q % L) * (q / L + 1) * (N / (L * Q))];
       o += (Q - 1) * L;
     }
