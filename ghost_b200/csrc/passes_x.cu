@@ -29,7 +29,8 @@ int launch_x_fused(ghost_ctx *c, const void *const *ins, void *const *outs, int 
   using G = XGeom<R, NX, BZ, YB>;
   constexpr size_t cap = 220 * 1024 / MINB;  // four stages while MINB CTAs fit an SM
   constexpr int STAGES = G::smem_bytes(4) <= cap ? 4 : (G::smem_bytes(3) <= 200 * 1024 ? 3 : 2);
-  const size_t smem = G::smem_bytes(STAGES);
+  constexpr size_t smem = G::smem_bytes(STAGES);
+  static_assert(smem <= 227 * 1024, "shared memory");
   auto kern = xpipe_nl_kernel<R, NX, E, BZ, PHYS, STAGES, MINB, YB>;
   GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   Fields<R> fo{};

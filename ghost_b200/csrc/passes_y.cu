@@ -30,7 +30,8 @@ int launch_y_cfg(ghost_ctx *c, const Fields<R> &f, int nf, const Prune &pr) {
   using G = YGeom<R, N, E, BZ, KB>;
   constexpr int STAGES = G::smem_bytes(3) <= 200 * 1024 ? 3 : 2;
   if (c->nz < BZ) return fail(GHOST_ERR_SIZE, "nz=%d below the y-pass tile width %d", c->nz, BZ);
-  const size_t smem = G::smem_bytes(STAGES);
+  constexpr size_t smem = G::smem_bytes(STAGES);
+  static_assert(smem <= 227 * 1024, "shared memory");
   auto kern = ypipe_kernel<R, N, E, BZ, STAGES, S, KB>;
   GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int ni = pr.jpos ? pr.ni : c->nxh;

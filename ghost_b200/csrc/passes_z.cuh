@@ -22,8 +22,10 @@ template <typename R, int N, int LPB, int STAGES0, int MINB, class Op>
 int launch_z_cfg(ghost_ctx *c, const Op &op, const Prune &pr) {
   constexpr int E = zE<R>() < N ? zE<R>() : N, T = N / E;
   using G = ZGeom<R, N, E, LPB, Op::NLOAD>;
-  constexpr int STAGES = G::smem_bytes(STAGES0) <= 200 * 1024 ? STAGES0 : 2;
-  const size_t smem = G::smem_bytes(STAGES);
+  // (six fields of 1024-point FP64 lines: two stages are 249 KB, one is 151)
+  constexpr int STAGES = G::smem_bytes(STAGES0) <= 200 * 1024 ? STAGES0 : (G::smem_bytes(2) <= 227 * 1024 ? 2 : 1);
+  constexpr size_t smem = G::smem_bytes(STAGES);
+  static_assert(smem <= 227 * 1024, "shared memory");
   const int nlines = pr.lines ? pr.nlines : c->ny * c->nxh * c->nruns;
   auto kern = zpipe_kernel<R, N, E, LPB, STAGES, MINB, Op>;
   GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

@@ -673,7 +673,8 @@ def test_mhd(prec):
 
 
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])
-@pytest.mark.parametrize("shape", [(16, 16, 16), (512, 16, 32), (16, 512, 32), (32, 16, 512), (1024, 16, 16)])
+@pytest.mark.parametrize("shape", [(16, 16, 16), (512, 16, 32), (16, 512, 32), (32, 16, 512), (1024, 16, 16),
+                                   (16, 1024, 16), (16, 16, 1024)])
 def test_mhd_line_lengths(prec, shape):
     """The fused MHD passes at the shortest and longest lines of each axis:
     two RK2 steps (the first substep full, the others zero-pruned) from fields
