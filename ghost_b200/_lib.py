@@ -125,6 +125,7 @@ SIGNATURES = {
     "ghost_mlp_create": [I, ctypes.POINTER(P)],
     "ghost_mlp_destroy": [P],
     "ghost_mlp_set_stream": [P, P],
+    "ghost_mlp_inject_stall": [P, I],
     "ghost_mlp_get_params": [P, P],
     "ghost_mlp_set_params": [P, P],
     "ghost_mlp_forward": [P, P, P, I],

@@ -591,10 +591,18 @@ __global__ void __launch_bounds__(2 * THREADS, 4) mlp_infer2_kernel(Gmlp g) {
 // row in order and the first warp adds the 8 sums in order, so the result is
 // the same on every run.  21 blocks summing the 148 rows one after the other
 // took 13 us, the loss being one thread's chain of loads.
+// A CTA of the training kernel whose wait ran out leaves its row unwritten, so
+// with the status word set nothing is summed and the weights stay as they are
+// until the host has seen it; status[1] keeps the first step left out.
 constexpr int ADAM_COLS = 32, ADAM_WARPS = 8;
 __global__ void __launch_bounds__(32 * ADAM_WARPS) adam_kernel(float *P, float *M, float *V, const float *partials,
                                                                int nparts, int step, float lr, float b1, float b2,
-                                                               float eps, float *grad_out, double *loss_out) {
+                                                               float eps, float *grad_out, double *loss_out,
+                                                               int *status) {
+  if (status[0] != 0) {
+    if (blockIdx.x == 0 && threadIdx.x == 0 && step > 0 && status[1] == 0) status[1] = step;
+    return;
+  }
   __shared__ double sh[ADAM_WARPS][ADAM_COLS];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, q = blockIdx.x * ADAM_COLS + lane;
   if (q < NPARAM) {
@@ -639,15 +647,16 @@ struct ghost_mlp {
   int step = 0;
   int device = 0;
   cudaStream_t stream = nullptr;
-  int *status = nullptr;
+  int *status = nullptr;  // GHOST_ERR_TIMEOUT or 0, and the first training step left out because of it
   uint32_t cap = 1u << 22;
+  bool stall = false;  // fault injection: waits give up at once
 };
 
 static int mlp_launch(ghost_mlp *m, const float *x, const float *t, float *y, int B, bool train) {
   int nsm = 148;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, m->device);
   const int ntiles = (B + ROWS - 1) / ROWS;
-  Gmlp g{m->P, x, t, y, train ? m->partials : nullptr, B, 2.f / ((float)B * (float)NOUT), m->status, m->cap};
+  Gmlp g{m->P, x, t, y, train ? m->partials : nullptr, B, 2.f / ((float)B * (float)NOUT), m->status, m->stall ? 0u : m->cap};
   if (train) {
     // one CTA per SM; the per-CTA gradient partials are summed by the Adam kernel
     const int grid = std::max(1, std::min(ntiles, nsm));
@@ -676,12 +685,15 @@ static bool dev_ptr(const void *p) {
   return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
 }
 
+// Reads and clears the status words (the caller has synchronised).  After a
+// timeout the step count goes back to the last step that was taken.
 static int mlp_check_status(ghost_mlp *m) {
-  int st = 0;
-  MLP_CUDA(cudaMemcpy(&st, m->status, sizeof(int), cudaMemcpyDeviceToHost));
-  if (st) {
-    cudaMemset(m->status, 0, sizeof(int));
-    return fail(GHOST_ERR_TIMEOUT, "an MMA completion wait gave up");
+  int st[2] = {0, 0};
+  MLP_CUDA(cudaMemcpy(st, m->status, sizeof(st), cudaMemcpyDeviceToHost));
+  if (st[0]) {
+    MLP_CUDA(cudaMemset(m->status, 0, sizeof(st)));
+    if (st[1] > 0) m->step = st[1] - 1;
+    return fail(GHOST_ERR_TIMEOUT, "an MMA completion wait gave up: calls since then gave no result");
   }
   return GHOST_OK;
 }
@@ -699,7 +711,7 @@ int ghost_mlp_create(int seed, ghost_mlp **out) {
   if (cudaMalloc(&m->P, pb) != cudaSuccess || cudaMalloc(&m->M, pb) != cudaSuccess ||
       cudaMalloc(&m->V, pb) != cudaSuccess || cudaMalloc(&m->grad, pb) != cudaSuccess ||
       cudaMalloc(&m->partials, sizeof(float) * (size_t)nsm * (NPARAM + 1)) != cudaSuccess ||
-      cudaMalloc(&m->loss, sizeof(double)) != cudaSuccess || cudaMalloc(&m->status, sizeof(int)) != cudaSuccess) {
+      cudaMalloc(&m->loss, sizeof(double)) != cudaSuccess || cudaMalloc(&m->status, 2 * sizeof(int)) != cudaSuccess) {
     cudaGetLastError();
     ghost_mlp_destroy(m);
     return fail(GHOST_ERR_ALLOC, "MLP buffers");
@@ -718,7 +730,7 @@ int ghost_mlp_create(int seed, ghost_mlp **out) {
   cudaMemcpy(m->P, h.data(), pb, cudaMemcpyHostToDevice);
   cudaMemset(m->M, 0, pb);
   cudaMemset(m->V, 0, pb);
-  cudaMemset(m->status, 0, sizeof(int));
+  cudaMemset(m->status, 0, 2 * sizeof(int));
   *out = m;
   return GHOST_OK;
 }
@@ -743,9 +755,17 @@ int ghost_mlp_set_stream(ghost_mlp *m, void *stream) {
   return GHOST_OK;
 }
 
+int ghost_mlp_inject_stall(ghost_mlp *m, int enable) {
+  if (!m) return fail(GHOST_ERR_ARG, "null mlp");
+  m->stall = enable != 0;
+  return GHOST_OK;
+}
+
 int ghost_mlp_get_params(ghost_mlp *m, float *host) {
   if (!m || !host) return fail(GHOST_ERR_ARG, "null argument");
   MLP_CUDA(cudaStreamSynchronize(m->stream));
+  const int st = mlp_check_status(m);
+  if (st) return st;
   MLP_CUDA(cudaMemcpy(host, m->P, sizeof(float) * NPARAM, cudaMemcpyDeviceToHost));
   return GHOST_OK;
 }
@@ -772,15 +792,16 @@ int ghost_mlp_gradients(ghost_mlp *m, const float *x, const float *t, int B, flo
   int st = mlp_launch(m, x, t, nullptr, B, true);
   if (st) return st;
   adam_kernel<<<(NPARAM + ADAM_COLS) / ADAM_COLS, 32 * ADAM_WARPS, 0, m->stream>>>(m->P, m->M, m->V, m->partials, m->nparts, 0, 0.f, 0.9f,
-                                                            0.999f, 1e-8f, m->grad, m->loss);
+                                                            0.999f, 1e-8f, m->grad, m->loss, m->status);
   MLP_CUDA(cudaGetLastError());
   MLP_CUDA(cudaStreamSynchronize(m->stream));
+  if ((st = mlp_check_status(m))) return st;
   if (grad_host) MLP_CUDA(cudaMemcpy(grad_host, m->grad, sizeof(float) * NPARAM, cudaMemcpyDeviceToHost));
   if (loss) {
     MLP_CUDA(cudaMemcpy(loss, m->loss, sizeof(double), cudaMemcpyDeviceToHost));
     *loss /= (double)B * NOUT;
   }
-  return mlp_check_status(m);
+  return GHOST_OK;
 }
 
 int ghost_mlp_train_step(ghost_mlp *m, const float *x, const float *t, int B, float lr, double *loss) {
@@ -790,7 +811,7 @@ int ghost_mlp_train_step(ghost_mlp *m, const float *x, const float *t, int B, fl
   if (st) return st;
   m->step += 1;
   adam_kernel<<<(NPARAM + ADAM_COLS) / ADAM_COLS, 32 * ADAM_WARPS, 0, m->stream>>>(m->P, m->M, m->V, m->partials, m->nparts, m->step, lr,
-                                                            0.9f, 0.999f, 1e-8f, nullptr, m->loss);
+                                                            0.9f, 0.999f, 1e-8f, nullptr, m->loss, m->status);
   MLP_CUDA(cudaGetLastError());
   if (loss) {
     MLP_CUDA(cudaMemcpyAsync(loss, m->loss, sizeof(double), cudaMemcpyDeviceToHost, m->stream));

@@ -528,6 +528,12 @@
          TYPE(C_PTR), VALUE :: mlp, stream
          INTEGER(C_INT) :: s
        END FUNCTION
+       FUNCTION ghost_mlp_inject_stall(mlp,enable) BIND(C,name="ghost_mlp_inject_stall") RESULT(s)
+         IMPORT :: C_INT, C_PTR
+         TYPE(C_PTR), VALUE :: mlp
+         INTEGER(C_INT), VALUE :: enable
+         INTEGER(C_INT) :: s
+       END FUNCTION
        FUNCTION ghost_mlp_get_params(mlp,params) BIND(C,name="ghost_mlp_get_params") RESULT(s)
          IMPORT :: C_INT, C_PTR, C_FLOAT
          TYPE(C_PTR), VALUE :: mlp

@@ -467,6 +467,12 @@ typedef struct ghost_mlp ghost_mlp;
 int ghost_mlp_create(int seed, ghost_mlp **mlp);
 int ghost_mlp_destroy(ghost_mlp *mlp);
 int ghost_mlp_set_stream(ghost_mlp *mlp, void *stream);
+/* Fault injection: with enable != 0 every bounded wait of the network's
+ * kernels gives up at once.  Nothing faults or hangs and nothing is computed:
+ * a training step leaves the weights as they are, and the next call that
+ * synchronises (train_step with a loss, gradients, get_params) returns
+ * GHOST_ERR_TIMEOUT, as after a real timeout. */
+int ghost_mlp_inject_stall(ghost_mlp *mlp, int enable);
 /* host copies of the FP32 parameters (set resets Adam's moments) */
 int ghost_mlp_get_params(ghost_mlp *mlp, float *params);
 int ghost_mlp_set_params(ghost_mlp *mlp, const float *params);

@@ -98,6 +98,39 @@ def test_adam_steps_match_oracle():
     assert rel_l2(m.params - p, pm - p) < 2e-2
 
 
+@pytest.mark.parametrize("B", [100, 30000])
+def test_a_training_wait_that_runs_out_leaves_the_weights(B):
+    """With the waits giving up at once (injected, nothing faults), a training
+    step without a loss changes no weight, and get_params, a step with a loss
+    and gradients report GHOST_ERR_TIMEOUT (code 5).  The network then trains
+    on as if the failed steps had not been asked for: the same weights, bit for
+    bit, as one that never saw them."""
+    import torch
+    from ghost_b200 import GhostError
+    from ghost_b200._lib import check
+    x, t = (torch.from_numpy(q).cuda() for q in _data(61, B))
+    m, ref = _mlp(M.glorot(62)), _mlp(M.glorot(62))
+    for q in (m, ref):
+        q.train_step(x, t, 1e-3, want_loss=False)
+
+    def stalled(call):
+        check(m.lib.ghost_mlp_inject_stall(m.h, 1), "ghost_mlp_inject_stall")
+        m.train_step(x, t, 1e-3, want_loss=False)
+        check(m.lib.ghost_mlp_inject_stall(m.h, 0), "ghost_mlp_inject_stall")
+        m.train_step(x, t, 1e-3, want_loss=False)  # before anybody looked: left out too
+        with pytest.raises(GhostError) as err:
+            call()
+        assert err.value.code == 5
+    stalled(lambda: m.params)
+    assert np.array_equal(m.params, ref.params)
+    stalled(lambda: m.train_step(x, t, 1e-3))
+    stalled(lambda: m.gradients(x, t))
+    assert np.array_equal(m.params, ref.params)
+    for q in (m, ref):
+        q.train_step(x, t, 1e-3, want_loss=False)
+    assert np.array_equal(m.params, ref.params)
+
+
 def test_training_reduces_loss():
     import torch
     teacher = M.glorot(41)
