@@ -446,6 +446,13 @@ __global__ void __launch_bounds__(2 * THREADS, 1) mlp_train_kernel(Gmlp g) {
     first = false;
   }
   if (!failed && !first) failed = !mma_done(&s.bar, phase, g.cap, g.status);
+  if (failed) {
+    // [X | H2]^T dY is issued behind the commit that dH2 waits for: tensor
+    // memory is given back only after everything issued has completed (bounded)
+    if (threadIdx.x == 0) mma_commit(&s.bar);
+    gb::mbar_wait(&s.bar, phase, gb::kDrainPolls);
+    tc_fence_after();
+  }
   if (!failed) {
     // accumulator row m = this thread's r: dZ2 or dZ1 index for the first
     // product (slot 0's threads write it), U column UW3 + r for the second
