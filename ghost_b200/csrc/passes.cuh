@@ -62,6 +62,41 @@ struct PipeCtl {
   int stall;      // fault injection: wait on a barrier nothing completes
 };
 
+// The wait of a thread for one load of a ring that a group of warps shares.
+// failed: the group's flag in shared memory.  Once a wait has run out nobody of
+// the group waits, refills a slot or stores any more: a body goes through its
+// remaining lines without loads and drains the ring at its end.  A body keeps
+// alive = alive && ring_wait(...) and counts a slot as read only while alive: a
+// load that never comes kills every warp at it, so its slot is not refilled.
+// (The flag read before each refill, or the slot's last load kept there, cost
+// the 256^3 FP64 X pass 2 %.)  stall: wait on never first.
+__device__ __forceinline__ bool ring_wait(uint64_t *bar, uint32_t parity, uint64_t *never, bool stall, const PipeCtl &ctl,
+                                          volatile int *failed) {
+  if (!stall && mbar_test(bar, parity)) return true;
+  if (!*failed && (!stall || injected_stall_wait(never, ctl.cap)) && mbar_wait(bar, parity, ctl.cap)) return true;
+  record_timeout(ctl.status);
+  *failed = 1;
+  return false;
+}
+// One lane says that its warp has read load L; true if the warp is the last of
+// NW to do so and refills the slot.  cnt[s]: the reads of slot s by now.
+template <int STAGES, int NW> __device__ __forceinline__ bool ring_read(unsigned *cnt, int L) {
+  __threadfence_block();
+  if (NW == 1) cnt[L % STAGES] = (unsigned)(L / STAGES) + 1;
+  else if (atomicAdd(&cnt[L % STAGES], 1u) % NW != NW - 1) return false;
+  __threadfence_block();
+  return true;
+}
+// One thread, once nobody reads any more: waits (bounded) for the loads in
+// flight; issued(L): load L belongs to a tile of this group.
+template <int STAGES, int NW, class F>
+__device__ __forceinline__ void ring_drain(uint64_t *full, const unsigned *cnt, F issued) {
+  for (int s = 0; s < STAGES; ++s) {
+    const int q = (int)(cnt[s] / NW);
+    if (issued(s + STAGES * q)) mbar_wait(&full[s], (uint32_t)q & 1u, kDrainPolls);
+  }
+}
+
 // The exchange buffer of a Z line: two halves HALF values apart, used in turn.
 // Slots keep the lanes of a shared-memory phase on different banks.  FP32 lines
 // of 16 lanes and more (radix 8): a phase is 16 values, the first stage writes

@@ -6,10 +6,12 @@
 // transforms the current one, so the copy engine, not warp occupancy,
 // hides the HBM latency.
 //
-// Every wait is bounded: after `cap` unsuccessful polls the CTA agrees (by
-// __syncthreads_or) to give up, records GHOST_ERR_TIMEOUT in the context's
-// device status word, drains its own copies still in flight (with a fixed
-// generous bound) and returns.
+// Every wait is bounded: after `cap` unsuccessful polls a pass records
+// GHOST_ERR_TIMEOUT in the context's device status word, stores nothing of
+// that tile, drains its own copies still in flight (with a fixed generous
+// bound) and returns.  CTA-wide kernels agree on it by __syncthreads_or;
+// warps that share a ring say so in shared memory (ring_wait in passes.cuh); a
+// warp with a ring of its own just leaves.
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>

@@ -436,6 +436,7 @@ __device__ __forceinline__ void xnl_body(int vb, int nvb, int g, unsigned char *
   const XLine<R, NX, E, BZ> ln(tid, xall, twg);
   uint64_t *full = reinterpret_cast<uint64_t *>(ln.tw3 + G::TW3), *never = full + STAGES;
   unsigned *cnt = reinterpret_cast<unsigned *>(never + 1);
+  volatile int *failed = reinterpret_cast<int *>(cnt + STAGES);  // ring_wait
   auto group_sync = [g] {
     if (NT == 32) __syncwarp();
     else named_sync(1 + g, NT);
@@ -448,6 +449,7 @@ __device__ __forceinline__ void xnl_body(int vb, int nvb, int g, unsigned char *
       mbar_init(&full[q], 1);
       cnt[q] = 0;
     }
+    *failed = 0;
     fence_barrier_init();
   }
   // rows beyond the live ones are zero and stay so: no load reaches them
@@ -477,7 +479,9 @@ __device__ __forceinline__ void xnl_body(int vb, int nvb, int g, unsigned char *
   if (tid == 0)
     for (int L = 0; L < STAGES; ++L) issue(L);
   int nout = 0;
-  // forward line of a product and its way out as output field c
+  bool alive = true;  // no wait of this thread has run out
+  // forward line of a product and its way out as output field c, unless a wait
+  // of the group has run out
   auto emit = [&](C(&P)[E], int tile, int c) {
     ln.template fft<-1>(P);
     unsigned char *ob = obuf + (size_t)(nout & 1) * G::tile;
@@ -485,7 +489,7 @@ __device__ __forceinline__ void xnl_body(int vb, int nvb, int g, unsigned char *
     fence_proxy_async();                  // the tile's generic writes, before the store reads them
     if (tid == 0) bulk_wait_read_all();   // the store before this one has read its buffer
     group_sync();
-    if (tid == 0) {
+    if (tid == 0 && !*failed) {
       for (int q = 0; q < nbox; ++q) {
         const int r0 = min(q * bstep, rows - rb);
         tma_store_3d(&omaps.m[c], ob + (size_t)r0 * RB, (tile % nzb) * BZ * U, (tile / nzb) % ny,
@@ -501,24 +505,13 @@ __device__ __forceinline__ void xnl_body(int vb, int nvb, int g, unsigned char *
     // inverse line of load f of the tile: x[e] = (r_{2m}, r_{2m+1}) at m = t + T e
     auto inverse = [&](int f, C(&x)[E]) {
       const int L = k * NIN + f, s = L % STAGES;
-      // a wait that times out records the status and stays in step with the
-      // ring (no barrier of the group waits on a warp that gave up)
-      const uint32_t par = (uint32_t)(L / STAGES) & 1u;
-      const bool got = (!ctl.stall || L > 0 || injected_stall_wait(never, ctl.cap)) && mbar_wait(&full[s], par, ctl.cap);
-      if (!got) {
-        if (lane == 0) record_timeout(ctl.status);
-        mbar_wait(&full[s], par, kDrainPolls);
-      }
+      // after a wait that ran out the line is computed from whatever the slot
+      // holds and goes nowhere
+      alive = alive && ring_wait(&full[s], (uint32_t)(L / STAGES) & 1u, never, ctl.stall && L == 0, ctl, failed);
       ln.template load_packed<LE>(x, sm + s * G::tile);
       // the last warp to read a slot refills it
       __syncwarp();
-      if (lane == 0) {
-        __threadfence_block();
-        if (NW == 1 || atomicAdd(&cnt[s], 1u) % NW == NW - 1) {
-          __threadfence_block();
-          issue(L + STAGES);
-        }
-      }
+      if (lane == 0 && alive && ring_read<STAGES, NW>(cnt, L)) issue(L + STAGES);
       ln.template fft<+1>(x);
     };
     // Loops where the live registers allow it: nine unrolled lines were 90 KB
@@ -589,7 +582,10 @@ __device__ __forceinline__ void xnl_body(int vb, int nvb, int g, unsigned char *
       }
     }
   }
-  if (tid == 0) bulk_wait_all();
+  if (tid == 0) {
+    if (*failed) ring_drain<STAGES, NW>(full, cnt, [&](int L) { return vb + L / NIN * nvb < ntiles; });
+    bulk_wait_all();
+  }
 }
 
 template <typename R, int NX, int E, int BZ, int PHYS, int LE, int STAGES, int MINB>

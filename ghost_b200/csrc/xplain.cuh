@@ -34,36 +34,35 @@ template <typename R, int NX, int E, int BZ> struct XPlainGeom {
 template <int STAGES, int NW> struct XRing {
   uint64_t *full, *never;
   unsigned *cnt;
+  volatile int *failed;  // ring_wait
   __device__ __forceinline__ XRing(void *at, int tid) {
     full = reinterpret_cast<uint64_t *>(at);
     never = full + STAGES;
     cnt = reinterpret_cast<unsigned *>(never + 1);
+    failed = reinterpret_cast<int *>(cnt + STAGES);
     if (tid == 0) {
       mbar_init(never, 1);
       for (int q = 0; q < STAGES; ++q) {
         mbar_init(&full[q], 1);
         cnt[q] = 0;
       }
+      *failed = 0;
       fence_barrier_init();
     }
   }
-  __device__ __forceinline__ void wait(int L, int lane, const PipeCtl &ctl) const {
-    const uint32_t par = (uint32_t)(L / STAGES) & 1u;
-    uint64_t *bar = &full[L % STAGES];
-    const bool got = (!ctl.stall || L > 0 || injected_stall_wait(never, ctl.cap)) && mbar_wait(bar, par, ctl.cap);
-    if (!got) {
-      if (lane == 0) record_timeout(ctl.status);
-      mbar_wait(bar, par, kDrainPolls);
-    }
+  __device__ __forceinline__ bool wait(int L, const PipeCtl &ctl) const {
+    return ring_wait(&full[L % STAGES], (uint32_t)(L / STAGES) & 1u, never, ctl.stall && L == 0, ctl, failed);
   }
-  // every lane has read the slot of load L; true in one lane of the group, which refills it
-  __device__ __forceinline__ bool read(int L, int lane) const {
+  // every lane has read the slot of load L (alive: as ring_wait asks); true in
+  // one lane of the group, which refills it
+  __device__ __forceinline__ bool read(int L, int lane, bool alive) const {
     __syncwarp();
-    if (lane != 0) return false;
-    __threadfence_block();
-    if (NW > 1 && atomicAdd(&cnt[L % STAGES], 1u) % NW != NW - 1) return false;
-    __threadfence_block();
-    return true;
+    return lane == 0 && alive && ring_read<STAGES, NW>(cnt, L);
+  }
+  // one thread at the end, per loads a tile of a CTA that takes every gridDim.x-th of ntiles
+  __device__ __forceinline__ void drain(int per, int ntiles) const {
+    if (*failed)
+      ring_drain<STAGES, NW>(full, cnt, [&](int L) { return (int)(blockIdx.x + L / per * gridDim.x) < ntiles; });
   }
 };
 
@@ -101,15 +100,16 @@ __global__ void __launch_bounds__(XnlGeom<R, NX, E, BZ, E>::NT)
   dep_wait();
   if (tid == 0)
     for (int k = 0; k < STAGES; ++k) issue(k);
+  bool alive = true;  // no wait of this thread has run out
   for (int k = 0;; ++k) {
     const int tile = blockIdx.x + k * gridDim.x;
     if (tile >= ntiles) break;
-    ring.wait(k, lane, ctl);
+    alive = alive && ring.wait(k, ctl);
     const C *src = reinterpret_cast<const C *>(ibuf + (k % STAGES) * P::line_tile + (size_t)ln.z * P::PITCH) + ln.t;
     C x[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) x[e] = src[T * e];
-    if (ring.read(k, lane)) issue(k + STAGES);
+    if (ring.read(k, lane, alive)) issue(k + STAGES);
     ln.template fft<-1>(x);
 #pragma unroll
     for (int e = 0; e < E; ++e) x[e] = mul2(x[e], both((R)0.5));  // store_unpacked gives twice the spectrum
@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(XnlGeom<R, NX, E, BZ, E>::NT)
     fence_proxy_async();                 // the tile's generic writes, before the store reads them
     if (tid == 0) bulk_wait_read_all();  // the store before this one has read its buffer
     __syncthreads();
-    if (tid == 0) {
+    if (tid == 0 && !*ring.failed) {
       const int ft = tile % nft;
       for (int q = 0; q < nbox; ++q) {
         const int r0 = min(q * bstep, M + 1 - rb);
@@ -127,7 +127,10 @@ __global__ void __launch_bounds__(XnlGeom<R, NX, E, BZ, E>::NT)
       bulk_commit();
     }
   }
-  if (tid == 0) bulk_wait_all();
+  if (tid == 0) {
+    ring.drain(1, ntiles);
+    bulk_wait_all();
+  }
 }
 
 template <typename R, int NX, int E, int BZ, int STAGES>
@@ -162,15 +165,17 @@ __global__ void __launch_bounds__(XnlGeom<R, NX, E, BZ, E>::NT)
   for (int k = 0;; ++k) {
     const int tile = blockIdx.x + k * gridDim.x;
     if (tile >= ntiles) break;
-    ring.wait(k, lane, ctl);
+    if (!__all_sync(0xffffffffu, ring.wait(k, ctl))) break;
     C x[E];
     ln.template load_packed<E>(x, sm + (k % STAGES) * G::tile);
-    if (ring.read(k, lane)) issue(k + STAGES);
+    if (ring.read(k, lane, true)) issue(k + STAGES);
     ln.template fft<+1>(x);
     C *row = reinterpret_cast<C *>(out + (size_t)NX * ((size_t)(tile / nzb) + (size_t)ny * ((tile % nzb) * BZ + ln.z))) + ln.t;
 #pragma unroll
     for (int e = 0; e < E; ++e) row[T * e] = x[e];
   }
+  __syncthreads();
+  if (tid == 0) ring.drain(1, ntiles);
 }
 
 // x[q][3a+b] = (real value / (nx ny nz)) * gs of the nine fields, x[q][9] = delta
@@ -208,16 +213,17 @@ __global__ void __launch_bounds__(XnlGeom<R, NX, E, BZ, E>::NT)
   if (tid == 0)
     for (int L = 0; L < STAGES; ++L) issue(L);
   float *mine = st + ln.z * P::ROWF + 20 * ln.t;
+  bool alive = true;  // no wait of this thread has run out
   for (int k = 0;; ++k) {
     const int tile = blockIdx.x + k * gridDim.x;
     if (tile >= ntiles) break;
 #pragma unroll 1
     for (int f = 0; f < 9; ++f) {
       const int L = 9 * k + f;
-      ring.wait(L, lane, ctl);
+      alive = alive && ring.wait(L, ctl);
       C x[E];
       ln.template load_packed<E>(x, sm + (L % STAGES) * G::tile);
-      if (ring.read(L, lane)) issue(L + STAGES);
+      if (ring.read(L, lane, alive)) issue(L + STAGES);
       ln.template fft<+1>(x);
       if (f == 0) {  // the last tile's rows have left shared memory
         if (tid == 0) bulk_wait_read_all();
@@ -231,14 +237,17 @@ __global__ void __launch_bounds__(XnlGeom<R, NX, E, BZ, E>::NT)
     }
     fence_proxy_async();
     __syncthreads();
-    if (tid == 0) {
+    if (tid == 0 && !*ring.failed) {
       for (int z = 0; z < BZ; ++z)
         bulk_s2g(xrows + (size_t)10 * NX * ((size_t)(tile / nzb) + (size_t)ny * ((tile % nzb) * BZ + z)), st + z * P::ROWF,
                  NX * 40);
       bulk_commit();
     }
   }
-  if (tid == 0) bulk_wait_all();
+  if (tid == 0) {
+    ring.drain(9, ntiles);
+    bulk_wait_all();
+  }
 }
 
 }  // namespace gb

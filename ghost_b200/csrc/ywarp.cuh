@@ -107,6 +107,7 @@ __device__ __forceinline__ void ywarp_body(int vb, int nvb, int g, unsigned char
   // W_N^(b m): FP32 pairs (2j, 2j+1) of m, [j][b]; FP64 [m][b]
   C *tw = reinterpret_cast<C *>(sm + STAGES * G::tile);
   uint64_t *full = reinterpret_cast<uint64_t *>(tw + N), *never = full + STAGES;
+  volatile int *failed = reinterpret_cast<int *>(never + 1);  // ring_wait
   const int tid = threadIdx.x - g * G::NT, lane = tid & 31, wp = tid >> 5;
   auto group_sync = [g] { named_sync(1 + g, G::NT); };
   // the lanes of a shared-memory phase: 8 t of the two lines of a 16-byte
@@ -124,6 +125,7 @@ __device__ __forceinline__ void ywarp_body(int vb, int nvb, int g, unsigned char
   if (tid == 0) {
     mbar_init(never, 1);
     for (int q = 0; q < STAGES; ++q) mbar_init(&full[q], 1);
+    *failed = 0;
     fence_barrier_init();
   }
   for (int q = tid; q < N; q += G::NT) {
@@ -169,6 +171,7 @@ __device__ __forceinline__ void ywarp_body(int vb, int nvb, int g, unsigned char
   dep_wait();
   if (tid == 0)
     for (int k = 0; k < STAGES - 1; ++k) issue(k);
+  int issued = STAGES - 2;  // the last load asked for; it and the one before may be in flight
   // off[c]: byte offset of this lane's column in row (t & 7) ^ c of an 8-row group
   uint32_t off[8];
 #pragma unroll
@@ -183,15 +186,7 @@ __device__ __forceinline__ void ywarp_body(int vb, int nvb, int g, unsigned char
     const int tile = vb + k * nvb;
     if (tile >= ntiles) break;
     const int s = k % STAGES;
-    {
-      // a wait that times out records the status and stays in step
-      const uint32_t par = (uint32_t)(k / STAGES) & 1u;
-      const bool got = (!ctl.stall || k > 0 || injected_stall_wait(never, ctl.cap)) && mbar_wait(&full[s], par, ctl.cap);
-      if (!got) {
-        if (lane == 0) record_timeout(ctl.status);
-        mbar_wait(&full[s], par, kDrainPolls);
-      }
-    }
+    ring_wait(&full[s], (uint32_t)(k / STAGES) & 1u, never, ctl.stall && k == 0, ctl, failed);
     const Tile tl = tile_of(tile);
     int jp = N, jn = 0;
     if (jpos) {
@@ -243,7 +238,7 @@ __device__ __forceinline__ void ywarp_body(int vb, int nvb, int g, unsigned char
     for (int e = 0; e < E; ++e) *reinterpret_cast<C *>(tb + trow + off[0] + (uint32_t)(T * e) * RB) = x[e];
     fence_proxy_async();
     group_sync();
-    if (tid == 0) {
+    if (tid == 0 && !*failed) {
       // rows written: all of them, or (pruned forward pass) boxes covering the
       // live rows; the extra rows of a box hold the transform's own values, in
       // rows nothing reads
@@ -261,9 +256,15 @@ __device__ __forceinline__ void ywarp_body(int vb, int nvb, int g, unsigned char
       // the store of the tile before this one has read its slot: refill it
       asm volatile("cp.async.bulk.wait_group.read 1;\n" ::: "memory");
       issue(k + STAGES - 1);
+      issued = k + STAGES - 1;
     }
   }
-  if (tid == 0) bulk_wait_all();
+  if (tid == 0) {
+    if (*failed)
+      for (int q = max(0, issued - 1); q <= issued && vb + q * nvb < ntiles; ++q)
+        mbar_wait(&full[q % STAGES], (uint32_t)(q / STAGES) & 1u, kDrainPolls);
+    bulk_wait_all();
+  }
 }
 
 template <typename R, int N, int E, int BZ, int S, int MINB>

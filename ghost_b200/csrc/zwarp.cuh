@@ -181,11 +181,11 @@ __device__ __forceinline__ void zwarp_body(int w, int nw, int wc, unsigned char 
   const ZWarpBuf<C> buf{reinterpret_cast<C *>(mine + (size_t)NL * LW * G::PITCH) + (size_t)li * G::PADL, tw};
   uint32_t par = 0;
   for (int g = w; g < ngroups; g += nw) {
-    // a wait that times out records the status and stays in step
     const bool got = (!ctl.stall || g > w || injected_stall_wait(never, ctl.cap)) && mbar_wait(full, par, ctl.cap);
-    if (!got) {
+    if (!__all_sync(0xffffffffu, got)) {
       if (lane == 0) record_timeout(ctl.status);
       mbar_wait(full, par, kDrainPolls);
+      return;
     }
     par ^= 1u;
     const long line = line_of(g, li);

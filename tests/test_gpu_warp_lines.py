@@ -73,3 +73,94 @@ def test_stresses_through_one_x_pass(prec, n):
     F = les.tau_force(to_dev(tau), 0.25)
     ref = les_oracle.tau_force(co, tau.astype(np.float64), 0.25)
     assert rel_l2([to_host(x) for x in F], ref) <= (1e-13 if prec == "fp64" else 2e-6)
+
+
+def _stalled(g, call, kept):
+    """call() with every pass's first wait made to run out: GHOST_ERR_TIMEOUT,
+    and not a bit of the tensors it would have written."""
+    import torch
+    from ghost_b200 import GhostError
+    before = [x.clone() for x in kept]
+    g.set_wait_cap(1000)
+    g.inject_stall(True)
+    with pytest.raises(GhostError) as err:
+        call()
+        g.synchronize()
+    assert err.value.code == 5
+    g.inject_stall(False)
+    g.set_wait_cap(0)
+    assert all(torch.equal(a, b) for a, b in zip(kept, before))
+
+
+# every warp-line kernel and size of its groups (one warp per group: nx = 64, FP64)
+STALL = [("fp32", (64, 64, 64)), ("fp64", (64, 64, 64)), ("fp32", (128, 256, 128)), ("fp64", (128, 256, 128)),
+         ("fp32", (256, 512, 32)), ("fp64", (256, 128, 32)), ("fp32", (1024, 64, 32)), ("fp64", (512, 64, 512)),
+         ("fp32", (512, 1024, 32))]
+
+
+@pytest.mark.parametrize("prec,shape", STALL)
+def test_a_wait_that_runs_out_stores_nothing(prec, shape):
+    """After a bounded wait ran out, a pass leaves its results unwritten: both
+    plain transforms (FP32 512-point x lines, which finish, aside), and steps
+    of the three solvers; afterwards the same calls give the bits of a context
+    that never saw a timeout."""
+    import torch
+    from ghost_b200 import GHOST_COMPLEX_TO_REAL, GHOST_REAL_TO_COMPLEX, Ghost
+    o = Oracle(*shape)
+    g, ref = Ghost(*shape, precision=prec), Ghost(*shape, precision=prec)
+    cd = g.cdtype_np
+    dev = lambda q: [to_dev(x.astype(cd)) for x in q]  # noqa: E731
+    v = dev(o.random_solenoidal(91, 1.0, 6.0, 1, 1.0)[0])
+    a = dev(o.random_solenoidal(92, 1.0, 6.0, 1, 0.3)[0])
+    th = v[2] * 0.1
+    r, s = to_dev(rand_real(o, 93).astype(g.rdtype_np)), to_dev(rand_spectral(o, 94).astype(cd))
+    n = shape
+    calls = []
+    if (prec, shape[0]) != ("fp32", 512):
+        def r2c(h, out):
+            h.fftp3d_real_to_complex(h.fftp3d_create_plan(n, GHOST_REAL_TO_COMPLEX), r, *out)
+
+        def c2r(h, out):
+            h.fftp3d_complex_to_real(h.fftp3d_create_plan(n, GHOST_COMPLEX_TO_REAL), s.clone(), *out)
+        calls += [(r2c, [torch.full_like(g.czeros(), 7.0)]), (c2r, [torch.full_like(g.rzeros(), 7.0)])]
+    calls += [(lambda h, x: h.hd_run(1, 2, 1e-3, 1e-3, *x), v),
+              (lambda h, x: h.bouss_run(1, 2, 2.5e-4, 5e-4, 5e-4, 0.5, 8.0, 8.0, *x), v + [th]),
+              (lambda h, x: h.mhd_run(1, 2, 1e-3, 1e-3, 1e-3, *x), v + a)]
+    for call, start in calls:
+        kept, want = [x.clone() for x in start], [x.clone() for x in start]
+        _stalled(g, lambda: call(g, kept), kept)
+        call(g, kept)
+        call(ref, want)
+        g.synchronize()
+        assert all(torch.equal(p, q) for p, q in zip(kept, want))
+
+
+def test_a_wait_that_runs_out_stores_nothing_in_a_closure_or_an_ensemble():
+    """The same for a step of an LES with the learned closure (the pass that
+    writes its inputs) and for the launches over all classes of an ensemble."""
+    import torch
+    from ghost_b200 import Ensemble, Ghost, GhostError
+    from ghost_b200.les import LES, MLP
+    for prec, n in (("fp32", 64), ("fp64", 64), ("fp32", 128)):
+        g = Ghost(n, precision=prec)
+        v = [g.czeros() for _ in range(3)]
+        g.init_random_solenoidal(95, 1.0, n / 3.0, 1, 1.0, *v)
+        les = LES(g, n // 3)
+        mlp = MLP(0)
+        les.set_model("mlp", mlp, grad_scale=0.1, tau_scale=0.02, delta=1.0)
+        _stalled(g, lambda: les.run(1, 2, 1e-3, 1e-3, *v), v)
+    for prec in ("fp32", "fp64"):
+        e = Ensemble([32, 64, 128], [3, 2, 1], precision=prec)
+        fields = [e.fields(q) for q in range(3)]
+        for q in range(3):
+            for x in fields[q]:
+                x.copy_(torch.randn(x.shape, dtype=x.real.dtype, device="cuda") * 1e-3)
+        torch.cuda.synchronize()
+        before = [[x.clone() for x in f] for f in fields]
+        for q in range(3):
+            e.class_ctx(q).set_wait_cap(1000)
+            e.class_ctx(q).inject_stall(True)
+        with pytest.raises(GhostError) as err:
+            e.run(1, 2, 1e-3)
+        assert err.value.code == 5
+        assert all(torch.equal(x, y) for f, b in zip(fields, before) for x, y in zip(f, b))
