@@ -599,17 +599,14 @@ __global__ void __launch_bounds__(2 * THREADS, 4) mlp_infer2_kernel(Gmlp g) {
 // the same on every run.  21 blocks summing the 148 rows one after the other
 // took 13 us, the loss being one thread's chain of loads.
 // A CTA of the training kernel whose wait ran out leaves its row unwritten, so
-// with the status word set nothing is summed and the weights stay as they are
+// with the status word set the sums go nowhere and the weights stay as they are
 // until the host has seen it; status[1] keeps the first step left out.
 constexpr int ADAM_COLS = 32, ADAM_WARPS = 8;
 __global__ void __launch_bounds__(32 * ADAM_WARPS) adam_kernel(float *P, float *M, float *V, const float *partials,
                                                                int nparts, int step, float lr, float b1, float b2,
                                                                float eps, float *grad_out, double *loss_out,
                                                                int *status) {
-  if (status[0] != 0) {
-    if (blockIdx.x == 0 && threadIdx.x == 0 && step > 0 && status[1] == 0) status[1] = step;
-    return;
-  }
+  const int failed = status[0];  // looked at after the sums
   __shared__ double sh[ADAM_WARPS][ADAM_COLS];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, q = blockIdx.x * ADAM_COLS + lane;
   if (q < NPARAM) {
@@ -622,6 +619,10 @@ __global__ void __launch_bounds__(32 * ADAM_WARPS) adam_kernel(float *P, float *
     sh[w][lane] = a;
   }
   __syncthreads();
+  if (failed != 0) {
+    if (blockIdx.x == 0 && threadIdx.x == 0 && step > 0 && status[1] == 0) status[1] = step;
+    return;
+  }
   if (w != 0 || q > NPARAM) return;
   if (q == NPARAM) {
     double l = 0.0;
@@ -654,7 +655,9 @@ struct ghost_mlp {
   int step = 0;
   int device = 0;
   cudaStream_t stream = nullptr;
-  int *status = nullptr;  // GHOST_ERR_TIMEOUT or 0, and the first training step left out because of it
+  // behind the parameters, so that one copy reads both (get_params: a copy more
+  // was 13 us): GHOST_ERR_TIMEOUT or 0, and the first training step left out
+  int *status = nullptr;
   uint32_t cap = 1u << 22;
   bool stall = false;  // fault injection: waits give up at once
 };
@@ -692,17 +695,21 @@ static bool dev_ptr(const void *p) {
   return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
 }
 
-// Reads and clears the status words (the caller has synchronised).  After a
-// timeout the step count goes back to the last step that was taken.
-static int mlp_check_status(ghost_mlp *m) {
-  int st[2] = {0, 0};
-  MLP_CUDA(cudaMemcpy(st, m->status, sizeof(st), cudaMemcpyDeviceToHost));
+// After a timeout the status words are cleared and the step count goes back to
+// the last step that was taken.
+static int mlp_status(ghost_mlp *m, const int st[2]) {
   if (st[0]) {
-    MLP_CUDA(cudaMemset(m->status, 0, sizeof(st)));
+    MLP_CUDA(cudaMemset(m->status, 0, 2 * sizeof(int)));
     if (st[1] > 0) m->step = st[1] - 1;
     return fail(GHOST_ERR_TIMEOUT, "an MMA completion wait gave up: calls since then gave no result");
   }
   return GHOST_OK;
+}
+// the same, reading the words (the caller has synchronised)
+static int mlp_check_status(ghost_mlp *m) {
+  int st[2] = {0, 0};
+  MLP_CUDA(cudaMemcpy(st, m->status, sizeof(st), cudaMemcpyDeviceToHost));
+  return mlp_status(m, st);
 }
 
 extern "C" {
@@ -715,14 +722,15 @@ int ghost_mlp_create(int seed, ghost_mlp **out) {
   int nsm = 148;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, m->device);
   const size_t pb = sizeof(float) * NPARAM;
-  if (cudaMalloc(&m->P, pb) != cudaSuccess || cudaMalloc(&m->M, pb) != cudaSuccess ||
+  if (cudaMalloc(&m->P, pb + 2 * sizeof(int)) != cudaSuccess || cudaMalloc(&m->M, pb) != cudaSuccess ||
       cudaMalloc(&m->V, pb) != cudaSuccess || cudaMalloc(&m->grad, pb) != cudaSuccess ||
       cudaMalloc(&m->partials, sizeof(float) * (size_t)nsm * (NPARAM + 1)) != cudaSuccess ||
-      cudaMalloc(&m->loss, sizeof(double)) != cudaSuccess || cudaMalloc(&m->status, 2 * sizeof(int)) != cudaSuccess) {
+      cudaMalloc(&m->loss, sizeof(double)) != cudaSuccess) {
     cudaGetLastError();
     ghost_mlp_destroy(m);
     return fail(GHOST_ERR_ALLOC, "MLP buffers");
   }
+  m->status = reinterpret_cast<int *>(m->P + NPARAM);
   // Glorot-uniform weights, zero biases (host RNG, seeded)
   std::vector<float> h(NPARAM, 0.f);
   std::mt19937 rng((uint32_t)seed);
@@ -751,7 +759,6 @@ int ghost_mlp_destroy(ghost_mlp *m) {
   cudaFree(m->grad);
   cudaFree(m->partials);
   cudaFree(m->loss);
-  cudaFree(m->status);
   delete m;
   return GHOST_OK;
 }
@@ -771,9 +778,14 @@ int ghost_mlp_inject_stall(ghost_mlp *m, int enable) {
 int ghost_mlp_get_params(ghost_mlp *m, float *host) {
   if (!m || !host) return fail(GHOST_ERR_ARG, "null argument");
   MLP_CUDA(cudaStreamSynchronize(m->stream));
-  const int st = mlp_check_status(m);
+  struct {
+    float p[NPARAM];
+    int st[2];
+  } got;
+  MLP_CUDA(cudaMemcpy(&got, m->P, sizeof(got), cudaMemcpyDeviceToHost));
+  const int st = mlp_status(m, got.st);
   if (st) return st;
-  MLP_CUDA(cudaMemcpy(host, m->P, sizeof(float) * NPARAM, cudaMemcpyDeviceToHost));
+  memcpy(host, got.p, sizeof(got.p));
   return GHOST_OK;
 }
 
