@@ -96,10 +96,8 @@ int ghost_ctx_set_kmax(ghost_ctx *ctx, double kmax);
  * 1 z-pass CTAs of 128 threads instead of 256; bits 1 and 2 together a
  * two-stage z ring with three CTAs per SM; bits 1, 2 and 5 (z lines of 256
  * points or more) a one-stage z ring with four CTAs per SM.  The other bits
- * are accepted; bit 8 picks the fused x pass of FP32 1024-point lines that is
- * not kept inside a warp, bits 3, 4, 6 and 7 change nothing.  Results do not
- * depend on the variant (0..511).  Default: bits 1, 2 and 5 for z lines of 256
- * points or more. */
+ * are accepted and change nothing.  Results do not depend on the variant
+ * (0..511).  Default: bits 1, 2 and 5 for z lines of 256 points or more. */
 int ghost_ctx_set_tile_cfg(ghost_ctx *ctx, int cfg);
 int ghost_ctx_get_tile_cfg(const ghost_ctx *ctx, int *cfg);
 /* Times one RK step of every tile variant on a copy of v (device arrays;

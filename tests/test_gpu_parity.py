@@ -800,6 +800,29 @@ def test_warp_line_x_pass(prec, shape):
         assert g.maxabs(*[to_dev(x.astype(cd)) for x in v0], kin) == pytest.approx(o.maxabs(*v0, kin), rel=1e-12 if prec == "fp64" else 2e-6)
 
 
+def test_no_tile_variant_changes_the_1024_point_x_pass():
+    """Results do not depend on the tile variant, bit 8 (which once chose
+    another x pass at 1024 FP32 points) included: HD and Boussinesq steps give
+    the same bits, and HD the oracle's result."""
+    import torch
+    shape = (1024, 16, 16)
+    o = Oracle(*shape)
+    g = ghost(*shape, precision="fp32")
+    v0 = o.random_solenoidal(77, 1.0, 5.0, 1, 1.0)[0]
+    th0 = rand_spectral(o, 78, 0.1)
+    out = {}
+    for cfg in (0, 256, 511):
+        g.set_tile_cfg(cfg)
+        V = [to_dev(x.astype(np.complex64)) for x in v0]
+        g.hd_run(2, 2, 1e-3, 2e-3, *V)
+        B = [to_dev(x.astype(np.complex64)) for x in [*v0, th0]]
+        g.bouss_run(2, 2, 2.5e-4, 5e-4, 5e-4, 0.5, 8.0, 8.0, *B)
+        out[cfg] = V + B
+    assert rel_l2([to_host(x) for x in out[256][:3]], o.hd_run(2, 2, 1e-3, 2e-3, v0)) <= 1e-5
+    for cfg in (256, 511):
+        assert all(torch.equal(a, b) for a, b in zip(out[cfg], out[0])), cfg
+
+
 # ------------------------------------------------ rand = 2 forcing update
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])
 def test_forcing_slow_matches_oracle(prec):
