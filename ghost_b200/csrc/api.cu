@@ -1143,6 +1143,7 @@ int ghost_ctx_create(int nx, int ny, int nz, double Lx, double Ly, double Lz, in
   c->nruns = 1;
   c->ntot = c->nspec;
   c->nu_run = nullptr;
+  c->shares_gpu = false;
   c->i0 = 0;
   c->nz_glob = nz;
   // the fastest variants measured for long lines (ghost_hd_autotune
@@ -2901,6 +2902,7 @@ int ghost_ensemble_create(int nclasses, const int *n, const int *nruns, int prec
       break;
     }
     e->cls[q]->stream = e->streams[q];
+    e->cls[q]->shares_gpu = true;
     for (int k = 0; k < 3 && st == GHOST_OK; ++k) {
       st = dalloc(&e->v[q][k], e->cls[q]->cbytes);
       if (st == GHOST_OK && cudaMemset(e->v[q][k], 0, e->cls[q]->cbytes) != cudaSuccess)

@@ -122,6 +122,7 @@ struct ghost_ctx {
   void *nu_run;       // per-run viscosity on the device (precision of ctx), or null
   int tile_cfg;       // tile variant (bit 0: y tile 16 wide, bit 1: z CTAs of 128 threads, bits 1+2: two-stage z ring,
                       // bits 1+2+5: one-stage z ring)
+  bool shares_gpu;    // a class of an ensemble: other classes' streams run beside it (launch_dep)
   int num_sms;
   // device status word written by kernels whose bounded waits ran out
   int *status;

@@ -79,8 +79,9 @@ template <class K> int persistent_grid(ghost_ctx *c, K kern, int threads, size_t
 // FP64 transform pair took 60 us without and 48 us with, a 128^3 FP32 closure
 // step 1697 and 1623.  Large ones are slower for it (256^3 FP64 step: 4055 us
 // without, 4236 with; 128^3 FP64 MHD: 905 and 945), so the attribute is left
-// out above kDepBytes of input, and for the classes of an ensemble, whose
-// streams share the GPU already.
+// out above kDepBytes of input, for batched contexts (256 runs: 5758 and 6377),
+// and for the classes of an ensemble, one-run ones too, whose streams share the
+// GPU already (4 + 2 + 1 runs of 16^3, 32^3, 64^3 FP32: 162 without, 182 with).
 constexpr size_t kDepBytes = (size_t)64 << 20;
 template <class... P, class... A>
 int launch_dep(ghost_ctx *c, int nf, void (*kern)(P...), int grid, int block, size_t smem, A &&...args) {
@@ -93,7 +94,7 @@ int launch_dep(ghost_ctx *c, int nf, void (*kern)(P...), int grid, int block, si
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
-  cfg.numAttrs = c->nruns == 1 && nf * c->cbytes <= kDepBytes ? 1 : 0;
+  cfg.numAttrs = c->nruns == 1 && !c->shares_gpu && nf * c->cbytes <= kDepBytes ? 1 : 0;
   GB_CUDA(cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...));
   return GHOST_OK;
 }
