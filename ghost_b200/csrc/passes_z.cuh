@@ -44,13 +44,20 @@ template <typename R, int N, int NL> constexpr int fit_lines(int want) {
   return lpb;
 }
 
-// whether the one-stage ring with four CTAs per SM is an Op's better one
-// (512^3 FP32: z_fwd 0.649 -> 0.596 ms, z_inv 0.569 -> 0.562; 1024 x 1024 x 256
-// Boussinesq: 2.10 -> 1.91 and 1.77 -> 1.56).  Not for the plain transforms
-// (0.178 -> 0.199 ms at 512^3 FP32) and the FP64 inverse (0.235 -> 0.238 at 256^3).
-template <class Op> struct OneStage { static constexpr bool value = true; };
-template <typename R, int S, int NF> struct OneStage<ZC2C<R, S, NF>> { static constexpr bool value = false; };
-template <int P> struct OneStage<ZInv<double, P>> { static constexpr bool value = false; };
+// whether the one-stage ring with four CTAs per SM is an Op's better one at
+// lines of N points.  us a step with two stages and three CTAs, and with one and
+// four: HD z_fwd FP32 256 x 128 x 512 246 and 218, x 1024 482 and 448, FP64 128 x
+// 128 x 256 123.3 and 120.3, x 512 252.4 and 253.6; Boussinesq z_inv FP32 256 x
+// 128 x 512 315 and 284, x 1024 745 and 696, its z_fwd x 512 339 and 309.  Not for
+// the plain transforms (0.178 and 0.199 ms at 512^3 FP32), the FP64 inverse (0.235
+// and 0.238 at 256^3), and the Boussinesq update where its 128 registers spill
+// four components: FP64 (128 x 128 x 256 176 and 193, x 512 387 and 423) and
+// FP32 at 1024 points (704 and 865).
+template <class Op, int N> struct OneStage { static constexpr bool value = true; };
+template <typename R, int S, int NF, int N> struct OneStage<ZC2C<R, S, NF>, N> { static constexpr bool value = false; };
+template <int P, int N> struct OneStage<ZInv<double, P>, N> { static constexpr bool value = false; };
+template <int N> struct OneStage<ZFwdBouss<double>, N> { static constexpr bool value = false; };
+template <> struct OneStage<ZFwdBouss<float>, 1024> { static constexpr bool value = false; };
 
 // CTAs of NWC warps (zwarp.cuh)
 template <typename R, int N, int E, int NWC, int MINB, class Op>
@@ -93,7 +100,7 @@ template <typename R, int N, class Op> int launch_z_n(ghost_ctx *c, const Op &op
     constexpr int L256 = fit_lines<R, N, Op::NLOAD>(256 / T > 0 ? 256 / T : 1);
     constexpr int L128 = fit_lines<R, N, Op::NLOAD>(128 / T > 0 ? 128 / T : 1);
     if constexpr (N >= 256 && L128 != L256) {
-      if constexpr (OneStage<Op>::value)
+      if constexpr (OneStage<Op, N>::value)
         if ((c->tile_cfg & 38) == 38) return launch_z_cfg<R, N, L128, 1, 4>(c, op, pr);
       if ((c->tile_cfg & 6) == 6) return launch_z_cfg<R, N, L128, 2, 3>(c, op, pr);
     }

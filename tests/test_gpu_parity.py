@@ -800,6 +800,30 @@ def test_warp_line_x_pass(prec, shape):
         assert g.maxabs(*[to_dev(x.astype(cd)) for x in v0], kin) == pytest.approx(o.maxabs(*v0, kin), rel=1e-12 if prec == "fp64" else 2e-6)
 
 
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("nz", [256, 512, 1024])
+def test_bouss_z_rings(prec, nz):
+    """The Boussinesq z passes at the lengths that have several rings (CTA
+    sizes and stages, tile variant bits 1, 2 and 5): the same bits from all,
+    over a full and a zero-pruned step, and the oracle's result."""
+    import torch
+    shape = (16, 16, nz)
+    box = dict(Lx=1, Ly=1, Lz=0.5, arbsize=True)
+    o, g = Oracle(*shape, **box), ghost(*shape, precision=prec, **box)
+    cd = np.complex128 if prec == "fp64" else np.complex64
+    v0, th0 = o.random_solenoidal(79, 1.0, 6.0, 1, 1.0)[0], rand_spectral(o, 80, 0.1)
+    args = (2, 2.5e-4, 5e-4, 5e-4, 0.5, 8.0, 8.0)
+    first = None
+    for cfg in (38, 6, 2, 0):
+        g.set_tile_cfg(cfg)
+        V = [to_dev(x.astype(cd)) for x in [*v0, th0]]
+        g.bouss_run(2, *args, *V)
+        first = first or V
+        assert all(torch.equal(a, b) for a, b in zip(V, first)), cfg
+    rv, rt = o.bouss_run(2, *args, v0, th0)
+    assert rel_l2([to_host(x) for x in first], list(rv) + [rt]) <= (1e-12 if prec == "fp64" else 1e-5)
+
+
 def test_no_tile_variant_changes_the_1024_point_x_pass():
     """Results do not depend on the tile variant, bit 8 (which once chose
     another x pass at 1024 FP32 points) included: HD and Boussinesq steps give
