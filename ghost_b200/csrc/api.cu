@@ -2191,13 +2191,23 @@ int ghost_hd_run(ghost_ctx *c, int nsteps, int ord, double dt, double nu, void *
 // Tile variants tried by the autotuners (bit 0: y tiles 16 z-lines wide;
 // bit 1: z CTAs of 128 threads; bits 1 and 2: two-stage z ring, three CTAs
 // per SM; bits 1, 2 and 5: one-stage z ring, four CTAs per SM, for lines of 256
-// points or more).  Bits 3, 4 and 6 chose y kernels that the warp-line pass has
-// replaced; they are accepted and change nothing.
+// points or more).  The other bits change nothing.
 static const int kTileCfgs[] = {0, 1, 2, 3, 6, 7, 38};
 
-// a variant with bit 5 runs the same kernels as without it on z lines
-// shorter than 256 points: the autotuners skip it there
-static bool tile_cfg_distinct(const ghost_ctx *c, int cfg) { return !(cfg & 32) || c->nz >= 256; }
+// whether a variant of the list runs other kernels in an HD step of this grid
+// than those before it: the autotuners skip the rest
+static bool tile_cfg_distinct(const ghost_ctx *c, int cfg) {
+  const bool sp = c->precision == GHOST_SINGLE;
+  auto kernels = [&](int q) {
+    const bool wide = (q & 1) && (sp ? y_wide_choice<float>(c) : y_wide_choice<double>(c));
+    return 2 * (sp ? hd_z_rings<float>(c, q) : hd_z_rings<double>(c, q)) + wide;
+  };
+  for (int q : kTileCfgs) {
+    if (q == cfg) return true;
+    if (kernels(q) == kernels(cfg)) return false;
+  }
+  return true;
+}
 
 int ghost_ctx_set_tile_cfg(ghost_ctx *c, int cfg) {
   CTX_CHECK(c);

@@ -62,6 +62,10 @@ template <typename R, int S> int launch_y(ghost_ctx *c, const Fields<R> &f, int 
 template <typename R, int KIND>
 int launch_x(ghost_ctx *c, const void *in, void *out, const void *const *ins = nullptr, void *const *outs = nullptr,
              int rows = 0);
+// what a tile variant chooses for an HD step: the z passes' rings, and whether
+// the y passes have a choice (bit 0)
+template <typename R> int hd_z_rings(const ghost_ctx *c, int cfg);
+template <typename R> bool y_wide_choice(const ghost_ctx *c);
 int encode_fn(PFN_cuTensorMapEncodeTiled_v12000 *fn);
 int sm_count(ghost_ctx *c);
 // Persistent grid: as many CTAs as fit on the device at once, or fewer

@@ -49,6 +49,23 @@ int launch_y_cfg(ghost_ctx *c, const Fields<R> &f, int nf, const Prune &pr) {
   return post_launch(c);
 }
 
+// whether lines of N points have a choice of tiles: the 16-wide one needs two
+// stages of 16 lines in shared memory (which leaves out FP64 lines of 512
+// points and more)
+template <typename R, int N> constexpr bool y_has_wide() {
+  constexpr int E = N < 8 ? N : 8, T = N / E;
+  return !y_warp_line<R>(N) && YGeom<R, N, E, (16 * T <= 1024 ? 16 : 1024 / T)>::smem_bytes(2) <= 227 * 1024;
+}
+template <typename R> bool y_wide_choice(const ghost_ctx *c) {
+  switch (c->ny) {
+#define GB_NY(N) \
+  case N: return y_has_wide<R, N>();
+    GB_NY(16) GB_NY(32) GB_NY(64) GB_NY(128) GB_NY(256) GB_NY(512) GB_NY(1024)
+#undef GB_NY
+  }
+  return false;
+}
+
 // tiles 8 z-lines wide, or 16 with tile variant bit 0
 template <typename R, int N, int S> int launch_y_n(ghost_ctx *c, const Fields<R> &f, int nf, const Prune &pr) {
   // lines the warp-line kernel takes, whatever the tile variant (its y bit
@@ -56,12 +73,7 @@ template <typename R, int N, int S> int launch_y_n(ghost_ctx *c, const Fields<R>
   if constexpr (y_warp_line<R>(N)) {
     return launch_ywarp<R, S>(c, f, nf, pr);
   } else {
-    // the 16-wide tile needs two stages of 16 lines in shared memory; where
-    // that does not fit (FP64, long lines) the variant falls back to 8
-    constexpr int E = N < 8 ? N : 8, T = N / E;
-    constexpr int BZ16 = 16 * T <= 1024 ? 16 : 1024 / T;
-    constexpr bool fits16 = YGeom<R, N, E, BZ16>::smem_bytes(2) <= 227 * 1024;
-    if constexpr (fits16) {
+    if constexpr (y_has_wide<R, N>()) {
       if ((c->tile_cfg & 1) && c->nz >= 16) return launch_y_cfg<R, N, S, 16>(c, f, nf, pr);
     }
     return launch_y_cfg<R, N, S, 8>(c, f, nf, pr);
@@ -82,6 +94,7 @@ template <typename R, int S> int launch_y(ghost_ctx *c, const Fields<R> &f, int 
 }
 
 #define GB_INST(R)                                                            \
+  template bool y_wide_choice<R>(const ghost_ctx *);                              \
   template int launch_y<R, +1>(ghost_ctx *, const Fields<R> &, int, const Prune &); \
   template int launch_y<R, -1>(ghost_ctx *, const Fields<R> &, int, const Prune &);
 GB_INST(float)

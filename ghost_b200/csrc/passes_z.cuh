@@ -88,24 +88,36 @@ template <typename R, int N, class Op> int launch_zwarp(ghost_ctx *c, const Op &
   else return launch_zwarp_cfg<R, N, E, 4, MINB>(c, op, pr);
 }
 
-// CTAs of 256 threads; with tile variant bit 1 of 128 threads; with bits 1
-// and 2, for lines of 256 points or more, of 128 threads with a two-stage ring
-// and at most 170 registers, so that three CTAs share an SM; with bit 5 too
-// with a one-stage ring and four CTAs.
+// The CTA-wide pass of an Op at lines of N points, and the tile variant's
+// choice of it.  0: CTAs of 256 threads; 1 (bit 1): of 128 threads; 2 (bits 1
+// and 2, lines of 256 points or more): of 128 threads with a two-stage ring and
+// at most 170 registers, so that three CTAs share an SM; 3 (bit 5 too): a
+// one-stage ring and four CTAs.
+template <typename R, int N, class Op> struct ZRing {
+  static constexpr int T = N / (zE<R>() < N ? zE<R>() : N);
+  static constexpr int L256 = fit_lines<R, N, Op::NLOAD>(256 / T > 0 ? 256 / T : 1);
+  static constexpr int L128 = fit_lines<R, N, Op::NLOAD>(128 / T > 0 ? 128 / T : 1);
+  static constexpr bool sizes = !z_warp_line<R, Op>(N) && L128 != L256, stages = sizes && N >= 256;
+  static constexpr bool one = stages && OneStage<Op, N>::value;
+  static int of(int cfg) {
+    if (one && (cfg & 38) == 38) return 3;
+    if (stages && (cfg & 6) == 6) return 2;
+    return sizes && (cfg & 2) ? 1 : 0;
+  }
+};
 template <typename R, int N, class Op> int launch_z_n(ghost_ctx *c, const Op &op, const Prune &pr) {
   if constexpr (z_warp_line<R, Op>(N)) {
     return launch_zwarp<R, N>(c, op, pr);
   } else {
-    constexpr int E = zE<R>() < N ? zE<R>() : N, T = N / E;
-    constexpr int L256 = fit_lines<R, N, Op::NLOAD>(256 / T > 0 ? 256 / T : 1);
-    constexpr int L128 = fit_lines<R, N, Op::NLOAD>(128 / T > 0 ? 128 / T : 1);
-    if constexpr (N >= 256 && L128 != L256) {
-      if constexpr (OneStage<Op, N>::value)
-        if ((c->tile_cfg & 38) == 38) return launch_z_cfg<R, N, L128, 1, 4>(c, op, pr);
-      if ((c->tile_cfg & 6) == 6) return launch_z_cfg<R, N, L128, 2, 3>(c, op, pr);
-    }
-    if ((c->tile_cfg & 2) && L128 != L256) return launch_z_cfg<R, N, L128, 3, 1>(c, op, pr);
-    return launch_z_cfg<R, N, L256, 3, 1>(c, op, pr);
+    using Z = ZRing<R, N, Op>;
+    const int ring = Z::of(c->tile_cfg);
+    if constexpr (Z::one)
+      if (ring == 3) return launch_z_cfg<R, N, Z::L128, 1, 4>(c, op, pr);
+    if constexpr (Z::stages)
+      if (ring == 2) return launch_z_cfg<R, N, Z::L128, 2, 3>(c, op, pr);
+    if constexpr (Z::sizes)
+      if (ring == 1) return launch_z_cfg<R, N, Z::L128, 3, 1>(c, op, pr);
+    return launch_z_cfg<R, N, Z::L256, 3, 1>(c, op, pr);
   }
 }
 
@@ -122,7 +134,19 @@ template <typename R, class Op> int launch_z(ghost_ctx *c, const Op &op, const P
   return fail(GHOST_ERR_SIZE, "nz=%d unsupported", c->nz);
 }
 
+// the rings of an HD step's two z passes with a tile variant
+template <typename R> int hd_z_rings(const ghost_ctx *c, int cfg) {
+  switch (c->nz) {
+#define GB_NZ(N) \
+  case N: return ZRing<R, N, ZInv<R, 0>>::of(cfg) + 4 * ZRing<R, N, ZFwdHD<R>>::of(cfg);
+    GB_NZ(16) GB_NZ(32) GB_NZ(64) GB_NZ(128) GB_NZ(256) GB_NZ(512) GB_NZ(1024)
+#undef GB_NZ
+  }
+  return 0;
+}
+
 #define GB_INST(R)                                                                    \
+  template int hd_z_rings<R>(const ghost_ctx *, int);                                 \
   template int launch_z<R, ZInv<R, 0>>(ghost_ctx *, const ZInv<R, 0> &, const Prune &);   \
   template int launch_z<R, ZInv<R, 1>>(ghost_ctx *, const ZInv<R, 1> &, const Prune &);   \
   template int launch_z<R, ZGrad<R>>(ghost_ctx *, const ZGrad<R> &, const Prune &);       \

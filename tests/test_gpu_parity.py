@@ -800,6 +800,22 @@ def test_warp_line_x_pass(prec, shape):
         assert g.maxabs(*[to_dev(x.astype(cd)) for x in v0], kin) == pytest.approx(o.maxabs(*v0, kin), rel=1e-12 if prec == "fp64" else 2e-6)
 
 
+@pytest.mark.parametrize("prec,shape,variants", [
+    ("fp32", (32, 64, 128), 1), ("fp64", (32, 128, 64), 1),     # every line inside a warp: nothing to choose
+    ("fp32", (32, 16, 128), 2), ("fp64", (16, 32, 64), 2),      # y tiles of 8 or 16 z-lines
+    ("fp32", (32, 64, 16), 2), ("fp32", (16, 16, 16), 4),       # z CTAs of 256 or 128 threads
+    ("fp32", (16, 64, 256), 4), ("fp64", (16, 64, 256), 4),     # and rings of three, two and one stages
+    ("fp32", (16, 16, 512), 7), ("fp64", (16, 64, 1024), 1)])
+def test_autotuner_times_each_choice_once(prec, shape, variants):
+    """The autotuner times three one-substep steps (five passes each) of every
+    tile variant that runs other kernels on this grid, and of no other."""
+    g = ghost(*shape, precision=prec)
+    v = [g.czeros() for _ in range(3)]
+    n0 = g.launch_count()
+    g.hd_autotune(1, 1e-3, 1e-3, *v)
+    assert g.launch_count() - n0 == 3 * 5 * variants
+
+
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])
 @pytest.mark.parametrize("nz", [256, 512, 1024])
 def test_bouss_z_rings(prec, nz):
