@@ -110,7 +110,7 @@ PipeCtl pipe_ctl(ghost_ctx *c);
 // the fused X pass with lines kept inside a warp (xnl.cuh): whether it
 // takes this grid, and its launch (ins: v, curl v (, grad theta); rows: live
 // kx rows, 0 for all)
-bool xnl_takes(const ghost_ctx *c);
+bool xnl_takes(ghost_ctx *c);
 int launch_xnl(ghost_ctx *c, bool bouss, const void *const *ins, void *const *outs, int rows);
 // plain x transforms with lines kept inside a warp (xplain.cuh): whether they
 // take this grid, and their launches

@@ -118,20 +118,13 @@ template <typename R, int NX, int KIND> int launch_x_n(ghost_ctx *c, const void 
     constexpr int YB = x_yb<R, NX, BZ>();
     GB_CHECK((launch_x_fused<R, NX, KIND, BZ, (YB * NT <= 128 ? 2 : 1)>(c, ins, outs, rows)));
   } else if constexpr (KIND == X_HD || KIND == X_BOUSS) {
-    // lines of 64 points and more: the warp-line kernel (xnl.cuh) where it
-    // takes the grid.  Left to the other kernel: shorter lines, FP64 at
-    // nx = 1024, and at FP32 below 1024 a z-slab of 8 planes more than a
-    // multiple of 16 (slabs are multiples of 8).
-    constexpr bool kBoth = sizeof(R) == 4 ? NX < 1024 : NX < 64 || NX == 1024;
-    if constexpr (NX >= 64) {
-      if (!kBoth || xnl_takes(c)) {
-        GB_CHECK(launch_xnl(c, KIND == X_BOUSS, ins, outs, rows));
-        timer_end(c, ts);
-        return post_launch(c);
-      }
+    // the warp-line kernel (xnl.cuh) where it takes the grid
+    if (xnl_takes(c)) {
+      GB_CHECK(launch_xnl(c, KIND == X_BOUSS, ins, outs, rows));
+      timer_end(c, ts);
+      return post_launch(c);
     }
-    if constexpr (kBoth)
-      GB_CHECK((launch_x_fused<R, NX, KIND, BZ, 2>(c, ins, outs, rows)));
+    GB_CHECK((launch_x_fused<R, NX, KIND, BZ, 2>(c, ins, outs, rows)));
   } else if (KIND == X_C2R && xw_plain_ok(c)) {
     GB_CHECK(launch_xw_c2r(c, in, out));
   } else if (KIND == X_R2C && xw_plain_ok(c)) {

@@ -43,9 +43,21 @@ static int pick(ghost_ctx *c, bool bouss, const void *const *ins, void *const *o
 // Lines of 64 points and more (shorter ones leave a warp's lines nothing to
 // exchange with); FP64 up to 512 (a 1024-point line would be 64 lanes).  The
 // tiles must divide nz, which only a rank's z-slab of a decomposed run can fail.
-bool xnl_takes(const ghost_ctx *c) {
-  if (c->precision == GHOST_SINGLE) return c->nx >= 64 && c->nz % (c->nx == 1024 ? 8 : 16) == 0;
-  return c->nx >= 64 && c->nx <= 512 && c->nz % 8 == 0;
+// Where a lane holds twice the values that a thread of the CTA-wide kernel
+// does (FP64, and FP32 from 256 points on), its chains are twice as long, and a
+// grid that gives a multiprocessor four warps or fewer is faster CTA-wide: us of
+// X a Boussinesq step, CTA-wide and here, FP64 64 x 64 x 32 (256 warps) 33.7 and
+// 39.8, 256 x 64 x 16 (512) 42.3 and 48.9, x 32 (1024) 72.4 and 56.5; FP32 1024 x
+// 16 x 16 (256) 58 and 69, 256 x 64 x 64 (1024) 74 and 50.  The classes of an
+// ensemble share the GPU, and their one launch a pass has this body only.
+bool xnl_takes(ghost_ctx *c) {
+  const bool sp = c->precision == GHOST_SINGLE;
+  const int bz = sp && c->nx < 1024 ? 16 : 8;
+  if (c->nx < 64 || c->nz % bz != 0 || (!sp && c->nx == 1024)) return false;
+  if (c->shares_gpu || (sp && c->nx < 256)) return true;
+  // warps of a tile: FP32 256 and FP64 as many as 64-point half lines fit, 8 above
+  const int nw = c->nx >= 512 ? 8 : c->nx / 64;
+  return (long)(c->nz / bz) * c->ny * c->nruns * nw > 4L * sm_count(c);
 }
 
 int launch_xnl(ghost_ctx *c, bool bouss, const void *const *ins, void *const *outs, int rows) {

@@ -774,10 +774,12 @@ def test_bouss_fp32_with_512_point_x_lines(shape):
 
 
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])
-@pytest.mark.parametrize("shape", [(64, 16, 16), (128, 16, 32), (256, 32, 16), (1024, 16, 32), (64, 256, 64)])
+@pytest.mark.parametrize("shape", [(64, 16, 16), (128, 16, 32), (256, 32, 16), (1024, 16, 32), (64, 256, 64),
+                                   (128, 64, 64), (256, 64, 64), (512, 64, 32), (1024, 16, 64)])
 def test_warp_line_x_pass(prec, shape):
-    """The fused X pass at every line length it keeps inside a warp, HD and
-    Boussinesq, one and several tiles per y, full (first substep, modes outside
+    """The fused X pass at every line length it keeps inside a warp, on grids
+    of few tiles (FP64, and FP32 from 256 points on, then run CTA-wide) and of
+    many, HD and Boussinesq, one and several tiles per y, full (first substep, modes outside
     the truncation) and zero-pruned substeps: two steps against the oracle."""
     box = dict(Lx=1, Ly=1, Lz=0.5, arbsize=True)
     o, ob = Oracle(*shape), Oracle(*shape, **box)

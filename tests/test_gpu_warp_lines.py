@@ -93,7 +93,7 @@ def _stalled(g, call, kept):
 
 
 # every warp-line kernel and size of its groups (one warp per group: nx = 64, FP64)
-STALL = [("fp32", (64, 64, 64)), ("fp64", (64, 64, 64)), ("fp32", (128, 256, 128)), ("fp64", (128, 256, 128)),
+STALL = [("fp32", (64, 64, 64)), ("fp64", (64, 128, 64)), ("fp32", (128, 256, 128)), ("fp64", (128, 256, 128)),
          ("fp32", (256, 512, 32)), ("fp64", (256, 128, 32)), ("fp32", (1024, 64, 32)), ("fp64", (512, 64, 512)),
          ("fp32", (512, 1024, 32))]
 
