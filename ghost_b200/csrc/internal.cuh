@@ -86,6 +86,9 @@ template <class K> int persistent_grid(ghost_ctx *c, K kern, int threads, size_t
 // out above kDepBytes of input, for batched contexts (256 runs: 5758 and 6377),
 // and for the classes of an ensemble, one-run ones too, whose streams share the
 // GPU already (4 + 2 + 1 runs of 16^3, 32^3, 64^3 FP32: 162 without, 182 with).
+// Neither do the passes over several fields gain with 16-point y lines, whose
+// CTAs hold eight kx each: 256 x 16 x 64 FP32 HD 89 without and 99 with, 1024 x 16 x
+// 16 FP64 118 and 134 (with 32 points, 1024 x 32 x 16 FP64: 160 and 145).
 constexpr size_t kDepBytes = (size_t)64 << 20;
 template <class... P, class... A>
 int launch_dep(ghost_ctx *c, int nf, void (*kern)(P...), int grid, int block, size_t smem, A &&...args) {
@@ -98,7 +101,7 @@ int launch_dep(ghost_ctx *c, int nf, void (*kern)(P...), int grid, int block, si
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
-  cfg.numAttrs = c->nruns == 1 && !c->shares_gpu && nf * c->cbytes <= kDepBytes ? 1 : 0;
+  cfg.numAttrs = c->nruns == 1 && !c->shares_gpu && (c->ny > 16 || nf == 1) && nf * c->cbytes <= kDepBytes ? 1 : 0;
   GB_CUDA(cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...));
   return GHOST_OK;
 }
