@@ -90,6 +90,7 @@ template <class K> int persistent_grid(ghost_ctx *c, K kern, int threads, size_t
 // CTAs hold eight kx each: 256 x 16 x 64 FP32 HD 89 without and 99 with, 1024 x 16 x
 // 16 FP64 118 and 134 (with 32 points, 1024 x 32 x 16 FP64: 160 and 145).
 constexpr size_t kDepBytes = (size_t)64 << 20;
+constexpr int kAlone = 1 << 20;  // as nf: a pass that starts when the one before it has ended
 template <class... P, class... A>
 int launch_dep(ghost_ctx *c, int nf, void (*kern)(P...), int grid, int block, size_t smem, A &&...args) {
   cudaLaunchConfig_t cfg = {};

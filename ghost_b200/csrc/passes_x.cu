@@ -46,7 +46,11 @@ int launch_x_fused(ghost_ctx *c, const void *const *ins, void *const *outs, int 
   FieldMaps maps;
   for (int q = 0; q < NIN; ++q) GB_CHECK(field_map(c, ins[q], BZ * U, YB, rb, &maps.m[q]));
   const int pgrid = persistent_grid(c, kern, NT, smem, (long)(c->nz / BZ) * (c->ny / YB) * nruns);
-  GB_CHECK(launch_dep(c, NIN, kern, pgrid, NT, smem, maps, fo, (const C *)c->tw_x, c->ny, c->nz, (R)1 / (nn * nn), nrows,
+  // A step's pass with fewer CTAs than multiprocessors is slower started early
+  // (us a step, early and not, 256 x 32 x 16 FP32 Boussinesq 150 and 142, 512 x 32 x
+  // 16 FP64 HD 106 and 93; 64^3 FP64 HD, 256 CTAs, 81 and 87).
+  const bool alone = NX >= 64 && (KIND == X_HD || KIND == X_BOUSS) && pgrid < sm_count(c);
+  GB_CHECK(launch_dep(c, alone ? kAlone : NIN, kern, pgrid, NT, smem, maps, fo, (const C *)c->tw_x, c->ny, c->nz, (R)1 / (nn * nn), nrows,
                       nbox, rb, nruns, c->nxh, pipe_ctl(c)));
   return GHOST_OK;
 }
