@@ -296,7 +296,7 @@ struct Gmlp {
 // Loss and gradients of one batch, two tiles of 128 rows per CTA and round
 // (warps 0-3 take slot 0, warps 4-7 slot 1; round k, slot u of CTA b takes
 // tile (2k + u) gridDim.x + b, so a batch of few tiles gives each CTA one).
-// Bound by latency: five dependent MMA + epilogue phases a round, 24 kFLOP a
+// Bound by latency: five dependent MMA + epilogue phases a round, 29 kFLOP a
 // row.  With the weight gradients on the tensor cores a training step of
 // 65536 rows (two rounds, and the Adam kernel) takes 37 us; with them summed
 // row by row on the CUDA cores, one tile at a time and gelu' kept in shared

@@ -20,8 +20,9 @@
 // mirror Z_{M-k} of the real-to-complex unpacking by shuffles, (d) adds in
 // packed FP32, and (e) sends the results out by TMA from a staging tile; the
 // CTA meets at three or four barriers a tile. ms a launch, by lines of a CTA with
-// radix-8 (FP64: radix-4) stages and by this kernel: 512^3 FP32 1.48 and 1.28,
-// 1024 x 1024 x 256 Boussinesq FP32 6.60 and 5.67, 256^3 FP64 0.515 and 0.435.
+// radix-8 (FP64: radix-4) stages and by this kernel: 512^3 FP32 1.48 and 1.22,
+// 1024 x 1024 x 256 Boussinesq FP32 6.60 and 4.95, 256^3 FP64 0.515 and 0.430.
+// Small grids stay with the lines of a CTA (xnl_takes, xnl.cu).
 #pragma once
 #include "f32x2.cuh"
 #include "passes.cuh"

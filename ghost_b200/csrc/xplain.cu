@@ -67,6 +67,8 @@ static int features(ghost_ctx *c, const void *const *spec, float *x, float gs, f
   FieldMaps maps;
   for (int q = 0; q < 9; ++q) GB_CHECK(field_map(c, spec[q], BZ * G::ES / 8, 1, bx.rb, &maps.m[q], swizzle_of(G::RB)));
   const int grid = persistent_grid(c, kern, G::NT, smem, (long)(c->nz / BZ) * c->ny);
+  // nine fields, but started early as three would be (launch_dep): with nine a
+  // closure step (RK2) of 128^3 FP32 took 773 us instead of 771, FP64 1245 instead of 1236
   GB_CHECK(launch_dep(c, 3, kern, grid, G::NT, smem, maps, x, (const cx<R> *)c->tw_x, c->ny, c->nz, bx.nbox, bx.rb, (R)(1.0 / (double)c->nreal), gs, delta, pipe_ctl(c)));
   return GHOST_OK;
 }

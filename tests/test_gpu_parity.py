@@ -485,8 +485,9 @@ def test_ensemble_graph_steps_match_oracle(prec):
 
 @pytest.mark.parametrize("prec", ["fp32", "fp64"])
 def test_tile_variants_are_bitwise_identical(prec):
-    """Every tile variant (y tile width, z CTA size, two-stage z ring) gives
-    the same bits, and the autotuner leaves the velocity untouched."""
+    """256^3: the z rings of the tile variant (bits 1, 2 and 5) give the same
+    bits, the other bits are accepted and change nothing (x and y lines stay
+    inside a warp), and the autotuner leaves the velocity untouched."""
     import torch
     n = 256
     g = ghost(n, precision=prec)
@@ -509,10 +510,36 @@ def test_tile_variants_are_bitwise_identical(prec):
             assert all(torch.equal(a, b) for a, b in zip(V, ref)), c
 
 
+@pytest.mark.parametrize("prec,shape", [
+    ("fp32", (32, 16, 128)), ("fp64", (16, 32, 64)),    # y tiles of 8 or 16 z-lines
+    ("fp32", (16, 16, 16)), ("fp64", (16, 16, 16)),     # and z CTAs of 256 or 128 threads
+    ("fp32", (16, 64, 256)), ("fp64", (16, 64, 256)),   # and rings of three, two and one stages
+    ("fp32", (16, 16, 512)), ("fp64", (16, 16, 512)), ("fp32", (16, 32, 1024))])
+def test_tile_variants_that_choose_kernels(prec, shape):
+    """The grids on which the variant picks other kernels: the same bits from
+    every one of them and from the bits that are accepted only, over a full and
+    a zero-pruned step, and the oracle's result."""
+    import torch
+    o = Oracle(*shape)
+    g = ghost(*shape, precision=prec)
+    cd = g.cdtype_np
+    v0 = o.random_solenoidal(53, 1.0, 6.0, 1, 1.0)[0]
+    f = o.random_solenoidal(54, 2.0, 3.0, 0, 1.0)[0]
+    F = [to_dev(x.astype(cd)) for x in f]
+    first = None
+    for cfg in (0, 1, 2, 3, 6, 7, 38, 39, 8, 16, 64, 128, 511):
+        g.set_tile_cfg(cfg)
+        V = [to_dev(x.astype(cd)) for x in v0]
+        g.hd_run(2, 2, 5e-4, 1e-3, *V, *F)
+        first = first or V
+        assert all(torch.equal(a, b) for a, b in zip(V, first)), cfg
+    assert rel_l2([to_host(x) for x in first], o.hd_run(2, 2, 5e-4, 1e-3, v0, f)) <= (1e-12 if prec == "fp64" else 1e-5)
+
+
 def test_wide_line_variants_at_512():
-    """The FP32 y passes with 16 values per thread (bit 4), alone and with the
-    other variants, give the same bits as the 8-value passes over unpruned
-    and pruned substeps, and match the oracle."""
+    """FP32 with 512 z points: the two-stage z ring (bits 1 and 2, in variants
+    14 and 30) gives the bits of the three-stage one over unpruned and pruned
+    substeps; bits 3 and 4 are accepted and change nothing; the oracle's result."""
     import torch
     shape = (64, 256, 512)
     o = Oracle(*shape)
@@ -707,15 +734,12 @@ def test_phaseshift(prec, shape):
 
 
 # ------------------------------------------- the benchmark's 512-point lines
-# Shapes whose lines along one axis (or two) have 512 points run the same
-# kernel instantiations as the 512^3 benchmark step: xpipe_nl_kernel<*, 512,
-# ...> for nx = 512, ypipe_kernel<*, 512, ...> for ny = 512 and
-# zpipe_kernel<*, 512, ...> for nz = 512.  Tile variants 30, 62 and 126 are
-# the FP32 benchmark's (y passes with 16 values per thread and a second
-# exchange buffer; a two-stage z ring with three CTAs per SM, or a one-stage
-# z ring with four; 126 also runs the y inverse in 4-line tiles); FP64 runs
-# the variants the autotuner picks at 512^3 (22, 6), the one-stage z ring
-# (38) and the default.
+# Shapes whose lines along one axis (or two) have 512 points.  They run the
+# z kernels of the 512^3 benchmark step (zpipe_kernel<float, 512, ...> with its
+# rings: two stages with variants 6, 22 and 30, one with 38, 62 and 126;
+# zwarp_kernel<double, 512, ...>) and its FP32 y kernel (ywarp_kernel<float,
+# 512, ...>; FP64: ypipe_kernel).  512-point x lines run its xnl_kernel on the
+# last shape only: the other two have too few tiles and run CTA-wide.
 LINE512 = [(512, 16, 16), (16, 512, 16), (16, 16, 512), (512, 512, 16)]
 
 
@@ -749,9 +773,8 @@ def test_forced_rk4_with_512_point_lines(shape, prec, cfgs, tol):
 
 @pytest.mark.parametrize("shape", [(512, 16, 16), (512, 32, 32)])
 def test_bouss_fp32_with_512_point_x_lines(shape):
-    """The Boussinesq substep's FP32 x pass at 512-point lines (16-line tiles,
-    work fields in the x-pass layout) against the FP64 oracle; tile variants
-    give the same bits."""
+    """The Boussinesq substep at FP32 512-point x lines, CTA-wide on these few
+    tiles, against the FP64 oracle; tile variants give the same bits."""
     import torch
     o = Oracle(*shape, Lx=1, Ly=1, Lz=0.25, arbsize=True)
     v0, _ = o.random_solenoidal(57, 1.0, 40.0, 1, 1.0)

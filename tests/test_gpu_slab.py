@@ -20,8 +20,13 @@ def _fields(g, seed):
 @pytest.mark.parametrize("overlap", [True, False])
 @pytest.mark.parametrize("prec,P,shape", [("fp64", 1, (64, 64, 64)), ("fp64", 2, (64, 64, 64)),
                                           ("fp64", 4, (64, 64, 64)), ("fp32", 2, (64, 64, 64)),
-                                          ("fp64", 4, (64, 32, 128))])
+                                          ("fp64", 4, (64, 32, 128)), ("fp32", 8, (64, 64, 64)),
+                                          ("fp32", 2, (256, 16, 16)), ("fp32", 4, (128, 128, 32)),
+                                          ("fp32", 2, (512, 16, 16)), ("fp32", 2, (1024, 16, 16))])
 def test_slab_run_matches_undivided_run(prec, P, shape, overlap):
+    """FP32 slabs of 8 planes included: at 64 to 512 x points they run the
+    CTA-wide X pass, where the undivided run's planes are enough for the
+    warp-line one."""
     import torch
 
     from ghost_b200 import Ghost
