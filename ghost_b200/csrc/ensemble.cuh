@@ -173,7 +173,10 @@ template <typename R> constexpr int ens_warp_BZ() { return sizeof(R) == 4 ? 16 :
 template <typename R, int NX> struct EnsWarp {
   template <int LE> using G = XnlGeom<R, NX, 8, ens_warp_BZ<R>(), LE>;
   static constexpr int NT = G<8>::NT, groups = kEnsThreads / NT;
-  static constexpr size_t group = (G<8>::fixed + kEnsXStages * G<8>::tile + 1023) / 1024 * 1024;
+  // FP64 groups with four stages left one CTA of four warps on an SM (64 runs of
+  // 64^3: 2.12 ms a step; with two stages, two CTAs, 1.71)
+  static constexpr int STAGES = sizeof(R) == 4 ? kEnsXStages : 2;
+  static constexpr size_t group = (G<8>::fixed + STAGES * G<8>::tile + 1023) / 1024 * 1024;
   static_assert(groups * NT == kEnsThreads, "one CTA size for all classes");
 };
 template <typename R, int NX> constexpr size_t ens_x_smem() {
@@ -192,10 +195,10 @@ template <typename R, int NX> __device__ __forceinline__ void ens_x_run(const XC
     nvb *= W::groups;
     constexpr int BZ = ens_warp_BZ<R>();
     if (k.rows <= 6 * W::template G<6>::T)
-      xnl_body<R, NX, 8, BZ, 0, 6, kEnsXStages>(vb, nvb, g, sm, k.maps, k.maps, k.tw, k.ny, k.nz, k.scale, k.rows, k.nbox,
+      xnl_body<R, NX, 8, BZ, 0, 6, W::STAGES>(vb, nvb, g, sm, k.maps, k.maps, k.tw, k.ny, k.nz, k.scale, k.rows, k.nbox,
                                                 k.rb, k.nruns, k.nxh, k.ctl);
     else
-      xnl_body<R, NX, 8, BZ, 0, 8, kEnsXStages>(vb, nvb, g, sm, k.maps, k.maps, k.tw, k.ny, k.nz, k.scale, k.rows, k.nbox,
+      xnl_body<R, NX, 8, BZ, 0, 8, W::STAGES>(vb, nvb, g, sm, k.maps, k.maps, k.tw, k.ny, k.nz, k.scale, k.rows, k.nbox,
                                                 k.rb, k.nruns, k.nxh, k.ctl);
   } else {
     xpipe_nl_body<R, NX, ens_x_E<R, NX>(), ens_xBZ<R>(), 0, kEnsXStages, ens_x_yb<R, NX>()>(
