@@ -2560,15 +2560,20 @@ static int ensemble_class_step(ghost_ensemble *e, int q, int ord, double dt, boo
 
 // ---- one launch per pass over all classes (ensemble.cuh)
 // Persistent CTAs of a multi-class launch: per_sm CTAs on each SM; the SM
-// slots are shared among the classes in proportion to their tiles (each
-// class gets at least one).  Returns the grid, per_sm times the SM count.
-template <class P> static int ens_split(ghost_ctx *c0, int per_sm, const long *tiles, P &p) {
+// slots are shared among the classes in proportion to their work, each class
+// getting at least one: the pass's complex values (tiles of the bodies differ
+// in size), and 8/5 of them for lines below 64 points, whose bodies take that
+// much longer a value.  s for 100 steps with factors 1, 8/5 and 2: 128 + 96 + 32
+// runs of 32^3, 64^3, 128^3 FP64 1.16, 1.07, 1.04, FP32 0.63, 0.56, 0.56; 200 + 4
+// of 16^3 and 128^3 FP32 0.099, 0.081, 0.077; 30 + 6 of 32^3 and 64^3 FP32 0.0208,
+// 0.0222, 0.0244.  Returns the grid, per_sm times the SM count.
+template <class P> static int ens_split(ghost_ctx *c0, int per_sm, const long *values, P &p) {
   const int nsm = sm_count(c0), nc = p.ncls;
-  long tot = 0;
-  for (int q = 0; q < nc; ++q) tot += tiles[q];
+  long work[kEnsMaxCls], tot = 0;
+  for (int q = 0; q < nc; ++q) tot += work[q] = values[q] * (p.n[q] < 64 ? 8 : 5);
   int sum = 0;
   for (int q = 0; q < nc; ++q) {
-    p.nb[q] = std::max(1, (int)((double)nsm * (double)tiles[q] / (double)std::max<long>(1, tot)));
+    p.nb[q] = std::max(1, (int)((double)nsm * (double)work[q] / (double)std::max<long>(1, tot)));
     sum += p.nb[q];
   }
   while (sum > nsm) {  // take slots from the class with the most
@@ -2578,10 +2583,10 @@ template <class P> static int ens_split(ghost_ctx *c0, int per_sm, const long *t
     --p.nb[m];
     --sum;
   }
-  while (sum < nsm) {  // give slots to the class with the most tiles per slot
+  while (sum < nsm) {  // give slots to the class with the most work per slot
     int m = 0;
     for (int q = 1; q < nc; ++q)
-      if ((double)tiles[q] / p.nb[q] > (double)tiles[m] / p.nb[m]) m = q;
+      if ((double)work[q] / p.nb[q] > (double)work[m] / p.nb[m]) m = q;
     ++p.nb[m];
     ++sum;
   }
@@ -2595,10 +2600,8 @@ template <class P> static int ens_split(ghost_ctx *c0, int per_sm, const long *t
   return p.per * nsm;
 }
 
-template <typename R> static int ens_T(int N, int E) { return N / (E < N ? E : N); }
-
 template <typename R, class Op>
-static int ens_launch_z(ghost_ensemble *e, ZMulti<R, Op> &P, const long *tiles) {
+static int ens_launch_z(ghost_ensemble *e, ZMulti<R, Op> &P, const long *values) {
   size_t smem = 0;
   for (int q = 0; q < P.ncls; ++q) {
     switch (P.n[q]) {
@@ -2613,12 +2616,12 @@ static int ens_launch_z(ghost_ensemble *e, ZMulti<R, Op> &P, const long *tiles) 
   GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int per = 0;
   GB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, kEnsThreads, smem));
-  const int grid = ens_split(e->cls[0], per, tiles, P);
+  const int grid = ens_split(e->cls[0], per, values, P);
   kern<<<grid, kEnsThreads, smem, e->main>>>(P);
   return post_launch(e->cls[0]);
 }
 
-template <typename R, int S> static int ens_launch_y(ghost_ensemble *e, YMulti<R> &P, const long *tiles) {
+template <typename R, int S> static int ens_launch_y(ghost_ensemble *e, YMulti<R> &P, const long *values) {
   size_t smem = 0;
   for (int q = 0; q < P.ncls; ++q) {
     switch (P.n[q]) {
@@ -2633,12 +2636,12 @@ template <typename R, int S> static int ens_launch_y(ghost_ensemble *e, YMulti<R
   GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int per = 0;
   GB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, kEnsThreads, smem));
-  const int grid = ens_split(e->cls[0], per, tiles, P);
+  const int grid = ens_split(e->cls[0], per, values, P);
   kern<<<grid, kEnsThreads, smem, e->main>>>(P);
   return post_launch(e->cls[0]);
 }
 
-template <typename R> static int ens_launch_x(ghost_ensemble *e, XMulti<R> &P, const long *tiles) {
+template <typename R> static int ens_launch_x(ghost_ensemble *e, XMulti<R> &P, const long *values) {
   size_t smem = 0;
   for (int q = 0; q < P.ncls; ++q) {
     switch (P.n[q]) {
@@ -2653,7 +2656,7 @@ template <typename R> static int ens_launch_x(ghost_ensemble *e, XMulti<R> &P, c
   GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int per = 0;
   GB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, kEnsThreads, smem));
-  const int grid = ens_split(e->cls[0], per, tiles, P);
+  const int grid = ens_split(e->cls[0], per, values, P);
   kern<<<grid, kEnsThreads, smem, e->main>>>(P);
   return post_launch(e->cls[0]);
 }
@@ -2665,15 +2668,6 @@ template <typename R> static int ens_x_yb_of(int NX) {
     case 32: return ens_x_yb<R, 32>();
     case 64: return ens_x_yb<R, 64>();
     case 128: return ens_x_yb<R, 128>();
-  }
-  return 1;
-}
-static int ens_y_kb_of(int N) {
-  switch (N) {
-    case 16: return ens_y_kb<16>();
-    case 32: return ens_y_kb<32>();
-    case 64: return ens_y_kb<64>();
-    case 128: return ens_y_kb<128>();
   }
   return 1;
 }
@@ -2696,7 +2690,7 @@ template <typename R> static int ens_substep_multi(ghost_ensemble *e, int o, dou
       C[q][k] = c->rk[k];
     }
   }
-  long tiles[kEnsMaxCls];
+  long values[kEnsMaxCls];
   // Z inverse
   {
     ZMulti<R, ZInv<R, 0>> P{};
@@ -2716,10 +2710,9 @@ template <typename R> static int ens_substep_multi(ghost_ensemble *e, int o, dou
       P.cl[q].lines = pr[q].lines;
       P.cl[q].nlines = pr[q].lines ? pr[q].nlines : c->ny * c->nxh * c->nruns;
       P.cl[q].ctl = pipe_ctl(c);
-      const int lpb = kEnsThreads / ens_T<R>(c->nz, c->nz >= 32 ? z_warp_E<R, ZInv<R, 0>>(c->nz) : zE<R>());
-      tiles[q] = (P.cl[q].nlines + lpb - 1) / lpb;
+      values[q] = (long)P.cl[q].nlines * c->nz;
     }
-    GB_CHECK((ens_launch_z<R, ZInv<R, 0>>(e, P, tiles)));
+    GB_CHECK((ens_launch_z<R, ZInv<R, 0>>(e, P, values)));
   }
   // Y inverse (6 fields) and, below, Y forward (3 fields)
   auto ypass = [&](auto sgn, int nf) -> int {
@@ -2731,7 +2724,7 @@ template <typename R> static int ens_substep_multi(ghost_ensemble *e, int o, dou
       YClass<R> &k = P.cl[q];
       const int N = c->ny;
       const bool wl = y_warp_line<R>(N);
-      const int kb = wl ? 1 : ens_y_kb_of(N), bz = wl ? ens_y_warp_BZ<R>() : kEnsYBZ;
+      const int bz = wl ? ens_y_warp_BZ<R>() : kEnsYBZ;
       const YWarpBoxes bx(N, pr[q].jpos != nullptr, S);
       k.rb = wl ? bx.rb : ((pr[q].jpos && S > 0) ? std::min(32, N / 2) : std::min(N, 256));
       k.rbo = bx.rbo;
@@ -2751,9 +2744,9 @@ template <typename R> static int ens_substep_multi(ghost_ensemble *e, int o, dou
       k.jneg = pr[q].jneg;
       k.ctl = pipe_ctl(c);
       P.n[q] = N;
-      tiles[q] = (long)(c->nz / bz) * ((k.ni + kb - 1) / kb) * c->nruns * nf;
+      values[q] = (long)c->nz * N * k.ni * c->nruns * nf;
     }
-    return ens_launch_y<R, S>(e, P, tiles);
+    return ens_launch_y<R, S>(e, P, values);
   };
   GB_CHECK(ypass(std::integral_constant<int, +1>(), 6));
   // X: omega x v
@@ -2787,9 +2780,9 @@ template <typename R> static int ens_substep_multi(ghost_ensemble *e, int o, dou
       k.nxh = c->nxh;
       k.ctl = pipe_ctl(c);
       P.n[q] = c->nx;
-      tiles[q] = (long)(c->nz / bz) * (c->ny / yb) * c->nruns;
+      values[q] = (long)c->nz * c->ny * c->nruns * M;
     }
-    GB_CHECK(ens_launch_x<R>(e, P, tiles));
+    GB_CHECK(ens_launch_x<R>(e, P, values));
   }
   GB_CHECK(ypass(std::integral_constant<int, -1>(), 3));
   // Z forward: nonlhd3, laplak3 and the truncated update
@@ -2814,10 +2807,9 @@ template <typename R> static int ens_substep_multi(ghost_ensemble *e, int o, dou
       P.cl[q].lines = pr[q].lines;
       P.cl[q].nlines = pr[q].lines ? pr[q].nlines : c->ny * c->nxh * c->nruns;
       P.cl[q].ctl = pipe_ctl(c);
-      const int lpb = kEnsThreads / ens_T<R>(c->nz, c->nz >= 32 ? z_warp_E<R, ZFwdHD<R>>(c->nz) : zE<R>());
-      tiles[q] = (P.cl[q].nlines + lpb - 1) / lpb;
+      values[q] = (long)P.cl[q].nlines * c->nz;
     }
-    GB_CHECK((ens_launch_z<R, ZFwdHD<R>>(e, P, tiles)));
+    GB_CHECK((ens_launch_z<R, ZFwdHD<R>>(e, P, values)));
   }
   e->cls[0]->launches += 5;
   return GHOST_OK;
