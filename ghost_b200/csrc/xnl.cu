@@ -55,7 +55,7 @@ bool xnl_takes(ghost_ctx *c) {
   const int bz = sp && c->nx < 1024 ? 16 : 8;
   if (c->nx < 64 || c->nz % bz != 0 || (!sp && c->nx == 1024)) return false;
   if (c->shares_gpu || (sp && c->nx < 256)) return true;
-  // warps of a tile: FP32 256 and FP64 as many as 64-point half lines fit, 8 above
+  // warps of a tile at these lengths (XnlGeom::NW)
   const int nw = c->nx >= 512 ? 8 : c->nx / 64;
   return (long)(c->nz / bz) * c->ny * c->nruns * nw > 4L * sm_count(c);
 }
